@@ -759,16 +759,34 @@ __global__ void coarse_solve_kernel(int n, const double* __restrict__ inv, const
 }
 
 // ---- FP64 PCG kernels -----------------------------------------------------------------
-// y = A p (rows in order, fused multiply-add) and a partial dot(y, p).
+// Row [a, b) of a CSR operator times p: entries in groups of 8 (all columns and values,
+// then all gathers), then the fused multiply-adds in entry order.
+__device__ __forceinline__ double csr_row(int a, int b, const int32_t* __restrict__ ci, const double* __restrict__ v,
+                                          const double* __restrict__ p) {
+  double s = 0.0;
+  for (int e0 = a; e0 < b; e0 += 8) {
+    int c[8];
+    double w[8], x[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      c[k] = e0 + k < b ? ci[e0 + k] : 0;
+      w[k] = e0 + k < b ? v[e0 + k] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) x[k] = e0 + k < b ? p[c[k]] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (e0 + k < b) s = fma(w[k], x[k], s);
+  }
+  return s;
+}
+
+// y = A x, one thread per row.
 __global__ void spmv_kernel(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                             const double* __restrict__ v, const double* __restrict__ x, double* __restrict__ y) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double s = 0.0;
-  for (int e = rp[i]; e < rp[i + 1]; e++) s = fma(v[e], x[ci[e]], s);
-  y[i] = s;
+  if (i < n) y[i] = csr_row(rp[i], rp[i + 1], ci, v, x);
 }
-
 
 // partial dot(a, b) (and dot(a, c) when c != nullptr into partial2)
 __global__ void dot_kernel(int n, const double* __restrict__ a, const double* __restrict__ b,
@@ -936,25 +954,8 @@ __global__ void spmv_dot_kernel(int n, const int32_t* __restrict__ rp, const int
   __shared__ double sh[32];
   double acc = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int a = rp[i], b = rp[i + 1];
     const double pi = p[i];
-    double s = 0.0;
-    // entries in groups of 8: all columns and values, then all gathers, then the
-    // fused multiply-adds in entry order
-    for (int e0 = a; e0 < b; e0 += 8) {
-      int c[8];
-      double w[8], x[8];
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        c[k] = e0 + k < b ? ci[e0 + k] : 0;
-        w[k] = e0 + k < b ? v[e0 + k] : 0.0;
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++) x[k] = e0 + k < b ? p[c[k]] : 0.0;
-#pragma unroll
-      for (int k = 0; k < 8; k++)
-        if (e0 + k < b) s = fma(w[k], x[k], s);
-    }
+    const double s = csr_row(rp[i], rp[i + 1], ci, v, p);
     y[i] = s;
     acc = fma(s, pi, acc);
   }

@@ -252,9 +252,9 @@ void build_mesh_pattern(Ctx& c);
 // coef: per-element coefficients (host array, or device array when coef_on_device), or null
 void assemble_operator(Ctx& c, const double* coef_host, double lambda, bool coef_on_device = false);
 void load_vector(Ctx& c, const double* f_host, double* b_host);
-// The two load-vector passes on device f/b with caller-provided scratch (`scale`
-// and `fsum`, one double per element each); enqueued on c.stream, allocates nothing.
-void load_vector_enqueue(Ctx& c, const double* d_f, double* d_b, double* scale, double* fsum);
+// The two load-vector passes on device f/b with caller-provided scratch (`part`, one
+// 16-byte pair per element); enqueued on c.stream, allocates nothing.
+void load_vector_enqueue(Ctx& c, const double* d_f, double* d_b, double2* part);
 void apply_dirichlet(Ctx& c, const uint8_t* mask_host);
 // out = in with the Dirichlet rows set to zero (n = rows of the operator).
 void zero_dirichlet_rows(Ctx& c, const double* d_in, double* d_out);

@@ -5,10 +5,10 @@
 // (the row of tetmesh2ell / trimesh2ell, src/core/cuda/cutil.cu:168-230,297-348,
 // with the diagonal in its sorted place).
 //
-// Assembly: one thread per element computes the element's upper-triangle
-// entries (perform_element_loop_3D.cuh:480-627 / perform_element_loop_2D.cuh:287-372)
-// into a per-element table; one thread per row then gathers its entries from the
-// incident elements in element order.  No floating-point atomics: the sum at
+// Assembly: one thread per element computes the element's matrix
+// (perform_element_loop_3D.cuh:480-627 / perform_element_loop_2D.cuh:287-372) and stores
+// its rows as 32-byte sectors; one thread per row of the operator then gathers its
+// entries from the incident elements in element order.  No floating-point atomics: the sum at
 // every slot is taken in element order, so results are bitwise reproducible and
 // equal to a sequential element loop.  Tetrahedra use a fused multiply-add gradient
 // formulation (tet_gradients), within a few units in the last place of the reference's
@@ -21,12 +21,33 @@ namespace femgpu {
 namespace {
 
 __constant__ double c_tet_mass[10];
-__constant__ double c_tri_q[24];  // zx[6], wx[6], zy[6], wy[6]
+// Triangle quadrature: wx[6], wy[6], (1 - zx)[6], (1 + zx)[6], (1 - zy)[6], (1 + zy)[6]
+__constant__ double c_tri_q[36];
 
-// Index of entry (a, b) in the packed upper triangle of a k x k element matrix.
-__device__ __forceinline__ int upper_index(int a, int b, int k) {
-  int i = a < b ? a : b, j = a < b ? b : a;
-  return i * k - (i * (i - 1)) / 2 + (j - i);
+// Row r of an element matrix is one 32-byte sector of the element table (four doubles,
+// the last one unused for triangles), at 4 * (e * k + r): the incidence code of the row's
+// vertex, so the gather reads exactly the sectors it adds.
+__device__ __forceinline__ void st_row(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
+// x / D rounded to nearest, for D = 6, 12, 20, in three FP64 operations (the compiler's
+// division takes about three times as many, and these kernels are bound by the FP64 pipe:
+// GB300 issues 2 per SM and clock).  With y = RN(1 / D) the quotient q = RN(x y) is within
+// 1.2 ulp of x / D, so x - D q is exact, and q + (x - D q) y is off x / D by less than
+// 2^-52 ulp before its rounding.  x / D is never that near a rounding boundary: in units of
+// ulp(q), x is a multiple of 4 (D = 6), 8 (12) or 16 (20) and a boundary lies at an odd
+// multiple of D / 2, so they differ by at least 1 / D ulp (Brisebarre, Muller and Raina,
+// "Accelerating correctly rounded floating-point division when the divisor is known in
+// advance", IEEE Trans. Computers 2004).  Tiny, huge and special x take the division.
+template <int D>
+__device__ __forceinline__ double div_const(double x) {
+  static_assert(D == 6 || D == 12 || D == 20, "proved for these divisors");
+  constexpr double y = 1.0 / D;
+  const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  if (hi - 0x03000000u >= 0x7a000000u) return x / (double)D;
+  const double q = x * y;
+  return fma(fma(-(double)D, q, x), y, q);
 }
 
 __device__ __forceinline__ double label_coef(int label) {
@@ -136,9 +157,14 @@ __device__ __forceinline__ void tet_gradients(const double* __restrict__ xyz, co
   }
 }
 
-// Element matrices of P1 tetrahedra: the 10 upper-triangle entries of co K_e + lambda M_e
-// (perform_element_loop_3D.cuh:28-116,480-627): K_ab = vol grad l_a . grad l_b, the mass
-// from the reference-element integrand table times |det| / 8.
+// Element matrices co K_e + lambda M_e of P1 tetrahedra (perform_element_loop_3D.cuh:28-116,
+// 480-627): K_ab = vol grad l_a . grad l_b, the mass from the reference-element integrand
+// table times |det| / 8.  Bound by the FP64 pipe (about 105 operations per element without
+// the mass term, 120 with it).  MASS == false is lambda = 0: the term is then a signed
+// zero, which the row sums (they start from +0) do not see.  Entry-major table, a
+// division by 6 and the mass term always added: 101^3 cells (6.2 M elements), lambda = 1:
+// 1365 us, now 1311; 96^3 cells, lambda = 0: 1172 us, now 909.
+template <bool MASS>
 __global__ void element3d_kernel(const double* __restrict__ xyz, const int32_t* __restrict__ conn,
                                  const int32_t* __restrict__ labels, const double* __restrict__ coef, int64_t ne,
                                  double lambda, double* __restrict__ ev) {
@@ -146,27 +172,40 @@ __global__ void element3d_kernel(const double* __restrict__ xyz, const int32_t* 
     double det, g[4][3];
     tet_gradients(xyz, conn, e, det, g);
     const double co = coef ? coef[e] : (labels ? label_coef(labels[e]) : 1.0);
-    const double wk = (fabs(det) / 6.0) * co;
+    const double wk = div_const<6>(fabs(det)) * co;
     const double jac = fabs(det) * 0.125;
+    double m[4][4];
     int c = 0;
 #pragma unroll
     for (int kk = 0; kk < 4; kk++) {
 #pragma unroll
       for (int q = kk; q < 4; q++) {
         const double st = fma(g[kk][0], g[q][0], fma(g[kk][1], g[q][1], g[kk][2] * g[q][2])) * wk;
-        ev[(int64_t)c * ne + e] = fma(lambda, c_tet_mass[c] * jac, st);  // SoA: entry-major stores
+        m[kk][q] = m[q][kk] = MASS ? fma(lambda, c_tet_mass[c] * jac, st) : st;
         c++;
       }
     }
+    double* o = ev + e * 16;
+#pragma unroll
+    for (int r = 0; r < 4; r++) st_row(o + 4 * r, m[r][0], m[r][1], m[r][2], m[r][3]);
   }
 }
 
-__global__ void element2d_kernel(const double* __restrict__ xyz, const int32_t* __restrict__ conn,
-                                 const double* __restrict__ coef, int64_t ne, double lambda, double* __restrict__ ev) {
-  const double* zx = c_tri_q;
-  const double* wx = c_tri_q + 6;
-  const double* zy = c_tri_q + 12;
-  const double* wy = c_tri_q + 18;
+// Element matrices of P1 triangles in the reference's arithmetic
+// (perform_element_loop_2D.cuh:287-372).  The mass quadrature's basis values at a point do
+// not depend on the entry: they are formed once per point for the three basis functions and
+// used for all six entries, and everything that depends on one quadrature index alone is
+// formed once per index; the operations that remain are the same in the same order (the
+// factors 0.5 are exact and are applied where they cost least).  Bound by the FP64 pipe:
+// 44 operations per point, 36 points.  500^2 cells (0.5 M elements), lambda = 1: 1798 us
+// (every entry its own quadrature: 5139 us).  MASS == false is lambda = 0, as above.
+template <bool MASS>
+__global__ void __launch_bounds__(128) element2d_kernel(const double* __restrict__ xyz,
+                                                        const int32_t* __restrict__ conn,
+                                                        const double* __restrict__ coef, int64_t ne, double lambda,
+                                                        double* __restrict__ ev) {
+  const double *wx = c_tri_q, *wy = c_tri_q + 6, *zxm = c_tri_q + 12, *zxp = c_tri_q + 18, *zym = c_tri_q + 24,
+               *zyp = c_tri_q + 30;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += (int64_t)gridDim.x * blockDim.x) {
     double x[3], y[3];
 #pragma unroll
@@ -183,28 +222,52 @@ __global__ void element2d_kernel(const double* __restrict__ xyz, const int32_t* 
                     (a12 * a23 - a13 * a22) / det, (a13 * a21 - a11 * a23) / det, (a11 * a22 - a12 * a21) / det};
     double jacobi = (x[0] * y[1] - x[1] * y[0] - x[0] * y[2] + x[2] * y[0] + x[1] * y[2] - x[2] * y[1]) / 8;
     double co = coef ? coef[e] : 1.0;
-    int c = 0;
-    for (int k = 0; k < 3; k++)
-      for (int q = k; q < 3; q++) {
-        double A1 = cf[3 * k], B1 = cf[3 * k + 1], C1 = cf[3 * k + 2];
-        double A2 = cf[3 * q], B2 = cf[3 * q + 1], C2 = cf[3 * q + 2];
-        double st = (A1 * A2 + B1 * B2) * area * co;
-        double integral = 0;
-        for (int i = 0; i < 6; i++) {
-          double ty = 0.0;
-          for (int j = 0; j < 6; j++) {
-            double px = x[0] * (1 - zx[i]) * 0.5 * (1 - zy[j]) * 0.5 + x[1] * (1 + zx[i]) * 0.5 * (1 - zy[j]) * 0.5 +
-                        x[2] * (1 + zy[j]) * 0.5;
-            double py = y[0] * (1 - zx[i]) * 0.5 * (1 - zy[j]) * 0.5 + y[1] * (1 + zx[i]) * 0.5 * (1 - zy[j]) * 0.5 +
-                        y[2] * (1 + zy[j]) * 0.5;
-            double f = (A1 * px + B1 * py + C1) * (A2 * px + B2 * py + C2) * jacobi;
-            ty += f * wy[j];
-          }
-          integral += ty * wx[i];
+    double integral[6] = {0, 0, 0, 0, 0, 0};
+    if (MASS) {
+      double x2[6], y2[6];  // the third vertex's share of a point, by the second index
+#pragma unroll
+      for (int j = 0; j < 6; j++) {
+        x2[j] = x[2] * zyp[j] * 0.5;
+        y2[j] = y[2] * zyp[j] * 0.5;
+      }
+#pragma unroll 1
+      for (int i = 0; i < 6; i++) {
+        const double x0 = x[0] * zxm[i] * 0.25, x1 = x[1] * zxp[i] * 0.25;
+        const double y0 = y[0] * zxm[i] * 0.25, y1 = y[1] * zxp[i] * 0.25;
+        double ty[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int j = 0; j < 6; j++) {
+          const double px = x0 * zym[j] + x1 * zym[j] + x2[j];
+          const double py = y0 * zym[j] + y1 * zym[j] + y2[j];
+          double l[3];
+#pragma unroll
+          for (int k = 0; k < 3; k++) l[k] = cf[3 * k] * px + cf[3 * k + 1] * py + cf[3 * k + 2];
+          int c = 0;
+#pragma unroll
+          for (int k = 0; k < 3; k++)
+#pragma unroll
+            for (int q = k; q < 3; q++) {
+              ty[c] += l[k] * l[q] * jacobi * wy[j];
+              c++;
+            }
         }
-        ev[(int64_t)c * ne + e] = st + lambda * integral;
+#pragma unroll
+        for (int c = 0; c < 6; c++) integral[c] += ty[c] * wx[i];
+      }
+    }
+    double m[3][3];
+    int c = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+      for (int q = k; q < 3; q++) {
+        const double st = (cf[3 * k] * cf[3 * q] + cf[3 * k + 1] * cf[3 * q + 1]) * area * co;
+        m[k][q] = m[q][k] = MASS ? st + lambda * integral[c] : st;
         c++;
       }
+    double* o = ev + e * 12;
+#pragma unroll
+    for (int r = 0; r < 3; r++) st_row(o + 4 * r, m[r][0], m[r][1], m[r][2], 0.0);
   }
 }
 
@@ -232,38 +295,81 @@ __global__ void slot_map_kernel(const int32_t* __restrict__ rowptr, const int32_
   }
 }
 
-// One thread per row with its row's sums in shared memory (at most kSlotRowMax entries,
-// kSlotRowMax + 1 doubles apart per thread): the incident elements' contributions added
-// in element order at the positions the slot map gives, then the row written out.
-__global__ void gather_rows_slot_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ vstart,
-                                        const int32_t* __restrict__ inc, const uint8_t* __restrict__ slot,
-                                        const double* __restrict__ ev, int64_t ne, int nv, int k,
-                                        double* __restrict__ vals) {
-  extern __shared__ double acc_all[];
-  double* acc = acc_all + threadIdx.x * (kSlotRowMax + 1);
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-    const int rb = rowptr[v], len = rowptr[v + 1] - rb;
-    for (int s = 0; s < len; s++) acc[s] = 0.0;
-    for (int q = vstart[v]; q < vstart[v + 1]; q++) {
-      const int code = inc[q];
-      const int e = code / k, a = code - e * k;
-      for (int b = 0; b < k; b++) acc[slot[(int64_t)q * k + b]] += ev[(int64_t)upper_index(a, b, k) * ne + e];
-    }
-    for (int s = 0; s < len; s++) vals[rb + s] = acc[s];
+// Four lanes per row with the row's sums in shared memory (at most kSlotRowMax entries,
+// kSlotRowMax + 1 doubles apart per row): lane b adds entry b of each incident element's
+// row, in element order, at the position the slot map gives (an element's vertices are
+// distinct, so the lanes of a row never meet; an element that repeats a vertex has zero
+// volume and only NaN entries).  Bound by the chain of shared-memory adds, 24 per row of a
+// tetrahedral mesh, so a row's lanes work side by side and the sectors, codes and slots of
+// the next four elements are loaded ahead.  101^3 cells: 335 us (one thread per row,
+// entry-major table, four 8-byte reads of as many sectors per incidence: 874 us; one thread
+// per row on this table: 705 us).
+constexpr int kGatherThreads = 256;
+
+template <int K>
+__global__ void __launch_bounds__(kGatherThreads, 6) gather_rows_slot_kernel(
+    const int32_t* __restrict__ rowptr, const int32_t* __restrict__ vstart, const int32_t* __restrict__ inc,
+    const uint8_t* __restrict__ slot, const double* __restrict__ ev, int nv, double* __restrict__ vals) {
+  __shared__ double acc_all[(kGatherThreads / 4) * (kSlotRowMax + 1)];
+  const int b = threadIdx.x & 3;
+  double* acc = acc_all + (threadIdx.x >> 2) * (kSlotRowMax + 1);
+  const int v = blockIdx.x * (kGatherThreads / 4) + (threadIdx.x >> 2);
+  int rb = 0, len = 0, q0 = 0, q1 = 0;
+  if (v < nv) {
+    rb = rowptr[v];
+    len = rowptr[v + 1] - rb;
+    q0 = vstart[v];
+    q1 = vstart[v + 1];
   }
+  for (int s = b; s < len; s += 4) acc[s] = 0.0;
+  __syncwarp();
+  // every row of the warp takes the trips of its longest one, so the warp stays together
+  constexpr int U = 4;
+  const int trips = (int)__reduce_max_sync(0xffffffffu, (unsigned)(q1 - q0));
+  if (b >= K) q1 = q0;  // triangles leave the fourth lane idle
+  int sl[U];
+  double r[U];
+  auto load = [&](int q) {
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (q + u < q1) {
+        sl[u] = slot[(int64_t)(q + u) * K + b];
+        r[u] = ev[(int64_t)inc[q + u] * 4 + b];
+      }
+  };
+  load(q0);
+  for (int t = 0; t < trips; t += U) {
+    const int q = q0 + t;
+    int at[U];
+    double w[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      at[u] = sl[u];
+      w[u] = r[u];
+    }
+    load(q + U);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (q + u < q1) acc[at[u]] += w[u];
+      __syncwarp();  // a column's next contribution may come from another lane of the row
+    }
+  }
+  __syncwarp();
+  for (int s = b; s < len; s += 4) vals[rb + s] = acc[s];
 }
 
-// One thread per row: contributions of the incident elements, in element order.
+// One thread per row, rows of any length: contributions of the incident elements, in
+// element order, their places found by binary search.
 __global__ void gather_rows_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ cols,
                                    const int32_t* __restrict__ vstart, const int32_t* __restrict__ inc,
-                                   const int32_t* __restrict__ conn, const double* __restrict__ ev, int64_t ne, int nv,
+                                   const int32_t* __restrict__ conn, const double* __restrict__ ev, int nv,
                                    int k, double* __restrict__ vals, int32_t* bad) {
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
     int rb = rowptr[v], re = rowptr[v + 1];
     for (int s = rb; s < re; s++) vals[s] = 0.0;
     for (int q = vstart[v]; q < vstart[v + 1]; q++) {
       int code = inc[q];
-      int e = code / k, a = code - e * k;
+      int e = code / k;
       for (int b = 0; b < k; b++) {
         int col = conn[(int64_t)e * k + b];
         int s = lower_bound_i32(cols, rb, re, col);
@@ -271,15 +377,19 @@ __global__ void gather_rows_kernel(const int32_t* __restrict__ rowptr, const int
           atomicExch(bad, 1);
           continue;
         }
-        vals[s] += ev[(int64_t)upper_index(a, b, k) * ne + e];
+        vals[s] += ev[(int64_t)code * 4 + b];
       }
     }
   }
 }
 
+// Per element: (measure / (k (k + 1)), sum of f over its vertices).  Bound by the FP64 pipe
+// (33 operations per tetrahedron).  60^3 cells (1.3 M elements): 90 us (two divisions:
+// 113 us).
+template <int K>
 __global__ void element_load_kernel(const double* __restrict__ xyz, const int32_t* __restrict__ conn,
-                                    const double* __restrict__ f, int64_t ne, int k, double* __restrict__ scale,
-                                    double* __restrict__ fsum) {
+                                    const double* __restrict__ f, int64_t ne, double2* __restrict__ part) {
+  constexpr int k = K;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += (int64_t)gridDim.x * blockDim.x) {
     double meas;
     if (k == 4) {
@@ -293,7 +403,8 @@ __global__ void element_load_kernel(const double* __restrict__ xyz, const int32_
       double a1 = x[1] - x[3], a2 = y[1] - y[3], a3 = z[1] - z[3];
       double b1 = x[2] - x[3], b2 = y[2] - y[3], b3 = z[2] - z[3];
       double c1 = x[0] - x[3], c2 = y[0] - y[3], c3 = z[0] - z[3];
-      meas = fabs(c1 * (a2 * b3 - a3 * b2) + c2 * (a3 * b1 - a1 * b3) + c3 * (a1 * b2 - a2 * b1)) / 6.0;
+      meas = fabs(c1 * (a2 * b3 - a3 * b2) + c2 * (a3 * b1 - a1 * b3) + c3 * (a1 * b2 - a2 * b1));
+      meas = div_const<6>(meas);
     } else {
       int v0 = conn[e * 3], v1 = conn[e * 3 + 1], v2 = conn[e * 3 + 2];
       double x0 = xyz[(int64_t)v0 * 3], y0 = xyz[(int64_t)v0 * 3 + 1];
@@ -302,20 +413,29 @@ __global__ void element_load_kernel(const double* __restrict__ xyz, const int32_
       meas = fabs(x0 * y2 - x0 * y1 + x1 * y0 - x1 * y2 + x2 * y1 - x2 * y0) / 2.0;
     }
     double fs = 0;
+#pragma unroll
     for (int a = 0; a < k; a++) fs += f[conn[e * k + a]];
-    scale[e] = meas / (double)(k * (k + 1));
-    fsum[e] = fs;
+    part[e] = make_double2(div_const<K*(K + 1)>(meas), fs);
   }
 }
 
-__global__ void gather_load_kernel(const int32_t* vstart, const int32_t* inc, const double* scale, const double* fsum,
-                                   const double* f, int nv, int k, double* b) {
+// b_v = sum over the incident elements, in element order (eight in flight).  60^3 cells:
+// 39 us (two arrays, one element at a time: 44 us).
+template <int K>
+__global__ void gather_load_kernel(const int32_t* __restrict__ vstart, const int32_t* __restrict__ inc,
+                                   const double2* __restrict__ part, const double* __restrict__ f, int nv,
+                                   double* __restrict__ b) {
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
     double s = 0.0;
-    double fv = f[v];
-    for (int q = vstart[v]; q < vstart[v + 1]; q++) {
-      int e = inc[q] / k;
-      s += scale[e] * (fsum[e] + fv);
+    const double fv = f[v];
+    const int q1 = vstart[v + 1];
+    for (int q0 = vstart[v]; q0 < q1; q0 += 8) {
+      double2 p[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) p[u] = part[inc[min(q0 + u, q1 - 1)] / K];
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        if (q0 + u < q1) s += p[u].x * (p[u].y + fv);
     }
     b[v] = s;
   }
@@ -408,20 +528,35 @@ int reduce_max_row_length(Ctx& c) {
   return reduce_max(len.p, c.A.n, c.stream);
 }
 
-// Row gather of the element entries into the operator's values (slot map when built).
+// The element matrices into the element table (4 doubles per incidence).
+void element_matrices(Ctx& c, const double* coef, double lambda, double* ev) {
+  cudaStream_t s = c.stream;
+  Mesh& M = c.mesh;
+  const int g = grid_for(M.ne, 128);
+  const int32_t* lab = M.has_labels ? M.labels.p : nullptr;
+  if (M.k == 4) {
+    auto k = lambda != 0.0 ? element3d_kernel<true> : element3d_kernel<false>;
+    FG_LAUNCH(k, g, 128, 0, s, M.xyz.p, M.conn.p, lab, coef, M.ne, lambda, ev);
+  } else {
+    auto k = lambda != 0.0 ? element2d_kernel<true> : element2d_kernel<false>;
+    FG_LAUNCH(k, g, 128, 0, s, M.xyz.p, M.conn.p, coef, M.ne, lambda, ev);
+  }
+}
+
+// Row gather of the element table into the operator's values (slot map when built).
 void gather_rows(Ctx& c, const double* ev, double* vals) {
   cudaStream_t s = c.stream;
   Mesh& M = c.mesh;
   if (M.slot.n) {
-    const size_t smem = (size_t)128 * (kSlotRowMax + 1) * sizeof(double);
-    FG_LAUNCH(gather_rows_slot_kernel, grid_for(M.nv, 128), 128, smem, s, c.A.rp.p, M.vstart.p, M.inc.p, M.slot.p,
-              ev, M.ne, (int)M.nv, M.k, vals);
+    auto k = M.k == 4 ? gather_rows_slot_kernel<4> : gather_rows_slot_kernel<3>;
+    FG_LAUNCH(k, grid_for(M.nv, kGatherThreads / 4), kGatherThreads, 0, s, c.A.rp.p, M.vstart.p, M.inc.p, M.slot.p, ev,
+              (int)M.nv, vals);
     return;
   }
   DBuf<int32_t> bad(1, s);
   bad.zero();
   FG_LAUNCH(gather_rows_kernel, grid_for(M.nv, 128), 128, 0, s, c.A.rp.p, c.A.ci.p, M.vstart.p, M.inc.p, M.conn.p,
-            ev, M.ne, (int)M.nv, M.k, vals, bad.p);
+            ev, (int)M.nv, M.k, vals, bad.p);
   FG_REQUIRE(read_scalar(bad.p, s) == 0, FEMGPU_ERR_INVALID, "element entry outside the pattern");
 }
 
@@ -485,19 +620,20 @@ void assemble_operator(Ctx& c, const double* coef_host, double lambda, bool coef
   Mesh& M = c.mesh;
   const int64_t ne = M.ne;
   const int k = M.k;
-  const int nup = k == 4 ? 10 : 6;
   if (k == 4) {
     double t[10];
     tet_mass_table(t);
     FG_CUDA(cudaMemcpyToSymbolAsync(c_tet_mass, t, sizeof(t), 0, cudaMemcpyHostToDevice, s));
   } else {
-    double zx[6], wx[6], zy[6], wy[6], q[24];
+    double zx[6], wx[6], zy[6], wy[6], q[36];
     tri_quadrature_table(zx, wx, zy, wy);
     for (int i = 0; i < 6; i++) {
-      q[i] = zx[i];
-      q[6 + i] = wx[i];
-      q[12 + i] = zy[i];
-      q[18 + i] = wy[i];
+      q[i] = wx[i];
+      q[6 + i] = wy[i];
+      q[12 + i] = 1 - zx[i];
+      q[18 + i] = 1 + zx[i];
+      q[24 + i] = 1 - zy[i];
+      q[30 + i] = 1 + zy[i];
     }
     FG_CUDA(cudaMemcpyToSymbolAsync(c_tri_q, q, sizeof(q), 0, cudaMemcpyHostToDevice, s));
   }
@@ -511,33 +647,29 @@ void assemble_operator(Ctx& c, const double* coef_host, double lambda, bool coef
     else
       coef.upload(coef_host, ne);
   }
-  DBuf<double> ev((size_t)ne * nup, s);
-  if (k == 4)
-    FG_LAUNCH(element3d_kernel, grid_for(ne, 128), 128, 0, s, M.xyz.p, M.conn.p, M.has_labels ? M.labels.p : nullptr,
-              coef.p, ne, lambda, ev.p);
-  else
-    FG_LAUNCH(element2d_kernel, grid_for(ne, 128), 128, 0, s, M.xyz.p, M.conn.p, coef.p, ne, lambda, ev.p);
+  DBuf<double> ev((size_t)ne * k * 4, s);
+  element_matrices(c, coef.p, lambda, ev.p);
   gather_rows(c, ev.p, c.A.v.p);
 }
 
 void load_vector(Ctx& c, const double* f_host, double* b_host) {
   cudaStream_t s = c.stream;
   Mesh& M = c.mesh;
-  DBuf<double> f(M.nv, s), b(M.nv, s), sc(M.ne, s), fs(M.ne, s);
+  DBuf<double> f(M.nv, s), b(M.nv, s);
+  DBuf<double2> part(M.ne, s);
   f.upload(f_host, M.nv);
-  FG_LAUNCH(element_load_kernel, grid_for(M.ne, 256), 256, 0, s, M.xyz.p, M.conn.p, f.p, M.ne, M.k, sc.p, fs.p);
-  FG_LAUNCH(gather_load_kernel, grid_for(M.nv, 256), 256, 0, s, M.vstart.p, M.inc.p, sc.p, fs.p, f.p, (int)M.nv, M.k,
-            b.p);
+  load_vector_enqueue(c, f.p, b.p, part.p);
   b.download(b_host, M.nv);
   FG_CUDA(cudaStreamSynchronize(s));
 }
 
-void load_vector_enqueue(Ctx& c, const double* d_f, double* d_b, double* scale, double* fsum) {
+void load_vector_enqueue(Ctx& c, const double* d_f, double* d_b, double2* part) {
   cudaStream_t s = c.stream;
   Mesh& M = c.mesh;
-  FG_LAUNCH(element_load_kernel, grid_for(M.ne, 256), 256, 0, s, M.xyz.p, M.conn.p, d_f, M.ne, M.k, scale, fsum);
-  FG_LAUNCH(gather_load_kernel, grid_for(M.nv, 256), 256, 0, s, M.vstart.p, M.inc.p, scale, fsum, d_f, (int)M.nv,
-            M.k, d_b);
+  auto el = M.k == 4 ? element_load_kernel<4> : element_load_kernel<3>;
+  auto ga = M.k == 4 ? gather_load_kernel<4> : gather_load_kernel<3>;
+  FG_LAUNCH(el, grid_for(M.ne, 256), 256, 0, s, M.xyz.p, M.conn.p, d_f, M.ne, part);
+  FG_LAUNCH(ga, grid_for(M.nv, 128), 128, 0, s, M.vstart.p, M.inc.p, part, d_f, (int)M.nv, d_b);
 }
 
 void zero_dirichlet_rows(Ctx& c, const double* d_in, double* d_out) {
@@ -561,16 +693,10 @@ void profile_assembly(Ctx& c, int which, int reps, double* ms, double* bytes) {
   cudaStream_t s = c.stream;
   Mesh& M = c.mesh;
   const int64_t ne = M.ne, nv = M.nv, nnz = c.A.nnz;
-  const int k = M.k, nup = k == 4 ? 10 : 6;
-  DBuf<double> ev((size_t)ne * nup, s), vals(nnz, s);
+  const int k = M.k;
+  DBuf<double> ev((size_t)ne * k * 4, s), vals(nnz, s);
   const double* coef = c.coef.n ? c.coef.p : nullptr;
-  auto element = [&]() {
-    if (k == 4)
-      FG_LAUNCH(element3d_kernel, grid_for(ne, 128), 128, 0, s, M.xyz.p, M.conn.p,
-                M.has_labels ? M.labels.p : nullptr, coef, ne, c.lambda_mass, ev.p);
-    else
-      FG_LAUNCH(element2d_kernel, grid_for(ne, 128), 128, 0, s, M.xyz.p, M.conn.p, coef, ne, c.lambda_mass, ev.p);
-  };
+  auto element = [&]() { element_matrices(c, coef, c.lambda_mass, ev.p); };
   auto gather = [&]() { gather_rows(c, ev.p, vals.p); };
   element();
   auto run = [&]() {
@@ -578,11 +704,11 @@ void profile_assembly(Ctx& c, int which, int reps, double* ms, double* bytes) {
     else gather();
   };
   if (which == 6)  // connectivity, coefficient and entries per element, coordinates once per vertex
-    *bytes = (double)ne * (4.0 * k + (coef ? 8.0 : 0.0) + 8.0 * nup) + 24.0 * nv;
+    *bytes = (double)ne * (4.0 * k + (coef ? 8.0 : 0.0) + 32.0 * k) + 24.0 * nv;
   else if (M.slot.n)  // row and incidence offsets, incidence lists, slot map, element entries, values out
-    *bytes = 8.0 * (nv + 1) + 4.0 * k * ne + 1.0 * k * k * ne + 8.0 * nup * ne + 8.0 * nnz;
+    *bytes = 8.0 * (nv + 1) + 4.0 * k * ne + 1.0 * k * k * ne + 32.0 * k * ne + 8.0 * nnz;
   else  // row offsets, columns, incidence offsets and lists, the incident elements' vertices and entries, values out
-    *bytes = 8.0 * (nv + 1) + 4.0 * nnz + 4.0 * k * ne + 4.0 * k * ne + 8.0 * nup * ne + 8.0 * nnz;
+    *bytes = 8.0 * (nv + 1) + 4.0 * nnz + 4.0 * k * ne + 4.0 * k * ne + 32.0 * k * ne + 8.0 * nnz;
   for (int i = 0; i < 3; i++) run();
   cudaEvent_t e0, e1;
   FG_CUDA(cudaEventCreate(&e0));

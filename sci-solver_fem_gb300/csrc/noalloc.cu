@@ -15,8 +15,7 @@ namespace {
 
 constexpr int64_t kMaxElements = FEMGPU_NOALLOC_MAX_ELEMENTS;
 
-// [0, kMaxElements): per-element measure / (k (k + 1)); [kMaxElements, 2 kMaxElements):
-// per-element sum of f over the element's vertices.
+// Element e: [2 e] measure / (k (k + 1)), [2 e + 1] sum of f over the element's vertices.
 static __device__ __align__(256) double g_load_scratch[2 * kMaxElements];
 
 // Device address of the region in the handle's context, looked up on the handle's first
@@ -42,8 +41,7 @@ extern "C" femgpu_status femgpu_load_vector_device_noalloc(femgpu_handle h, cons
     FG_REQUIRE(h->has_mesh, FEMGPU_ERR_NOT_READY, "femgpu_set_mesh first");
     FG_REQUIRE(h->mesh.ne <= kMaxElements, FEMGPU_ERR_LIMIT,
                "mesh has more elements than the no-alloc scratch holds (FEMGPU_NOALLOC_MAX_ELEMENTS)");
-    double* base = scratch_of(h);
-    load_vector_enqueue(*h, d_f, d_b, base, base + kMaxElements);
+    load_vector_enqueue(*h, d_f, d_b, reinterpret_cast<double2*>(scratch_of(h)));
     return FEMGPU_OK;
   } catch (const Error& e) {
     h->last_error = e.what();
