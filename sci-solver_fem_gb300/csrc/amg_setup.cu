@@ -407,8 +407,7 @@ int aggregate(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int depth,
   random_mis(c, n, xadj, adj, depth, mis);
   pt.mark("mis");
   DBuf<int32_t> incl(n + 1, s), aggregated(n, s), pout(n, s), counters(2, s);
-  FG_CUDA(cudaMemcpyAsync(incl.p, mis.p, n * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-  inclusive_scan_inplace(incl.p, n, s);
+  inclusive_scan(mis.p, incl.p, n, s);
   // the MIS size (= the number of parts, labelled 0 .. count-1 by label_roots_kernel)
   // comes back with the first allocation counters
   int mis_count = -1;

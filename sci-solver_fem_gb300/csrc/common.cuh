@@ -165,8 +165,8 @@ inline T read_scalar(const T* d, cudaStream_t s) {
 int64_t exclusive_scan(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s);
 // The same scan with the total left on the device (out[n]); no host round trip.
 void exclusive_scan_async(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s);
-// Inclusive scan in place.
-void inclusive_scan_inplace(int32_t* a, int64_t n, cudaStream_t s);
+// Inclusive scan (out may alias in); no host round trip.
+void inclusive_scan(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s);
 int32_t reduce_max(const int32_t* a, int64_t n, cudaStream_t s);
 // The same maximum written to out[0] on the device (INT32_MIN when n == 0).
 void reduce_max_async(const int32_t* a, int64_t n, int32_t* out, cudaStream_t s);

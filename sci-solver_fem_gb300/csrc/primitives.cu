@@ -22,11 +22,27 @@ void ensure_dynamic_smem(const void* func, size_t bytes) {
 
 namespace {
 
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;
+#define FG_RUN(...)    \
+  do {                 \
+    __VA_ARGS__;       \
+    FG_CHECK_LAUNCH(); \
+  } while (0)
 
-// Block-wide exclusive scan of ITEMS consecutive values per thread.
+// ---- scans ----------------------------------------------------------------------
+// Setup runs about 20 scans per level, most of them over a few thousand counts, where a
+// launch (2.2-3 us back to back) costs more than the work: up to kScanOne counts are
+// scanned by one block that carries its total from tile to tile and writes the total entry
+// itself (one launch; a scan with separate kernels for the saved last entry, the tiles, the
+// tile sums, their addition and the total took three to five).  Longer arrays take two
+// launches: tile sums, then every block adds up the sums before its tile and scans it.
+// 2 k counts: 7.8 -> 3.6 us of device time; 2.1 M: 28 -> 12 us.
+constexpr int kScanThreads = 1024;
+constexpr int kScanItems = 8;
+constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int64_t kScanOne = 2 * kScanTile;   // two tiles by one block: 4.6 us, as two launches
+constexpr int64_t kScanSumsInBlock = 2048;    // tile sums that every block adds up by itself
+
+// Block-wide exclusive scan of one value per thread; *total gets the block's sum.
 __device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t* warp_sums, int32_t* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int32_t x = v;
@@ -52,58 +68,125 @@ __device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t* warp
   return warp_sums[warp] + x - v;
 }
 
-__global__ void scan_tiles_kernel(const int32_t* in, int32_t* out, int64_t n, int32_t* tile_sums) {
-  __shared__ int32_t warp_sums[32];
-  __shared__ int32_t total;
-  int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
+// A thread's kScanItems consecutive values of a tile (zero past n): two 16-byte loads when
+// the array and the range allow it.
+__device__ __forceinline__ void scan_load(const int32_t* in, int64_t base, int64_t n, int32_t v[kScanItems]) {
+  if (base + kScanItems <= n && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
+    const int4* p = reinterpret_cast<const int4*>(in + base);
+    const int4 a = p[0], b = p[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) v[k] = base + k < n ? in[base + k] : 0;
+}
+
+// Scans tile `tile` from `carry`; returns the tile's sum.  The block reads its tile before
+// it writes it, so in and out may be the same array.
+template <bool INCLUSIVE>
+__device__ __forceinline__ int32_t scan_tile(const int32_t* in, int32_t* out, int64_t n, int64_t tile, int32_t carry,
+                                             int32_t* warp_sums, int32_t* total) {
+  const int64_t base = tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
   int32_t v[kScanItems];
+  scan_load(in, base, n, v);
   int32_t local = 0;
 #pragma unroll
-  for (int k = 0; k < kScanItems; k++) {
-    int64_t i = base + k;
-    v[k] = (i < n) ? in[i] : 0;
-    local += v[k];
-  }
-  int32_t off = block_exclusive_scan(local, warp_sums, &total);
+  for (int k = 0; k < kScanItems; k++) local += v[k];
+  int32_t off = carry + block_exclusive_scan(local, warp_sums, total);
 #pragma unroll
   for (int k = 0; k < kScanItems; k++) {
-    int64_t i = base + k;
-    if (i < n) out[i] = off;
+    const int32_t e = off;
     off += v[k];
+    v[k] = INCLUSIVE ? off : e;
   }
-  if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+  if (base + kScanItems <= n && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    int4* p = reinterpret_cast<int4*>(out + base);
+    p[0] = make_int4(v[0], v[1], v[2], v[3]);
+    p[1] = make_int4(v[4], v[5], v[6], v[7]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++)
+      if (base + k < n) out[base + k] = v[k];
+  }
+  return *total;
 }
 
-__global__ void add_tile_offsets_kernel(int32_t* out, int64_t n, const int32_t* tile_offsets) {
-  int64_t base = (int64_t)blockIdx.x * kScanTile;
-  int32_t add = tile_offsets[blockIdx.x];
-  for (int k = threadIdx.x; k < kScanTile; k += blockDim.x) {
-    int64_t i = base + k;
-    if (i < n) out[i] += add;
+template <bool INCLUSIVE>
+__global__ void __launch_bounds__(kScanThreads) scan_one_kernel(const int32_t* in, int32_t* out, int64_t n) {
+  __shared__ int32_t warp_sums[32];
+  __shared__ int32_t total;
+  int32_t carry = 0;
+  for (int64_t t = 0; t * kScanTile < n; t++) {
+    carry += scan_tile<INCLUSIVE>(in, out, n, t, carry, warp_sums, &total);
+    __syncthreads();  // warp_sums and total are free for the next tile
+  }
+  if (!INCLUSIVE && threadIdx.x == 0) out[n] = carry;
+}
+
+__global__ void __launch_bounds__(kScanThreads) tile_sums_kernel(const int32_t* in, int64_t n, int32_t* sums) {
+  __shared__ int32_t ws[32];
+  int32_t v[kScanItems], s = 0;
+  scan_load(in, (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems, n, v);
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) s += v[k];
+  s = __reduce_add_sync(0xffffffffu, s);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = __reduce_add_sync(0xffffffffu, ws[threadIdx.x]);
+    if (threadIdx.x == 0) sums[blockIdx.x] = s;
   }
 }
 
-__global__ void write_total_kernel(int32_t* out, int64_t n, const int32_t* last_in_copy, int32_t has_last) {
-  // out[n] = out[n-1] + in[n-1] (in[n-1] saved before an in-place scan)
-  if (threadIdx.x == 0 && blockIdx.x == 0) out[n] = (n > 0 ? out[n - 1] + (has_last ? *last_in_copy : 0) : 0);
+// `scanned`: sums holds the exclusive scan of the tile sums, else the sums themselves.
+template <bool INCLUSIVE>
+__global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(const int32_t* in, int32_t* out, int64_t n,
+                                                                  const int32_t* sums, int scanned) {
+  __shared__ int32_t warp_sums[32];
+  __shared__ int32_t total;
+  int32_t carry;
+  if (scanned) {
+    carry = sums[blockIdx.x];
+  } else {
+    int32_t s = 0;
+    for (int t = threadIdx.x; t < (int)blockIdx.x; t += kScanThreads) s += sums[t];
+    block_exclusive_scan(s, warp_sums, &total);
+    carry = total;
+    __syncthreads();
+  }
+  carry += scan_tile<INCLUSIVE>(in, out, n, blockIdx.x, carry, warp_sums, &total);
+  if (!INCLUSIVE && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = carry;
 }
 
-// Recursive exclusive scan without the total entry.
-void exclusive_scan_rec(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s) {
-  if (n <= 0) return;
-  int64_t tiles = (n + kScanTile - 1) / kScanTile;
+template <bool INCLUSIVE>
+void scan(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s) {
+  if (n <= kScanOne) {
+    if (INCLUSIVE && n <= 0) return;
+    FG_RUN(scan_one_kernel<INCLUSIVE><<<1, kScanThreads, 0, s>>>(in, out, n < 0 ? 0 : n));
+    return;
+  }
+  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
   DBuf<int32_t> sums(tiles + 1, s);
-  scan_tiles_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(in, out, n, sums.p);
-  FG_CHECK_LAUNCH();
-  if (tiles > 1) {
-    exclusive_scan_rec(sums.p, sums.p, tiles, s);
-    add_tile_offsets_kernel<<<(unsigned)tiles, 256, 0, s>>>(out, n, sums.p);
-    FG_CHECK_LAUNCH();
-  }
+  FG_RUN(tile_sums_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, sums.p));
+  const bool deep = tiles > kScanSumsInBlock;
+  if (deep) scan<false>(sums.p, sums.p, tiles, s);
+  FG_RUN(scan_tiles_kernel<INCLUSIVE><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, out, n, sums.p, deep));
 }
 
-__global__ void copy_one_kernel(const int32_t* src, int32_t* dst) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *dst = *src;
+// One block: the maximum of a[0 .. n) straight to *out.
+__global__ void __launch_bounds__(1024) reduce_max_one_kernel(const int32_t* a, int64_t n, int32_t* out) {
+  __shared__ int32_t wm[32];
+  int32_t m = INT32_MIN;
+#pragma unroll 4
+  for (int64_t i = threadIdx.x; i < n; i += 1024) m = max(m, a[i]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    m = __reduce_max_sync(0xffffffffu, wm[threadIdx.x]);
+    if (threadIdx.x == 0) *out = m;
+  }
 }
 
 __global__ void reduce_max_kernel(const int32_t* a, int64_t n, int32_t* out) {
@@ -208,24 +291,6 @@ __global__ void segsort_warp_kernel(int32_t* vals, const int32_t* off, int nseg,
   }
 }
 
-__global__ void segsort_block_kernel(int32_t* vals, const int32_t* off, int nseg, int32_t* ucount) {
-  __shared__ int32_t s[kBlockCap];
-  __shared__ int32_t cnt;
-  const int seg = blockIdx.x;
-  int b = off[seg], e = off[seg + 1], len = e - b;
-  if (len <= kWarpCap || len > kBlockCap) return;
-  int np2 = next_pow2(len);
-  for (int i = threadIdx.x; i < np2; i += blockDim.x) s[i] = (i < len) ? vals[b + i] : INT32_MAX;
-  __syncthreads();
-  bitonic_sort_shared(s, np2, threadIdx.x, blockDim.x, BlockSync());
-  if (ucount) {
-    int c = unique_write(s, len, vals + b, threadIdx.x, blockDim.x, &cnt, BlockSync());
-    if (threadIdx.x == 0) ucount[seg] = c;
-  } else {
-    for (int i = threadIdx.x; i < len; i += blockDim.x) vals[b + i] = s[i];
-  }
-}
-
 // Heap sort in global memory for segments beyond the shared-memory tiers.
 __device__ void sift_down(int32_t* a, int start, int end) {
   int root = start;
@@ -241,72 +306,81 @@ __device__ void sift_down(int32_t* a, int start, int end) {
   }
 }
 
-__global__ void segsort_serial_kernel(int32_t* vals, const int32_t* off, int nseg, int32_t* ucount) {
-  for (int seg = blockIdx.x * blockDim.x + threadIdx.x; seg < nseg; seg += gridDim.x * blockDim.x) {
-    int b = off[seg], e = off[seg + 1], len = e - b;
-    if (len <= kBlockCap) continue;
-    int32_t* a = vals + b;
-    for (int st = (len - 2) / 2; st >= 0; st--) sift_down(a, st, len - 1);
-    for (int end = len - 1; end > 0; end--) {
-      int32_t t = a[0];
-      a[0] = a[end];
-      a[end] = t;
-      sift_down(a, 0, end - 1);
+// Segments longer than a warp's capacity: block b looks at segments 1024 b .. 1024 b + 1023
+// (and so on over the grid), lists the long ones and sorts them one after the other, so the
+// host needs no look at the lengths.  Lists of that length are rare (a vertex in more than
+// 256 elements); without one the kernel reads the offsets and ends.
+__global__ void __launch_bounds__(1024) segsort_long_kernel(int32_t* vals, const int32_t* off, int nseg,
+                                                            int32_t* ucount) {
+  __shared__ int32_t s[kBlockCap];
+  __shared__ int32_t list[1024];
+  __shared__ int32_t cnt, nlist;
+  for (int64_t s0 = (int64_t)blockIdx.x * 1024; s0 < nseg; s0 += (int64_t)gridDim.x * 1024) {
+    const int mine = (int)s0 + (int)threadIdx.x;
+    const bool is_long = mine < nseg && off[mine + 1] - off[mine] > kWarpCap;
+    if (!__syncthreads_or(is_long)) continue;
+    if (threadIdx.x == 0) nlist = 0;
+    __syncthreads();
+    if (is_long) list[atomicAdd(&nlist, 1)] = mine;
+    __syncthreads();
+    for (int k = 0; k < nlist; k++) {
+      const int seg = list[k], b = off[seg], len = off[seg + 1] - b;
+      if (len <= kBlockCap) {
+        const int np2 = next_pow2(len);
+        for (int i = threadIdx.x; i < np2; i += blockDim.x) s[i] = (i < len) ? vals[b + i] : INT32_MAX;
+        __syncthreads();
+        bitonic_sort_shared(s, np2, threadIdx.x, blockDim.x, BlockSync());
+        if (ucount) {
+          const int c = unique_write(s, len, vals + b, threadIdx.x, blockDim.x, &cnt, BlockSync());
+          if (threadIdx.x == 0) ucount[seg] = c;
+        } else {
+          for (int i = threadIdx.x; i < len; i += blockDim.x) vals[b + i] = s[i];
+        }
+      } else if (threadIdx.x == 0) {
+        int32_t* a = vals + b;
+        for (int st = (len - 2) / 2; st >= 0; st--) sift_down(a, st, len - 1);
+        for (int end = len - 1; end > 0; end--) {
+          const int32_t t = a[0];
+          a[0] = a[end];
+          a[end] = t;
+          sift_down(a, 0, end - 1);
+        }
+        if (ucount) {
+          int c = 0;
+          for (int p = 0; p < len; p++)
+            if (p == 0 || a[p] != a[p - 1]) a[c++] = a[p];
+          ucount[seg] = c;
+        }
+      }
+      __syncthreads();
     }
-    if (ucount) {
-      int c = 0;
-      for (int p = 0; p < len; p++)
-        if (p == 0 || a[p] != a[p - 1]) a[c++] = a[p];
-      ucount[seg] = c;
-    }
+    __syncthreads();
   }
-}
-
-__global__ void seg_len_kernel(const int32_t* off, int nseg, int32_t* out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nseg; i += gridDim.x * blockDim.x) out[i] = off[i + 1] - off[i];
 }
 
 }  // namespace
 
-void exclusive_scan_async(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s) {
-  DBuf<int32_t> last(1, s);
-  if (n > 0) {
-    copy_one_kernel<<<1, 32, 0, s>>>(in + (n - 1), last.p);
-    FG_CHECK_LAUNCH();
-  }
-  exclusive_scan_rec(in, out, n, s);
-  write_total_kernel<<<1, 32, 0, s>>>(out, n, last.p, n > 0);
-  FG_CHECK_LAUNCH();
-}
+void exclusive_scan_async(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s) { scan<false>(in, out, n, s); }
 
 int64_t exclusive_scan(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s) {
   exclusive_scan_async(in, out, n, s);
   return (int64_t)read_scalar(out + n, s);
 }
 
-void inclusive_scan_inplace(int32_t* a, int64_t n, cudaStream_t s) {
-  if (n <= 0) return;
-  DBuf<int32_t> tmp(n + 1, s);
-  exclusive_scan_async(a, tmp.p, n, s);
-  // inclusive[i] = exclusive[i+1]
-  FG_CUDA(cudaMemcpyAsync(a, tmp.p + 1, n * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
-}
+void inclusive_scan(const int32_t* in, int32_t* out, int64_t n, cudaStream_t s) { scan<true>(in, out, n, s); }
 
 void reduce_max_async(const int32_t* a, int64_t n, int32_t* out, cudaStream_t s) {
-  fill_i32(out, 1, INT32_MIN, s);
-  if (n > 0) {
-    reduce_max_kernel<<<reduce_grid(n), 256, 0, s>>>(a, n, out);
-    FG_CHECK_LAUNCH();
+  if (n <= kScanOne) {
+    FG_RUN(reduce_max_one_kernel<<<1, 1024, 0, s>>>(a, n, out));
+    return;
   }
+  fill_i32(out, 1, INT32_MIN, s);
+  FG_RUN(reduce_max_kernel<<<reduce_grid(n), 256, 0, s>>>(a, n, out));
 }
 
 int32_t reduce_max(const int32_t* a, int64_t n, cudaStream_t s) {
   DBuf<int32_t> out(1, s);
-  fill_i32(out.p, 1, INT32_MIN, s);
-  if (n > 0) {
-    reduce_max_kernel<<<reduce_grid(n), 256, 0, s>>>(a, n, out.p);
-    FG_CHECK_LAUNCH();
-  }
+  reduce_max_async(a, n, out.p, s);
   return read_scalar(out.p, s);
 }
 
@@ -334,20 +408,9 @@ void iota_i32(int32_t* a, int64_t n, cudaStream_t s) {
 
 void segmented_sort_i32(int32_t* vals, const int32_t* off, int nseg, int32_t* ucount, cudaStream_t s) {
   if (nseg <= 0) return;
-  DBuf<int32_t> lens(nseg, s);
-  seg_len_kernel<<<grid_for(nseg, 256), 256, 0, s>>>(off, nseg, lens.p);
-  FG_CHECK_LAUNCH();
-  int32_t maxlen = reduce_max(lens.p, nseg, s);
-  segsort_warp_kernel<<<grid_for(nseg, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, s>>>(vals, off, nseg, ucount);
-  FG_CHECK_LAUNCH();
-  if (maxlen > kWarpCap) {
-    segsort_block_kernel<<<nseg, 1024, 0, s>>>(vals, off, nseg, ucount);
-    FG_CHECK_LAUNCH();
-  }
-  if (maxlen > kBlockCap) {
-    segsort_serial_kernel<<<grid_for(nseg, 128), 128, 0, s>>>(vals, off, nseg, ucount);
-    FG_CHECK_LAUNCH();
-  }
+  FG_RUN(segsort_warp_kernel<<<grid_for(nseg, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, s>>>(vals, off, nseg, ucount));
+  const int64_t blocks = ((int64_t)nseg + 1023) / 1024;
+  FG_RUN(segsort_long_kernel<<<(int)(blocks < 152 * 4 ? blocks : 152 * 4), 1024, 0, s>>>(vals, off, nseg, ucount));
 }
 
 }  // namespace femgpu

@@ -49,3 +49,17 @@ def test_assembly_and_load_match_oracle(name, mass):
     assert np.array_equal(grp, rp) and np.array_equal(gci, ci)
     assert np.array_equal(gv, O.assemble(xyz, conn, rp, ci, coef=coef, lambda_mass=mass))
     assert np.array_equal(b, O.load_vector(xyz, conn, f))
+
+
+@pytest.mark.parametrize("mesh", [("square", 89), ("square", 90), ("square", 127), ("square", 128), ("square", 180),
+                                  ("fan", 341), ("fan", 342), ("fan", 2730), ("fan", 2731)])
+def test_pattern_at_scan_and_sort_limits(mesh):
+    # vertex counts around one and two scan tiles (8100, 8281, 16384, 16641) and beyond;
+    # candidate lists around the warp's and the block's sort capacity (1024 and 8192 / 3)
+    xyz, conn = meshes.jittered_square(mesh[1]) if mesh[0] == "square" else fan(mesh[1])
+    rp, ci = O.build_pattern(xyz.shape[0], conn)
+    with femgpu.Solver() as s:
+        s.set_mesh(xyz, conn)
+        s.assemble(None, 1.0)
+        grp, gci, _ = s.matrix()
+    assert np.array_equal(grp, rp) and np.array_equal(gci, ci)
