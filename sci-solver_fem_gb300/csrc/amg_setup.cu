@@ -24,7 +24,11 @@
 #include <limits>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "context.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace femgpu {
 
@@ -1970,65 +1974,335 @@ __global__ void dense_lu_kernel(int n, double* F, int32_t* piv, int32_t* status)
   }
 }
 
-// The same factorization with the matrix in shared memory (n * n doubles), one block:
-// warp 0 finds the pivot (first maximal |a| in row order), every thread then swaps,
-// scales and updates the trailing block.  Identical arithmetic to dense_lu_kernel.
-__global__ void __launch_bounds__(1024) dense_lu_smem_kernel(int n, double* F, int32_t* piv, int32_t* status) {
-  extern __shared__ double sf[];
-  __shared__ int s_p;
-  __shared__ double s_pb;
-  for (int q = threadIdx.x; q < n * n; q += blockDim.x) sf[q] = F[q];
+// The same factorisation on a cluster of kLuCluster CTAs, the matrix in their shared memory
+// (n <= kLuMax).  Columns go to the CTAs in panels of kLuPanel (panel p to CTA p mod
+// kLuCluster).  Per panel: its CTA factorises it (a thread per row, the row's entries in
+// registers) and writes it into every CTA's shared memory; after one cluster barrier each
+// CTA applies its row exchanges to its own columns and updates the columns on the right,
+// first the panel's rows, then the rows below.  Every entry receives the same
+// updates in the same order (k ascending) as in dense_lu_kernel, so the factors keep their
+// bits; the matrix is read from CSR and the factors leave column by column, as the inverse
+// reads them.  Row exchanges leave as pos[j], the row where the unit entry of e_j ends.
+// Bound by the panels' chains (pivot search, division) and by the FP64 pipe: one SM has 2
+// FP64 units, so one block spends n^3 / 6 cycles on the updates alone; eight CTAs share
+// them.  105 rows: 340 -> 152 us; 2D 64^2: 46 -> 28 us.
+constexpr int kLuCluster = 8;
+constexpr int kLuPanel = 8;
+constexpr int kLuMax = 392;  // the CTA's columns and two panels: 225,792 bytes
+constexpr int kLuThreads = 512;
+
+inline size_t lu_smem_bytes(int n) {
+  const int panels = (n + kLuPanel - 1) / kLuPanel, own = (panels + kLuCluster - 1) / kLuCluster;
+  return (size_t)(own + 2) * kLuPanel * n * sizeof(double);
+}
+
+// (key, row) with the largest key, lowest row first, over the warp.
+__device__ __forceinline__ void warp_first_max(unsigned long long& key, int& row) {
+  const unsigned hi = (unsigned)(key >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = hi == mh ? (unsigned)key : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
+  const bool top = hi == mh && (unsigned)key == ml;
+  row = (int)__reduce_min_sync(0xffffffffu, top ? (unsigned)row : 0xffffffffu);
+  key = (unsigned long long)mh << 32 | ml;
+}
+
+template <class T>
+__global__ void __launch_bounds__(kLuThreads) dense_lu_cluster_kernel(int n, const int32_t* __restrict__ rp,
+                                                                      const int32_t* __restrict__ ci,
+                                                                      const T* __restrict__ v,
+                                                                      double* __restrict__ Fc,
+                                                                      int32_t* __restrict__ pos, int32_t* status) {
+  extern __shared__ __align__(16) double lu_sm[];
+  __shared__ unsigned long long s_key[32];
+  __shared__ int s_row[32];
+  __shared__ double s_prow[kLuPanel], s_krow[kLuPanel];
+  __shared__ int s_piv[kLuMax + kLuPanel];  // every pivot so far
+  __shared__ int s_bad;                     // a panel's owner met a zero pivot
+  cg::cluster_group cl = cg::this_cluster();
+  const int me = (int)cl.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int panels = (n + kLuPanel - 1) / kLuPanel;
+  const int own = me < panels ? (panels - me + kLuCluster - 1) / kLuCluster : 0;  // own panels
+  double* const cols = lu_sm;  // local column l: rows at cols + l n; l = 8 (panel / 8) + column in panel
+  // the current panel, written by its owner; two, so that an owner may write its panel while
+  // another CTA still reads the one before
+  double* const Lb0 = lu_sm + (size_t)((panels + kLuCluster - 1) / kLuCluster) * kLuPanel * n;
+  for (int q = tid; q < own * kLuPanel * n; q += kLuThreads) cols[q] = 0.0;
+  if (tid == 0) s_bad = 0;
+  cl.sync();  // every CTA is running before another writes its shared memory
+  for (int i = warp; i < n; i += kLuThreads / 32)
+    for (int e = rp[i] + lane; e < rp[i + 1]; e += 32) {
+      const int j = ci[e], p = j / kLuPanel;
+      if (p % kLuCluster == me) cols[(size_t)((p / kLuCluster) * kLuPanel + j % kLuPanel) * n + i] = (double)v[e];
+    }
   __syncthreads();
-  for (int k = 0; k < n; k++) {
-    if (threadIdx.x < 32) {
-      double best = -1.0;
-      int bi = n;
-      for (int i = k + (int)threadIdx.x; i < n; i += 32) {
-        const double a = fabs(sf[i * n + k]);
-        if (a > best) {  // rows visited in ascending order per lane
-          best = a;
-          bi = i;
-        }
-      }
+  const int nt = (n + 31) / 32 * 32;  // threads of the panel factorisation
+  bool bad = false;
+  for (int p = 0; p < panels; p++) {
+    const int owner = p % kLuCluster, k0 = p * kLuPanel, nk = min(kLuPanel, n - k0);
+    double* const Lb = Lb0 + (size_t)(p & 1) * kLuPanel * n;
+    if (me == owner && tid < nt) {
+      double* const pan = cols + (size_t)(p / kLuCluster) * kLuPanel * n;
+      double a[kLuPanel];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
+      for (int c = 0; c < kLuPanel; c++) a[c] = tid < n ? pan[(size_t)c * n + tid] : 0.0;
+      bool ok = true;
+#pragma unroll
+      for (int kk = 0; kk < kLuPanel; kk++) {
+        const int k = k0 + kk;
+        if (kk < nk && ok) {
+          // first maximal |a| at or below the diagonal: magnitudes order like their bits; 0
+          // stands for rows above and for NaN, 1 for a zero
+          // (integer compares: a floating-point one would take the FP64 pipe)
+          unsigned long long key = (unsigned long long)__double_as_longlong(a[kk]) & 0x7fffffffffffffffull;
+          key = tid >= k && tid < n && key <= 0x7ff0000000000000ull ? key + 1 : 0;
+          int row = tid;
+          warp_first_max(key, row);
+          if (lane == 0) {
+            s_key[warp] = key;
+            s_row[warp] = row;
+          }
+          asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
+          key = lane < nt / 32 ? s_key[lane] : 0;
+          row = lane < nt / 32 ? s_row[lane] : 0x7fffffff;
+          warp_first_max(key, row);
+          ok = key > 1;
+          if (ok) {
+            if (tid == row)
+#pragma unroll
+              for (int c = 0; c < kLuPanel; c++) s_prow[c] = a[c];
+            if (tid == k)
+#pragma unroll
+              for (int c = 0; c < kLuPanel; c++) s_krow[c] = a[c];
+            asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
+            double pr[kLuPanel];
+#pragma unroll
+            for (int c = 0; c < kLuPanel; c++) pr[c] = s_prow[c];
+            if (tid == row && row != k)
+#pragma unroll
+              for (int c = 0; c < kLuPanel; c++) a[c] = s_krow[c];
+            if (tid == k)
+#pragma unroll
+              for (int c = 0; c < kLuPanel; c++) a[c] = pr[c];
+            if (tid > k) {
+              // a zero (padding rows, sparse columns) keeps its warp out of the division's
+              // slow path: +-0 / d is a zero of the product's sign
+              const long long ab = __double_as_longlong(a[kk]);
+              if ((ab << 1) != 0) a[kk] = a[kk] / pr[kk];
+              else a[kk] = __longlong_as_double(ab ^ (__double_as_longlong(pr[kk]) & (1ll << 63)));
+#pragma unroll
+              for (int c = kk + 1; c < kLuPanel; c++) a[c] = fma(-a[kk], pr[c], a[c]);
+            }
+            if (tid < kLuCluster) *cl.map_shared_rank(&s_piv[k], tid) = row;
+          } else if (tid < kLuCluster) {
+            *cl.map_shared_rank(&s_bad, tid) = 1;
+          }
         }
       }
-      if (threadIdx.x == 0) {
-        s_p = bi;
-        s_pb = best;
+      if (tid < n) {
+#pragma unroll
+        for (int c = 0; c < kLuPanel; c++) pan[(size_t)c * n + tid] = a[c];
+        if (tid >= k0)
+          for (int d = 0; d < kLuCluster; d++) {
+            double* const dst = cl.map_shared_rank(Lb, d);
+#pragma unroll
+            for (int c = 0; c < kLuPanel; c++) dst[c * n + tid] = a[c];
+          }
       }
     }
-    __syncthreads();
-    const int p = s_p;
-    if (s_pb == 0.0) {
-      if (threadIdx.x == 0) *status = 1;
-      return;
-    }
-    if (threadIdx.x == 0) piv[k] = p;
-    if (p != k)
-      for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const double t = sf[k * n + j];
-        sf[k * n + j] = sf[p * n + j];
-        sf[p * n + j] = t;
+    cl.sync();  // the panel is everywhere; every CTA is done with the panel before it
+    bad = s_bad != 0;
+    if (bad) break;
+    // own columns outside the panel, eight lanes each: the panel's row exchanges, then (right
+    // of the panel) the panel's rows
+    const int r = tid & 7;
+    for (int l0 = warp * 4; l0 < own * kLuPanel; l0 += kLuThreads / 8) {
+      const int l = l0 + (lane >> 3), gp = me + (l / kLuPanel) * kLuCluster;  // global panel
+      const bool live = l < own * kLuPanel && gp != p;
+      double* const col = cols + (size_t)l * n;
+      if (live && r == 0)
+        for (int kk = 0; kk < nk; kk++) {
+          const int pv = s_piv[k0 + kk];
+          if (pv != k0 + kk) {
+            const double t = col[k0 + kk];
+            col[k0 + kk] = col[pv];
+            col[pv] = t;
+          }
+        }
+      __syncwarp();
+      const bool right = live && gp > p;
+      double x = right && r < nk ? col[k0 + r] : 0.0;
+#pragma unroll
+      for (int kk = 0; kk < kLuPanel; kk++) {
+        const double u = __shfl_sync(0xffffffffu, x, kk, 8);
+        if (right && kk < r && r < nk) x = fma(-Lb[kk * n + k0 + r], u, x);
       }
+      if (right && r < nk) col[k0 + r] = x;
+    }
     __syncthreads();
-    const double d = sf[k * n + k];
-    for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) sf[i * n + k] = sf[i * n + k] / d;
-    __syncthreads();
-    const int m = n - k - 1;
-    for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
-      const int i = k + 1 + q / m, j = k + 1 + q % m;
-      sf[i * n + j] = fma(-sf[i * n + k], sf[k * n + j], sf[i * n + j]);
+    // rows below the panel of the own columns right of it (a right column exists only when
+    // the panel is full): one warp per column and 32 rows
+    const int first = p < me ? 0 : (p - me) / kLuCluster + 1;  // first own panel right of p
+    const int ncol = (own - first) * kLuPanel, i0 = k0 + kLuPanel;
+    const int chunks = (n - i0 + 31) / 32;
+    for (int t = warp; t < ncol * chunks; t += kLuThreads / 32) {
+      double* const col = cols + (size_t)(first * kLuPanel + t / chunks) * n;
+      const int i = i0 + (t % chunks) * 32 + lane;
+      if (i < n) {
+        double x = col[i];
+#pragma unroll
+        for (int kk = 0; kk < kLuPanel; kk++) x = fma(-Lb[kk * n + i], col[k0 + kk], x);
+        col[i] = x;
+      }
     }
     __syncthreads();
   }
-  for (int q = threadIdx.x; q < n * n; q += blockDim.x) F[q] = sf[q];
+  if (bad) {
+    if (me == 0 && tid == 0) *status = 1;
+  } else {
+    for (int q = tid; q < own * kLuPanel * n; q += kLuThreads) {
+      const int l = q / n, j = (me + (l / kLuPanel) * kLuCluster) * kLuPanel + l % kLuPanel;
+      if (j < n) Fc[(size_t)j * n + q % n] = cols[q];
+    }
+    if (me == 0 && tid < n) {
+      int at = tid;
+      for (int k = 0; k < n; k++) {
+        const int pv = s_piv[k];
+        at = at == k ? pv : at == pv ? k : at;
+      }
+      pos[tid] = at;
+    }
+  }
+  cl.sync();  // no CTA leaves while another may still read its shared memory
+}
+
+// Column j of the inverse from the factors of dense_lu_cluster_kernel, one warp per column,
+// row i in lane i mod 32, register i / 32: the operations of dense_inverse_kernel in the same
+// order, with the factors' columns loaded G steps ahead.  Bound by the chain of 2 n steps
+// (a shuffle and a fused multiply-add each, and a division in the back substitution).
+// 107 rows: 133 -> 101 us.
+// Division by d with y = 1 / d at hand (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990): s y corrected once is within one ulp of s / d,
+// its remainder is exact, and a second correction with the correctly rounded reciprocal y
+// rounds s / d correctly, unless d's significand is all ones.  That d, and operands whose
+// remainders could leave the normal range, take the division itself; a zero s keeps s y.
+__device__ __forceinline__ bool recip_usable(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d) & 0x7fffffffu, lo = (unsigned)__double2loint(d);
+  return hi - 0x20000000u < 0x3fe00000u && !((hi & 0xfffffu) == 0xfffffu && lo == 0xffffffffu);
+}
+__device__ __forceinline__ double div_by_recip(double s, double d, double y, bool usable) {
+  const unsigned hi = (unsigned)__double2hiint(s) & 0x7fffffffu;
+  const double q0 = s * y;
+  if (usable && hi - 0x20000000u < 0x3fe00000u) {
+    const double q1 = fma(fma(-d, q0, s), y, q0);
+    return fma(fma(-d, q1, s), y, q1);
+  }
+  if (usable && (hi | (unsigned)__double2loint(s)) == 0u) return q0;
+  return s / d;
+}
+
+template <int R, int G>
+__global__ void __launch_bounds__(32) dense_inverse_warp_kernel(int n, const double* __restrict__ Fc,
+                                                                const int32_t* __restrict__ pos,
+                                                                const int32_t* __restrict__ status,
+                                                                double* __restrict__ inv) {
+  if (*status != 0) return;
+  const int j = blockIdx.x, lane = threadIdx.x;
+  const int at = pos[j];
+  double x[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) x[r] = lane + 32 * r == at ? 1.0 : 0.0;
+  double f[G][R];
+  // forward: column q of L, q ascending
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    auto load = [&](int g, int q) {
+#pragma unroll
+      for (int s = r; s < R; s++) {
+        const int i = lane + 32 * s;
+        f[g][s] = (q < n && i < n) ? Fc[(size_t)q * n + i] : 0.0;
+      }
+    };
+#pragma unroll
+    for (int g = 0; g < G; g++) load(g, 32 * r + g);
+    for (int l0 = 0; l0 < 32 && 32 * r + l0 < n; l0 += G) {
+#pragma unroll
+      for (int g = 0; g < G; g++) {
+        const int q = 32 * r + l0 + g;
+        const double b = __shfl_sync(0xffffffffu, x[r], l0 + g);
+        if (q < n) {
+#pragma unroll
+          for (int s = r; s < R; s++)
+            if (lane + 32 * s > q) x[s] = fma(-f[g][s], b, x[s]);
+        }
+        if (l0 + G < 32) load(g, q + G);
+      }
+    }
+  }
+  // back: column q of U, q descending; x_q is divided by the diagonal first
+  double y[R];  // reciprocals of the diagonal of this lane's rows
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const int i = lane + 32 * r;
+    y[r] = i < n ? 1.0 / Fc[(size_t)i * n + i] : 1.0;
+  }
+#pragma unroll
+  for (int r = R - 1; r >= 0; r--) {
+    auto load = [&](int g, int q) {
+#pragma unroll
+      for (int s = 0; s <= r; s++) {
+        const int i = lane + 32 * s;
+        f[g][s] = (q < n && i < n) ? Fc[(size_t)q * n + i] : 1.0;
+      }
+    };
+#pragma unroll
+    for (int g = 0; g < G; g++) load(g, 32 * r + 31 - g);
+    for (int l0 = 31; l0 >= 0; l0 -= G) {
+#pragma unroll
+      for (int g = 0; g < G; g++) {
+        const int l = l0 - g, q = 32 * r + l;
+        if (q < n) {  // the same for the whole warp
+          if (lane == l) x[r] = div_by_recip(x[r], f[g][r], y[r], recip_usable(f[g][r]));
+          const double b = __shfl_sync(0xffffffffu, x[r], l);
+#pragma unroll
+          for (int s = r; s >= 0; s--)  // the next step's register first
+            if (lane + 32 * s < q) x[s] = fma(-f[g][s], b, x[s]);
+        }
+        if (l0 - G >= 0) load(g, q - G);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; r++)
+    if (lane + 32 * r < n) inv[(size_t)(lane + 32 * r) * n + j] = x[r];
+}
+
+// The explicit inverse of a coarsest matrix of at most kLuMax rows; *status is set when it
+// is singular.
+template <class T>
+void dense_inverse(cudaStream_t s, int n, const int32_t* rp, const int32_t* ci, const T* v, double* F, int32_t* pos,
+                   int32_t* status, double* inv) {
+  const size_t smem = lu_smem_bytes(n);
+  auto lu = dense_lu_cluster_kernel<T>;
+  ensure_dynamic_smem(reinterpret_cast<const void*>(lu), smem);  // with the static arrays it may pass 48 KB first
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kLuCluster);
+  cfg.blockDim = dim3(kLuThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kLuCluster;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  FG_CUDA(cudaLaunchKernelEx(&cfg, lu, n, rp, ci, v, F, pos, status));
+  auto iv = n <= 64    ? dense_inverse_warp_kernel<2, 8>
+            : n <= 128 ? dense_inverse_warp_kernel<4, 8>
+            : n <= 256 ? dense_inverse_warp_kernel<8, 4>
+                       : dense_inverse_warp_kernel<14, 2>;
+  FG_LAUNCH(iv, n, 32, 0, s, n, F, pos, status, inv);
 }
 
 // Column j of the inverse (block j): solve L U x = P e_j column by column, so each
@@ -2247,27 +2521,27 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
       L.coarsest = true;
       DBuf<double> F((size_t)N * N, s);
       DBuf<int32_t> piv(N, s), st(1, s);
-      F.zero();
       st.zero();
-      if (L.A64v.n)  // formed in FP64: the dense factorisation takes those values
-        FG_LAUNCH(densify_kernel<double>, grid_for(N, 128), 128, 0, s, N, L.A.rp.p, L.A.ci.p, L.A64v.p, F.p);
-      else
-        FG_LAUNCH(densify_kernel<T>, grid_for(N, 128), 128, 0, s, N, L.A.rp.p, L.A.ci.p, L.A.v.p, F.p);
-      const size_t fbytes = (size_t)N * N * sizeof(double);
-      if (fbytes <= 200 * 1024) {
-        if (fbytes > 48 * 1024)
-          ensure_smem(dense_lu_smem_kernel, fbytes);
-        FG_LAUNCH(dense_lu_smem_kernel, 1, 1024, fbytes, s, N, F.p, piv.p, st.p);
-      } else {
-        FG_LAUNCH(dense_lu_kernel, 1, 1024, 0, s, N, F.p, piv.p, st.p);
-      }
-      FG_REQUIRE(read_scalar(st.p, s) == 0, FEMGPU_ERR_BREAKDOWN, "coarsest matrix is singular");
       L.Ainv.alloc((size_t)N * N, s);
-      const size_t bbytes = (size_t)N * sizeof(double);
-      if (bbytes > 48 * 1024)
-        ensure_smem(dense_inverse_kernel, bbytes);
-      FG_LAUNCH(dense_inverse_kernel, N, std::min(1024, std::max(32, (N + 31) / 32 * 32)), bbytes, s, N, F.p, piv.p,
-                L.Ainv.p);
+      if (N <= kLuMax) {
+        if (L.A64v.n)  // formed in FP64: the dense factorisation takes those values
+          dense_inverse<double>(s, N, L.A.rp.p, L.A.ci.p, L.A64v.p, F.p, piv.p, st.p, L.Ainv.p);
+        else
+          dense_inverse<T>(s, N, L.A.rp.p, L.A.ci.p, L.A.v.p, F.p, piv.p, st.p, L.Ainv.p);
+        FG_REQUIRE(read_scalar(st.p, s) == 0, FEMGPU_ERR_BREAKDOWN, "coarsest matrix is singular");
+      } else {
+        F.zero();
+        if (L.A64v.n)
+          FG_LAUNCH(densify_kernel<double>, grid_for(N, 128), 128, 0, s, N, L.A.rp.p, L.A.ci.p, L.A64v.p, F.p);
+        else
+          FG_LAUNCH(densify_kernel<T>, grid_for(N, 128), 128, 0, s, N, L.A.rp.p, L.A.ci.p, L.A.v.p, F.p);
+        FG_LAUNCH(dense_lu_kernel, 1, 1024, 0, s, N, F.p, piv.p, st.p);
+        FG_REQUIRE(read_scalar(st.p, s) == 0, FEMGPU_ERR_BREAKDOWN, "coarsest matrix is singular");
+        const size_t bbytes = (size_t)N * sizeof(double);
+        if (bbytes > 48 * 1024) ensure_smem(dense_inverse_kernel, bbytes);
+        FG_LAUNCH(dense_inverse_kernel, N, std::min(1024, std::max(32, (N + 31) / 32 * 32)), bbytes, s, N, F.p, piv.p,
+                  L.Ainv.p);
+      }
       L.b.alloc(N, s);
       L.x.alloc(N, s);
       break;
