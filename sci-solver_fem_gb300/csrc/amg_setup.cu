@@ -91,7 +91,7 @@ __device__ __forceinline__ uint32_t taus(uint32_t z) {
 }
 
 // ---- randomized MIS (randomizedMIS_GPU.cu:3-152) ---------------------------------
-__global__ void mis_randoms_kernel(int n, int iterations, uint32_t* randoms, const uint32_t* seeds) {
+__global__ void mis_randoms_kernel(int n, int iterations, uint32_t* randoms, const uint32_t* __restrict__ seeds) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 32768) return;
   uint32_t z = seeds[t];
@@ -161,23 +161,34 @@ __global__ void mis_iterate_kernel(int n, const uint64_t* __restrict__ kin, uint
   }
 }
 
+// The 32768 generator seeds of cfg.seed, made once per handle and seed.
+const uint32_t* mis_seeds(Ctx& c) {
+  if (c.mis_seeds.n == 0 || c.mis_seeds_of != c.cfg.seed) {
+    std::vector<uint32_t> seeds;
+    glibc_rand_stream(c.cfg.seed, 32768, seeds);
+    c.mis_seeds.alloc(32768, c.stream);
+    c.mis_seeds.upload(seeds.data(), 32768);
+    FG_CUDA(cudaStreamSynchronize(c.stream));  // the host copy ends here
+    c.mis_seeds_of = c.cfg.seed;
+  }
+  return c.mis_seeds.p;
+}
+
 void random_mis(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int k, DBuf<int32_t>& mis) {
   cudaStream_t s = c.stream;
   PhaseTimer pt(s, -5);
   mis.alloc(n, s);
   fill_i32(mis.p, n, -1, s);
-  std::vector<uint32_t> seeds;
-  glibc_rand_stream(c.cfg.seed, 32768, seeds);
-  DBuf<uint32_t> dseeds(32768, s), randoms(n, s);
-  dseeds.upload(seeds.data(), 32768);
+  const uint32_t* seeds = mis_seeds(c);
+  DBuf<uint32_t> randoms(n, s);
   DBuf<uint64_t> k0(n, s), k1(n, s);
   DBuf<int32_t> flag(1, s);
-  FG_LAUNCH(mis_randoms_kernel, 128, 256, 0, s, n, (n + 32767) / 32768, randoms.p, dseeds.p);
+  FG_LAUNCH(mis_randoms_kernel, 128, 256, 0, s, n, (n + 32767) / 32768, randoms.p, seeds);
   FG_LAUNCH(mis_first_init_kernel, grid_for(n, 256), 256, 0, s, n, randoms.p, k0.p);
   pt.mark("mis init");
-  // Rounds are enqueued in batches and the flag of a batch's last round is read once:
-  // a round after the one that completes the set changes nothing (decided nodes keep
-  // their state), so the extra rounds only cost time.  Small levels, where a host
+  // Rounds are enqueued in batches and the flag of a batch's last round is read once: a
+  // round after the one that completes the set changes nothing (decided nodes keep their
+  // state), so the extra rounds only cost time.  Small levels, where a host
   // round trip costs more than a round, take larger batches.
   const int batch = n < (1 << 18) ? 4 : 2;
   for (int round = 0;; round++) {
@@ -272,17 +283,20 @@ __global__ void remove_parts_kernel(int n, int32_t* part, const int32_t* rm, con
   }
 }
 
-// findDesirabilityKernel (misHelpers.cu:297-382) with IEEE float steps spelled out.
-__global__ void desirability_kernel(int n, int opt, const int32_t* __restrict__ xadj, const int32_t* __restrict__ adj,
-                                    const int32_t* __restrict__ part, const int32_t* __restrict__ sizes,
-                                    const int32_t* __restrict__ w, int32_t* to,
-                                    unsigned long long* best /* per partition: (desirability bits, node) */) {
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= n) return;
-  int cur = part[idx];
-  int cs = sizes[cur];
+// findDesirabilityKernel (misHelpers.cu:297-382) with IEEE float steps spelled out: the
+// partition node idx would move to, and the packed (desirability, node) key of the move.
+// L2: part and sizes are written by other CTAs of the running kernel (read past L1).
+template <bool L2>
+__device__ __forceinline__ unsigned long long desirability(int idx, int opt, const int32_t* __restrict__ xadj,
+                                                           const int32_t* __restrict__ adj, const int32_t* part,
+                                                           const int32_t* sizes, const int32_t* __restrict__ w,
+                                                           int& cur, int& addTo) {
+  auto ld = [](const int32_t* p) { return L2 ? __ldcg(p) : *p; };
+  cur = ld(part + idx);
+  int cs = ld(sizes + cur);
   int nw = w[idx];
-  int selfAdj = 0, addTo = -1;
+  int selfAdj = 0;
+  addTo = -1;
   float bestD = 0.0f;
   float cwf = __fdiv_rn((float)abs(cs - opt), (float)opt);
   float selfImp = __fmul_rn((float)(abs(cs - opt) - abs((cs - nw) - opt)), cwf);
@@ -293,24 +307,31 @@ __global__ void desirability_kernel(int n, int opt, const int32_t* __restrict__ 
       cand[q] = -1;
       cnt[q] = 0;
     }
-    for (int e = xadj[idx]; e < xadj[idx + 1]; e++) {
-      int cc = part[adj[e]];
-      if (cc == cur) {
-        selfAdj++;
-        continue;
-      }
-      // distinct candidates in first-seen order, at most 10 (junk counts of free
-      // slots in the reference never reach a used slot)
+    // neighbours in groups of 8: all indices, then all parts, so the loads overlap
+    const int e1 = xadj[idx + 1];
+    for (int e0 = xadj[idx]; e0 < e1; e0 += 8) {
+      int nb[8], pc[8];
 #pragma unroll
-      for (int q = 0; q < 10; q++) {
-        if (cand[q] == cc) {
-          cnt[q]++;
-          break;
+      for (int u = 0; u < 8; u++) nb[u] = e0 + u < e1 ? adj[e0 + u] : idx;
+#pragma unroll
+      for (int u = 0; u < 8; u++) pc[u] = e0 + u < e1 ? ld(part + nb[u]) : -1;
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int cc = pc[u];
+        if (cc == -1) continue;  // past the list's end (every node has a part)
+        if (cc == cur) {
+          selfAdj++;
+          continue;
         }
-        if (cand[q] == -1) {
-          cand[q] = cc;
-          cnt[q] = 1;
-          break;
+        // distinct candidates in first-seen order, at most 10 (junk counts of free
+        // slots in the reference never reach a used slot)
+        bool placed = false;
+#pragma unroll
+        for (int q = 0; q < 10; q++) {
+          const bool here = !placed && (cand[q] == cc || cand[q] == -1);
+          cnt[q] += here;
+          if (here) cand[q] = cc;
+          placed |= here;
         }
       }
     }
@@ -319,7 +340,7 @@ __global__ void desirability_kernel(int n, int opt, const int32_t* __restrict__ 
     for (int q = 1; q < 10; q++) {
       if (cand[q] == -1) continue;
       int np_ = cand[q];
-      int nsz = sizes[np_];
+      int nsz = ld(sizes + np_);
       float nwf = __fdiv_rn((float)abs(nsz - opt), (float)opt);
       float imp = __fmul_rn((float)(abs(nsz - opt) - abs((nsz + nw) - opt)), nwf);
       imp = __fadd_rn(imp, selfImp);
@@ -331,8 +352,18 @@ __global__ void desirability_kernel(int n, int opt, const int32_t* __restrict__ 
       }
     }
   }
-  to[idx] = addTo;
-  unsigned long long key = ((unsigned long long)__float_as_uint(bestD) << 32) | (unsigned)idx;
+  return ((unsigned long long)__float_as_uint(bestD) << 32) | (unsigned)idx;
+}
+
+__global__ void desirability_kernel(int n, int opt, const int32_t* __restrict__ xadj, const int32_t* __restrict__ adj,
+                                    const int32_t* __restrict__ part, const int32_t* __restrict__ sizes,
+                                    const int32_t* __restrict__ w, int32_t* to,
+                                    unsigned long long* best /* per partition: (desirability bits, node) */) {
+  int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= n) return;
+  int cur, add;
+  const unsigned long long key = desirability<false>(idx, opt, xadj, adj, part, sizes, w, cur, add);
+  to[idx] = add;
   atomicMax(&best[cur], key);
 }
 
@@ -400,12 +431,386 @@ int restrict_partitions(Ctx& c, int max_size, int full_size, int n, const int32_
   return np;
 }
 
-// aggregateGraph / aggregateWeightedGraph (misHelpers.cu:513-677).  Returns the number
-// of parts for the unweighted graph (the parts are labelled 0 .. count-1), -1 for the
-// weighted one (whose partition restriction may empty a part).
-int aggregate(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int depth, bool weighted, int min_size,
-              int max_size, int full_size, const int32_t* weights, DBuf<int32_t>& part) {
+[[noreturn]] void throw_stalled() {
+  throw Error(FEMGPU_ERR_LIMIT,
+              "aggregation stalled: nodes unreachable from any aggregate, or every aggregate was removed "
+              "as undersized");
+}
+
+// ---- aggregation of small graphs in one kernel ------------------------------------------
+// The whole of aggregate() below (MIS rounds, labels, allocation passes, removal of small
+// parts, partition restriction) for a graph of at most kClusterAggEdges edges, as one
+// thread-block cluster: CTA c owns a contiguous range of the nodes (and of the parts), the
+// arrays stay in L2, and what ended a launch or a read by the host is a cluster barrier
+// (0.3 us).  As separate launches these graphs are bound by launches (2.5-4 us each, 25-60 of
+// them) and by the flags the host reads (12-20 us each, 5-10 of them).  Every step computes
+// what its kernel computes, so the labels are the same.
+// The line is drawn by edges, whose gathers the cluster's 16 SMs must do alone (ms per call,
+// launches against cluster): 1,590 nodes 0.33 / 0.14; 39,304 nodes with 0.53 M edges 0.49 /
+// 0.42; 90,601 nodes with 0.54 M edges 0.60 / 0.30; 80,338 nodes with 1.2 M edges 0.49 / 0.77;
+// 132,651 nodes with 1.8 M edges 0.60 / 1.30.
+constexpr int kAggThreads = 1024;
+constexpr int kAggCtas = 16;  // largest cluster (8 where 16 cannot be scheduled)
+constexpr int64_t kClusterAggEdges = 600000;
+
+enum AggStatus { AGG_OK = 0, AGG_MIS_CAP, AGG_LOOP_CAP, AGG_RESTRICT_CAP, AGG_STALLED };
+
+struct AggArgs {
+  int n;
+  const int32_t *xadj, *adj, *w;  // w: node weights (weighted graph), else null
+  const uint32_t* seeds;
+  int depth, min_size, max_size, full_size;
+  uint32_t* rnd;                // n
+  unsigned long long *k0, *k1;  // n each; k0 also holds the partitions' best moves
+  int32_t *mis, *part, *pout, *sizes, *map, *to;  // n each
+  int32_t* res;  // status, parts after the removals, largest label + 1, 1 when the labels are in pout
+};
+
+// Exchanges one value per CTA; v[r] = CTA r's value on return.  Two buffers: a value is
+// overwritten two exchanges later, when every CTA has passed the barrier between.
+struct ClusterExchange {
+  int (*buf)[kAggCtas];
+  int turn = 0, C, me;
+  __device__ const int* operator()(cg::cluster_group& cl, int value) {
+    __syncthreads();
+    if ((int)threadIdx.x < C) *cl.map_shared_rank(&buf[turn][me], threadIdx.x) = value;
+    cl.sync();
+    const int* v = buf[turn];
+    turn ^= 1;
+    return v;
+  }
+  __device__ int sum(cg::cluster_group& cl, int value) {
+    const int* v = (*this)(cl, value);
+    int t = 0;
+    for (int r = 0; r < C; r++) t += v[r];
+    return t;
+  }
+  __device__ int max(cg::cluster_group& cl, int value) {
+    const int* v = (*this)(cl, value);
+    int t = v[0];
+    for (int r = 1; r < C; r++) t = ::max(t, v[r]);
+    return t;
+  }
+  // (sum of the lower CTAs' values, sum of all)
+  __device__ int2 prefix(cg::cluster_group& cl, int value) {
+    const int* v = (*this)(cl, value);
+    int lower = 0, all = 0;
+    for (int r = 0; r < C; r++) {
+      if (r < me) lower += v[r];
+      all += v[r];
+    }
+    return make_int2(lower, all);
+  }
+};
+
+// Sum (or maximum) of one value per thread; the result in every thread.
+__device__ __forceinline__ int agg_block_sum(int v, int* sh) {
+  v = __reduce_add_sync(0xffffffffu, v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return __reduce_add_sync(0xffffffffu, sh[threadIdx.x & 31]);
+}
+__device__ __forceinline__ int agg_block_max(int v, int* sh) {
+  v = __reduce_max_sync(0xffffffffu, v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return __reduce_max_sync(0xffffffffu, sh[threadIdx.x & 31]);
+}
+// Inclusive prefix of a flag over the block, in thread order; *total gets the block's count.
+__device__ __forceinline__ int agg_block_rank(bool flag, int* sh, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned m = __ballot_sync(0xffffffffu, flag);
+  __syncthreads();
+  if (lane == 0) sh[warp] = __popc(m);
+  __syncthreads();
+  const int mine = sh[lane];
+  *total = (int)__reduce_add_sync(0xffffffffu, mine);
+  const int below = (int)__reduce_add_sync(0xffffffffu, lane < warp ? mine : 0);
+  return below + __popc(m & (0xffffffffu >> (31 - lane)));
+}
+
+// Arrays that other CTAs write are read from L2 (__ldcg): a line of this SM's L1 may be old.
+__global__ void __launch_bounds__(kAggThreads) aggregate_cluster_kernel(AggArgs a) {
+  __shared__ int xbuf[2][kAggCtas];
+  __shared__ int sh[32];
+  cg::cluster_group cl = cg::this_cluster();
+  ClusterExchange x{xbuf};
+  x.C = (int)cl.num_blocks();
+  x.me = (int)cl.block_rank();
+  const int n = a.n, tid = threadIdx.x;
+  const int per = (n + x.C - 1) / x.C, lo = min(n, x.me * per), hi = min(n, lo + per);
+  const int32_t* __restrict__ xadj = a.xadj;
+  const int32_t* __restrict__ adj = a.adj;
+  int status = AGG_OK;
+  // ---- randomized MIS: rounds of `depth` propagations until every node is decided
+  unsigned long long *ki = a.k0, *ko = a.k1;
+  for (int round = 0;; round++) {
+    if (round >= kCap) {
+      status = AGG_MIS_CAP;
+      break;
+    }
+    for (int i = lo + tid; i < hi; i += kAggThreads) {
+      uint32_t z;
+      if (round == 0) {
+        z = a.seeds[i & 32767];
+        for (int t = 0; t <= i >> 15; t++) z = taus(z);
+        ki[i] = mis_key((int32_t)(z % 1000000u), i);
+      } else {
+        z = taus(a.rnd[i]);
+        const int st = a.mis[i];
+        ki[i] = mis_key(st == -1 ? (int32_t)(z % 1000000u) : (st == 1 ? 1000001 : 0), i);
+      }
+      a.rnd[i] = z;
+    }
+    cl.sync();
+    int undecided = 0;
+    for (int it = 0; it < a.depth; it++) {
+      for (int i = lo + tid; i < hi; i += kAggThreads) {
+        unsigned long long k = ki[i];
+        if ((k >> 32) < 1000001u) {
+          const int e1 = xadj[i + 1];
+          for (int e0 = xadj[i]; e0 < e1; e0 += 8) {
+            int nb[8];
+            unsigned long long kn[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) nb[q] = e0 + q < e1 ? adj[e0 + q] : i;
+#pragma unroll
+            for (int q = 0; q < 8; q++) kn[q] = __ldcg(ki + nb[q]);
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+              if ((kn[q] >> 32) > 0u && kn[q] > k) k = kn[q];
+          }
+        }
+        ko[i] = k;
+        if (it == a.depth - 1) {
+          const int best = (int)(k >> 32), org = (int)(uint32_t)k;
+          const int st = org == i ? 1 : best == 1000001 ? 0 : -1;
+          a.mis[i] = st;
+          undecided |= st == -1;
+        }
+      }
+      unsigned long long* t = ki;
+      ki = ko;
+      ko = t;
+      if (it < a.depth - 1) cl.sync();
+    }
+    if (x.sum(cl, __syncthreads_or(undecided)) == 0) break;
+  }
+  // ---- labels: the MIS nodes numbered in order
+  int32_t *pin = a.part, *po = a.pout;
+  int count;
+  {
+    int ones = 0;
+    for (int i = lo + tid; i < hi; i += kAggThreads) ones += a.mis[i] == 1;
+    const int2 pre = x.prefix(cl, agg_block_sum(ones, sh));
+    count = pre.y;
+    int base = pre.x;
+    for (int i0 = lo; i0 < hi; i0 += kAggThreads) {
+      const int i = i0 + tid;
+      const bool root = i < hi && a.mis[i] == 1;
+      int total;
+      const int rank = agg_block_rank(root, sh, &total);
+      if (i < hi) pin[i] = root ? base + rank - 1 : -1;
+      base += total;
+    }
+  }
+  cl.sync();
+  bool first = true;
+  for (int loop = 0; status == AGG_OK; loop++) {
+    if (loop >= kCap) {
+      status = AGG_LOOP_CAP;
+      break;
+    }
+    // ---- allocation passes: each node without a part takes its first labelled neighbour's
+    for (;;) {
+      int left = 0, changed = 0;
+      for (int i = lo + tid; i < hi; i += kAggThreads) {
+        int p = pin[i];
+        if (p == -1) {
+          const int e1 = xadj[i + 1];
+          for (int e0 = xadj[i]; e0 < e1 && p == -1; e0 += 8) {
+            int nb[8], cnd[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) nb[q] = e0 + q < e1 ? adj[e0 + q] : -1;
+#pragma unroll
+            for (int q = 0; q < 8; q++) cnd[q] = nb[q] >= 0 ? __ldcg(pin + nb[q]) : -1;
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+              if (p == -1 && cnd[q] != -1) p = cnd[q];
+          }
+          if (p != -1) changed = 1;
+          else left = 1;
+        }
+        po[i] = p;
+      }
+      int32_t* t = pin;
+      pin = po;
+      po = t;
+      // nodes are left and none joined: bit 0 of any CTA set, bit 1 of none
+      const int* v = x(cl, (__syncthreads_or(left) ? 1 : 0) | (__syncthreads_or(changed) ? 2 : 0));
+      int any = 0;
+      for (int r = 0; r < x.C; r++) any |= v[r];
+      if (!(any & 1)) break;
+      if (!(any & 2)) {
+        status = AGG_STALLED;
+        break;
+      }
+    }
+    if (status != AGG_OK) break;
+    const bool restrict_now = a.w && (!first || count < 10);
+    // ---- sizes (weights) of the parts
+    const int pper = (count + x.C - 1) / x.C, plo = min(count, x.me * pper), phi = min(count, plo + pper);
+    for (int p = plo + tid; p < phi; p += kAggThreads) {
+      a.sizes[p] = 0;
+      if (restrict_now) a.k0[p] = 0ull;
+    }
+    cl.sync();
+    for (int i = lo + tid; i < hi; i += kAggThreads) atomicAdd(&a.sizes[pin[i]], a.w ? a.w[i] : 1);
+    cl.sync();
+    if (restrict_now) {
+      // ---- partitions above max_size give nodes away, one per round
+      const int opt = a.full_size / count;
+      for (int loops = 0;; loops++) {
+        int m = INT32_MIN;
+        for (int p = plo + tid; p < phi; p += kAggThreads) m = max(m, __ldcg(a.sizes + p));
+        if (x.max(cl, agg_block_max(m, sh)) <= a.max_size) break;
+        if (loops >= kCap) {
+          status = AGG_RESTRICT_CAP;
+          break;
+        }
+        for (int i = lo + tid; i < hi; i += kAggThreads) {
+          int cur, add;
+          const unsigned long long key = desirability<true>(i, opt, xadj, adj, pin, a.sizes, a.w, cur, add);
+          a.to[i] = add;
+          atomicMax(&a.k0[cur], key);
+        }
+        cl.sync();
+        for (int p = plo + tid; p < phi; p += kAggThreads) {
+          const unsigned long long key = __ldcg(a.k0 + p);
+          a.k0[p] = 0ull;
+          const float d = __uint_as_float((unsigned)(key >> 32));
+          const int idx = (int)(key & 0xffffffffu);
+          if ((double)d > .1) {
+            const int t = __ldcg(a.to + idx);
+            __stcg(pin + idx, t);
+            atomicAdd(&a.sizes[t], a.w[idx]);
+            atomicAdd(&a.sizes[p], -a.w[idx]);
+          }
+        }
+        cl.sync();
+      }
+      break;
+    }
+    // ---- parts below the threshold dissolve, the others are renumbered in order
+    int threshold = a.min_size;
+    if (a.w) {
+      first = false;
+      const double avg = (double)a.full_size / count;
+      threshold = (int)(avg * .7);
+    }
+    int small = 0;
+    for (int p = plo + tid; p < phi; p += kAggThreads) small += __ldcg(a.sizes + p) < threshold;
+    const int2 pre = x.prefix(cl, agg_block_sum(small, sh));
+    if (pre.y == 0 && !a.w) break;
+    int base = pre.x;
+    for (int p0 = plo; p0 < phi; p0 += kAggThreads) {
+      const int p = p0 + tid;
+      const bool rm = p < phi && __ldcg(a.sizes + p) < threshold;
+      int total;
+      const int rank = agg_block_rank(rm, sh, &total);
+      if (p < phi) a.map[p] = rm ? -1 : p - (base + rank);
+      base += total;
+    }
+    count -= pre.y;
+    cl.sync();
+    for (int i = lo + tid; i < hi; i += kAggThreads) pin[i] = __ldcg(a.map + pin[i]);
+    cl.sync();
+  }
+  int m = -1;
+  for (int i = lo + tid; i < hi; i += kAggThreads) m = max(m, __ldcg(pin + i));
+  m = x.max(cl, agg_block_max(m, sh));
+  if (x.me == 0 && tid == 0) {
+    a.res[0] = status;
+    a.res[1] = count;
+    a.res[2] = m + 1;
+    a.res[3] = pin == a.pout;
+  }
+  cl.sync();  // no CTA leaves while another may still write to its exchange buffers
+}
+
+// Runs aggregate_cluster_kernel: the labels in `part`, (parts after the removals, largest
+// label + 1) in count and labels.
+void aggregate_small(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int depth, int min_size, int max_size,
+                     int full_size, const int32_t* weights, DBuf<int32_t>& part, int* count, int* labels) {
   cudaStream_t s = c.stream;
+  PhaseTimer pt(s, -4);
+  DBuf<unsigned long long> keys((size_t)2 * n, s);
+  DBuf<uint32_t> rnd(n, s);
+  DBuf<int32_t> work((size_t)4 * n + 4, s), pout(n, s);
+  part.alloc(n, s);
+  AggArgs a{};
+  a.n = n;
+  a.xadj = xadj;
+  a.adj = adj;
+  a.w = weights;
+  a.seeds = mis_seeds(c);
+  a.depth = depth;
+  a.min_size = min_size;
+  a.max_size = max_size;
+  a.full_size = full_size;
+  a.rnd = rnd.p;
+  a.k0 = keys.p;
+  a.k1 = keys.p + n;
+  a.part = part.p;
+  a.pout = pout.p;
+  a.res = work.p;
+  a.mis = work.p + 4;
+  a.sizes = a.mis + n;
+  a.map = a.sizes + n;
+  a.to = a.map + n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kAggThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const int most = largest_cluster(reinterpret_cast<const void*>(aggregate_cluster_kernel), kAggThreads, kAggCtas);
+  const int ctas = std::min(most, next_pow2((n + kAggThreads - 1) / kAggThreads));
+  at[0].val.clusterDim.x = (unsigned)ctas;
+  cfg.gridDim = dim3((unsigned)ctas);
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  FG_CUDA(cudaLaunchKernelEx(&cfg, aggregate_cluster_kernel, a));
+  int32_t h[4];
+  FG_CUDA(cudaMemcpyAsync(h, a.res, sizeof(h), cudaMemcpyDeviceToHost, s));
+  FG_CUDA(cudaStreamSynchronize(s));
+  g_host_syncs.fetch_add(1, std::memory_order_relaxed);
+  pt.mark("cluster");
+  if (h[0] == AGG_MIS_CAP) throw Error(FEMGPU_ERR_LIMIT, "randomized MIS did not complete");
+  if (h[0] == AGG_LOOP_CAP) throw Error(FEMGPU_ERR_LIMIT, "aggregation did not complete");
+  if (h[0] == AGG_RESTRICT_CAP) throw Error(FEMGPU_ERR_LIMIT, "partition size restriction did not converge");
+  if (h[0] == AGG_STALLED) throw_stalled();
+  if (h[3]) std::swap(part.p, pout.p);
+  *count = h[1];
+  *labels = h[2];
+}
+
+// aggregateGraph / aggregateWeightedGraph (misHelpers.cu:513-677).  Returns the number
+// of parts (the largest label + 1: the partition restriction of the weighted graph may
+// empty a part).
+int aggregate(Ctx& c, int n, int64_t edges, const int32_t* xadj, const int32_t* adj, int depth, bool weighted,
+              int min_size, int max_size, int full_size, const int32_t* weights, DBuf<int32_t>& part) {
+  cudaStream_t s = c.stream;
+  if (edges <= kClusterAggEdges && n <= kClusterAggEdges / 4 && depth > 0) {
+    int count = 0, labels = 0;
+    aggregate_small(c, n, xadj, adj, depth, min_size, max_size, full_size, weighted ? weights : nullptr, part, &count,
+                    &labels);
+    return weighted ? labels : count;
+  }
   PhaseTimer pt(s, -4);
   DBuf<int32_t> mis;
   random_mis(c, n, xadj, adj, depth, mis);
@@ -447,7 +852,7 @@ int aggregate(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int depth,
         // empty a partition, but nothing reads the count after it): tracked, not read
         if (!first || mis_count < 10) {
           restrict_partitions(c, max_size, full_size, n, xadj, adj, part, weights, mis_count);
-          return -1;
+          return reduce_max(part.p, n, s) + 1;
         }
         first = false;
         mis_count -= remove_small_parts(c, n, part, weights, 1, 0, full_size, aggregated, mis_count);
@@ -455,9 +860,7 @@ int aggregate(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int depth,
     } else if (h[1] == 0) {
       // also the case where every aggregate was removed as undersized (the reference
       // loops forever there)
-      throw Error(FEMGPU_ERR_LIMIT,
-                  "aggregation stalled: nodes unreachable from any aggregate, or every aggregate was removed "
-                  "as undersized");
+      throw_stalled();
     }
   }
 }
@@ -646,13 +1049,13 @@ struct OldMisOut {
 };
 
 // misHelpers::CP::OldMIS (ComputePermutationMethods.cu:22-151).
-void old_mis(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, OldMisOut& o) {
+void old_mis(Ctx& c, int n, int64_t edges, const int32_t* xadj, const int32_t* adj, OldMisOut& o) {
   cudaStream_t s = c.stream;
   const int params = c.cfg.randMisParameters;
   const int fine_depth = params % 100, coarse_depth = (params / 100) % 100, min_agg = (params / 10000) % 10;
   PhaseTimer pt(s, -1);
   DBuf<int32_t> fine;
-  const int nagg = aggregate(c, n, xadj, adj, fine_depth, false, min_agg, 0, n, nullptr, fine);
+  const int nagg = aggregate(c, n, edges, xadj, adj, fine_depth, false, min_agg, 0, n, nullptr, fine);
   pt.mark("fine agg");
   // aggregate member lists, ascending node id
   DBuf<int32_t> acount(nagg + 1, s), astart(nagg + 1, s), cursor(nagg, s), members(n, s);
@@ -710,9 +1113,9 @@ void old_mis(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, OldMisOut& 
   pt.mark("induced");
   // partitions of aggregates (aggregateWeightedGraph, weights = aggregate sizes)
   DBuf<int32_t> coarse;
-  aggregate(c, nagg, ixadj.p, iadj.p, coarse_depth, true, 0, c.cfg.partitionMaxSize, n, acount.p, coarse);
+  const int npart =
+      aggregate(c, nagg, induced_nnz, ixadj.p, iadj.p, coarse_depth, true, 0, c.cfg.partitionMaxSize, n, acount.p, coarse);
   pt.mark("partitions");
-  const int npart = reduce_max(coarse.p, nagg, s) + 1;
   // new aggregate ids: order (partition, old id)
   DBuf<int32_t> pcount(npart + 1, s), pcur(npart, s), old_of(nagg, s), new_id(nagg, s);
   pcount.zero();
@@ -2549,7 +2952,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
     PhaseTimer pt(s, num_levels - 1);
     const TraceRange level_range("femgpu setup: level");
     OldMisOut o;
-    old_mis(c, N, L.gxadj.p, L.gadj.p, o);
+    old_mis(c, N, L.gnnz, L.gxadj.p, L.gadj.p, o);
     pt.mark("aggregate");
     L.nagg = o.nagg;
     L.npart = o.npart;

@@ -197,6 +197,9 @@ struct Ctx {
   int64_t graph_nnz = 0;
   bool has_matrix = false;
 
+  DBuf<uint32_t> mis_seeds;      // generator seeds of the randomized MIS for cfg.seed ...
+  uint32_t mis_seeds_of = 0;     // ... made for this seed
+
   // hierarchy (built by femgpu_setup)
   std::unique_ptr<HierarchyBase> H;
   DBuf<int32_t> perm0;           // level-0 old -> new (identity if level 0 is the coarsest)

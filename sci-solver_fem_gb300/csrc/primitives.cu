@@ -20,6 +20,33 @@ void ensure_dynamic_smem(const void* func, size_t bytes) {
 }
 
 
+int largest_cluster(const void* func, int threads, int most) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, int> known;
+  int dev = 0;
+  FG_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  int& size = known[{dev, func}];
+  if (size > 0) return size;
+  if (most > 8) FG_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  for (int c = most; c > 1; c >>= 1) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)c);
+    cfg.blockDim = dim3((unsigned)threads);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)c;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, func, &cfg) == cudaSuccess && clusters > 0) return size = c;
+    (void)cudaGetLastError();
+  }
+  return size = 1;
+}
+
 namespace {
 
 #define FG_RUN(...)    \
