@@ -68,26 +68,33 @@ __device__ __forceinline__ void st8(T* p, const V8<T>& r) {
   }
 }
 
-// ---- reductions: eight columns at once over the fixed grid -----------------------------
-// Block sums of v[0..7] (blockDim kBT); valid in thread 0.
-__device__ __forceinline__ void block_sum8(double v[kBlock], double (*sh)[kBlock]) {
+// ---- vector kernels and reductions over the fixed grid -------------------------------
+// A block vector is walked as n x 4 pairs of columns, pair q mod 4 = columns 2 (q mod 4) and
+// the next: consecutive threads read consecutive 16 bytes, and a thread keeps its two columns
+// because the grid's stride is a multiple of 4.  (A thread per row, 64 bytes apart, ran these
+// kernels at 0.8 TB/s: 64^3, eight columns, dot 67 -> 22 us, update 66 -> 26 us.)
+constexpr int kPairs = kBlock / 2;
+
+// Block sums of a pair of columns per thread (the pair of threadIdx.x mod 4) to
+// out[0 .. 8), by threads 0..7.
+__device__ __forceinline__ void block_columns(double2 v, double (*sh)[kBlock], double* out) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-  for (int j = 0; j < kBlock; j++) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(kAll, v[j], o);
-    if (lane == 0) sh[w][j] = v[j];
+  for (int o = 16; o >= kPairs; o >>= 1) {
+    v.x += __shfl_xor_sync(kAll, v.x, o);
+    v.y += __shfl_xor_sync(kAll, v.y, o);
+  }
+  __syncthreads();  // sh may still be read from an earlier call
+  if (lane < kPairs) {
+    sh[w][2 * lane] = v.x;
+    sh[w][2 * lane + 1] = v.y;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int j = 0; j < kBlock; j++) {
-      double t = sh[0][j];
-      for (int q = 1; q < kBT / 32; q++) t += sh[q][j];
-      v[j] = t;
-    }
+  if (threadIdx.x < kBlock) {
+    double t = sh[0][threadIdx.x];
+    for (int q = 1; q < kBT / 32; q++) t += sh[q][threadIdx.x];
+    out[threadIdx.x] = t;
   }
-  __syncthreads();
 }
 
 // After every block wrote its partials: true in the block that finishes last.
@@ -101,16 +108,21 @@ __device__ __forceinline__ bool last_block(unsigned* counter) {
   return s_last;
 }
 
-// Totals of partial[j * kBG + b] over b for each column j, in a fixed order (thread t adds
-// b = t, t + kBT, ...; then the block sum); valid in thread 0.
-__device__ __forceinline__ void column_totals(const double* partial, double tot[kBlock], double (*sh)[kBlock]) {
-#pragma unroll
-  for (int j = 0; j < kBlock; j++) {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < kBG; b += kBT) s += partial[j * kBG + b];
-    tot[j] = s;
-  }
-  block_sum8(tot, sh);
+// Total of partial[b * 8 + j] over b for column j = threadIdx.x mod 8, in a fixed order; in
+// threads 0..7.
+__device__ __forceinline__ double column_total(const double* partial, double (*sh)[kBlock]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, j = threadIdx.x & (kBlock - 1);
+  double s = 0.0;
+#pragma unroll 4
+  for (int b = threadIdx.x / kBlock; b < kBG; b += kBT / kBlock) s += partial[b * kBlock + j];
+  s += __shfl_xor_sync(kAll, s, 8);
+  s += __shfl_xor_sync(kAll, s, 16);
+  __syncthreads();
+  if (lane < kBlock) sh[w][lane] = s;
+  __syncthreads();
+  s = sh[0][j];
+  for (int q = 1; q < kBT / 32; q++) s += sh[q][j];
+  return s;
 }
 
 // ---- FP64 outer kernels -------------------------------------------------------------
@@ -141,62 +153,69 @@ __global__ void __launch_bounds__(kBT) blk_dot_kernel(int n, const double* __res
                                                        double* partial, double* sc, int slot, int slot2,
                                                        unsigned* counter) {
   __shared__ double sh[kBT / 32][kBlock];
-  double s1[kBlock] = {}, s2[kBlock] = {};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const V8<double> va = ld8(a + (int64_t)i * kBlock), vb = ld8(b + (int64_t)i * kBlock);
-#pragma unroll
-    for (int j = 0; j < kBlock; j++) s1[j] = fma(va.v[j], vb.v[j], s1[j]);
+  const double2 *va = reinterpret_cast<const double2*>(a), *vb = reinterpret_cast<const double2*>(b),
+                *vc = reinterpret_cast<const double2*>(c);
+  const int64_t pairs = (int64_t)n * kPairs;
+  double2 s1 = make_double2(0.0, 0.0), s2 = s1;
+#pragma unroll 2
+  for (int64_t q = (int64_t)blockIdx.x * kBT + threadIdx.x; q < pairs; q += (int64_t)kBG * kBT) {
+    const double2 x = va[q], y = vb[q];
+    s1.x = fma(x.x, y.x, s1.x);
+    s1.y = fma(x.y, y.y, s1.y);
     if (c) {
-      const V8<double> vc = ld8(c + (int64_t)i * kBlock);
-#pragma unroll
-      for (int j = 0; j < kBlock; j++) s2[j] = fma(va.v[j], vc.v[j], s2[j]);
+      const double2 z = vc[q];
+      s2.x = fma(x.x, z.x, s2.x);
+      s2.y = fma(x.y, z.y, s2.y);
     }
   }
-  block_sum8(s1, sh);
-  if (threadIdx.x == 0)
-    for (int j = 0; j < kBlock; j++) partial[j * kBG + blockIdx.x] = s1[j];
-  if (c) {
-    block_sum8(s2, sh);
-    if (threadIdx.x == 0)
-      for (int j = 0; j < kBlock; j++) partial[(kBlock + j) * kBG + blockIdx.x] = s2[j];
-  }
+  block_columns(s1, sh, partial + blockIdx.x * kBlock);
+  if (c) block_columns(s2, sh, partial + (kBG + blockIdx.x) * kBlock);
   if (!last_block(counter)) return;
-  double t[kBlock];
-  column_totals(partial, t, sh);
-  if (threadIdx.x == 0)
-    for (int j = 0; j < kBlock; j++) sc[slot * kBlock + j] = t[j];
+  const double t1 = column_total(partial, sh);
+  if (threadIdx.x < kBlock) sc[slot * kBlock + threadIdx.x] = t1;
   if (c) {
-    column_totals(partial + kBlock * kBG, t, sh);
-    if (threadIdx.x == 0)
-      for (int j = 0; j < kBlock; j++) sc[slot2 * kBlock + j] = t[j];
+    const double t2 = column_total(partial + kBG * kBlock, sh);
+    if (threadIdx.x < kBlock) sc[slot2 * kBlock + threadIdx.x] = t2;
   }
   if (threadIdx.x == 0) *counter = 0u;
 }
 
-// Row i of the outer FP64 operator times the block (sliced layout when off != nullptr:
-// rows 32 s .. 32 s + 31 column-major from off[s], padding column -1; else CSR).
-__device__ __forceinline__ V8<double> outer_row(int i, const int32_t* __restrict__ off, const int32_t* __restrict__ rp,
-                                                const int32_t* __restrict__ ci, const double* __restrict__ v,
-                                                const double* __restrict__ p) {
-  V8<double> s;
-#pragma unroll
-  for (int j = 0; j < kBlock; j++) s.v[j] = 0.0;
-  int e = off ? off[i >> 5] + (i & 31) : rp[i];
+// Columns 2 t, 2 t + 1 (t = the lane's pair) of row i of the outer FP64 operator times the
+// block (sliced layout when off != nullptr: rows 32 s .. 32 s + 31 column-major from off[s],
+// padding column -1; else CSR), entries in order, four in flight.  Four lanes share a row, so
+// a gathered row of the block is one 64-byte access.  Bound by the FP64 pipe: 8 fused
+// multiply-adds per entry (64^3: 32 M, 64 us at 0.5 T/s).
+__device__ __forceinline__ double2 outer_row(int i, int t, const int32_t* __restrict__ off,
+                                             const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                             const double* __restrict__ v, const double* __restrict__ p) {
+  const double2* __restrict__ p2 = reinterpret_cast<const double2*>(p);
+  double2 s = make_double2(0.0, 0.0);
   const int end = off ? off[(i >> 5) + 1] : rp[i + 1];
   const int step = off ? 32 : 1;
-  for (; e < end; e += step) {
-    const int col = ci[e];
-    if (col < 0) break;  // slice padding comes after a row's entries
-    const double a = v[e];
-    const V8<double> x = ld8(p + (int64_t)col * kBlock);
+  for (int e = off ? off[i >> 5] + (i & 31) : rp[i]; e < end; e += 4 * step) {
+    int c[4];
+    double a[4];
+    double2 x[4];
 #pragma unroll
-    for (int j = 0; j < kBlock; j++) s.v[j] = fma(a, x.v[j], s.v[j]);
+    for (int k = 0; k < 4; k++) {
+      c[k] = e + k * step < end ? ci[e + k * step] : -1;
+      a[k] = e + k * step < end ? v[e + k * step] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) x[k] = c[k] >= 0 ? p2[(int64_t)c[k] * kPairs + t] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (c[k] >= 0) {
+        s.x = fma(a[k], x[k].x, s.x);
+        s.y = fma(a[k], x[k].y, s.y);
+      }
   }
   return s;
 }
 
 // y = A p, p.y per column; the last block forms alpha = rz / p.y for the active columns
-// (a non-positive or non-finite p.y flags the column and stops it).
+// (a non-positive or non-finite p.y flags the column and stops it).  64^3, eight columns:
+// 105 -> 84 us (a thread per row, eight columns each).
 __global__ void __launch_bounds__(kBT) blk_spmv_dot_kernel(int n, const int32_t* __restrict__ off,
                                                             const int32_t* __restrict__ rp,
                                                             const int32_t* __restrict__ ci,
@@ -204,57 +223,53 @@ __global__ void __launch_bounds__(kBT) blk_spmv_dot_kernel(int n, const int32_t*
                                                             const double* __restrict__ p, double* __restrict__ y,
                                                             double* partial, double* sc, unsigned* counter) {
   __shared__ double sh[kBT / 32][kBlock];
-  double acc[kBlock] = {};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const V8<double> s = outer_row(i, off, rp, ci, v, p);
-    st8(y + (int64_t)i * kBlock, s);
-    const V8<double> pi = ld8(p + (int64_t)i * kBlock);
-#pragma unroll
-    for (int j = 0; j < kBlock; j++) acc[j] = fma(s.v[j], pi.v[j], acc[j]);
+  const double2* p2 = reinterpret_cast<const double2*>(p);
+  double2* y2 = reinterpret_cast<double2*>(y);
+  const int64_t pairs = (int64_t)n * kPairs;
+  double2 acc = make_double2(0.0, 0.0);
+  for (int64_t q = (int64_t)blockIdx.x * kBT + threadIdx.x; q < pairs; q += (int64_t)kBG * kBT) {
+    const double2 s = outer_row((int)(q / kPairs), (int)(q & (kPairs - 1)), off, rp, ci, v, p), pi = p2[q];
+    y2[q] = s;
+    acc.x = fma(s.x, pi.x, acc.x);
+    acc.y = fma(s.y, pi.y, acc.y);
   }
-  block_sum8(acc, sh);
-  if (threadIdx.x == 0)
-    for (int j = 0; j < kBlock; j++) partial[j * kBG + blockIdx.x] = acc[j];
+  block_columns(acc, sh, partial + blockIdx.x * kBlock);
   if (!last_block(counter)) return;
-  double t[kBlock];
-  column_totals(partial, t, sh);
-  if (threadIdx.x == 0) {
-    for (int j = 0; j < kBlock; j++) {
-      double* s = sc;
-      s[B_PY * kBlock + j] = t[j];
-      double alpha = 0.0;
-      if (s[B_ACTIVE * kBlock + j] != 0.0) {
-        if (t[j] > 0.0 && isfinite(t[j])) {
-          alpha = s[B_RZ * kBlock + j] / t[j];
-        } else {
-          s[B_FLAG * kBlock + j] = 1.0;
-          s[B_ACTIVE * kBlock + j] = 0.0;
-        }
+  const double t = column_total(partial, sh);
+  const int j = threadIdx.x;
+  if (j < kBlock) {
+    double* s = sc;
+    s[B_PY * kBlock + j] = t;
+    double alpha = 0.0;
+    if (s[B_ACTIVE * kBlock + j] != 0.0) {
+      if (t > 0.0 && isfinite(t)) {
+        alpha = s[B_RZ * kBlock + j] / t;
+      } else {
+        s[B_FLAG * kBlock + j] = 1.0;
+        s[B_ACTIVE * kBlock + j] = 0.0;
       }
-      s[B_ALPHA * kBlock + j] = alpha;
     }
-    *counter = 0u;
+    s[B_ALPHA * kBlock + j] = alpha;
   }
+  if (j == 0) *counter = 0u;
 }
 
 // y = A x (start of the solve).
 __global__ void blk_spmv_kernel(int n, const int32_t* __restrict__ off, const int32_t* __restrict__ rp,
                                 const int32_t* __restrict__ ci, const double* __restrict__ v,
                                 const double* __restrict__ x, double* __restrict__ y) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) st8(y + (int64_t)i * kBlock, outer_row(i, off, rp, ci, v, x));
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < (int64_t)n * kPairs)
+    reinterpret_cast<double2*>(y)[q] = outer_row((int)(q / kPairs), (int)(q & (kPairs - 1)), off, rp, ci, v, x);
 }
 
 // r = b - y
 __global__ void blk_sub_kernel(int n, const double* __restrict__ b, const double* __restrict__ y,
                                double* __restrict__ r) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const V8<double> vb = ld8(b + (int64_t)i * kBlock), vy = ld8(y + (int64_t)i * kBlock);
-  V8<double> o;
-#pragma unroll
-  for (int j = 0; j < kBlock; j++) o.v[j] = vb.v[j] - vy.v[j];
-  st8(r + (int64_t)i * kBlock, o);
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= (int64_t)n * kPairs) return;
+  const double2 vb = reinterpret_cast<const double2*>(b)[q], vy = reinterpret_cast<const double2*>(y)[q];
+  reinterpret_cast<double2*>(r)[q] = make_double2(vb.x - vy.x, vb.y - vy.y);
 }
 
 // beta per column (cgcycle.cu:52-54; Polak-Ribiere when flexible), 0 on the first
@@ -275,13 +290,11 @@ __global__ void blk_beta_kernel(double* sc) {
 // p = z + beta p
 __global__ void blk_pupdate_kernel(int n, const double* __restrict__ sc, const double* __restrict__ z,
                                    double* __restrict__ p) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const V8<double> vz = ld8(z + (int64_t)i * kBlock), vp = ld8(p + (int64_t)i * kBlock);
-  V8<double> o;
-#pragma unroll
-  for (int j = 0; j < kBlock; j++) o.v[j] = fma(sc[B_BETA * kBlock + j], vp.v[j], vz.v[j]);
-  st8(p + (int64_t)i * kBlock, o);
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= (int64_t)n * kPairs) return;
+  const double2 beta = reinterpret_cast<const double2*>(sc + B_BETA * kBlock)[q & (kPairs - 1)];
+  const double2 vz = reinterpret_cast<const double2*>(z)[q], vp = reinterpret_cast<const double2*>(p)[q];
+  reinterpret_cast<double2*>(p)[q] = make_double2(fma(beta.x, vp.x, vz.x), fma(beta.y, vp.y, vz.y));
 }
 
 // x += alpha p; r -= alpha y (rold = r first when flexible); r.r per column; the last
@@ -291,54 +304,69 @@ __global__ void __launch_bounds__(kBT) blk_update_kernel(int n, double* sc, cons
                                                           double* __restrict__ r, double* __restrict__ rold,
                                                           double* partial, unsigned* counter) {
   __shared__ double sh[kBT / 32][kBlock];
-  double alpha[kBlock], acc[kBlock] = {};
-#pragma unroll
-  for (int j = 0; j < kBlock; j++) alpha[j] = sc[B_ALPHA * kBlock + j];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int64_t o = (int64_t)i * kBlock;
-    const V8<double> vr = ld8(r + o), vp = ld8(p + o), vx = ld8(x + o), vy = ld8(y + o);
-    if (rold) st8(rold + o, vr);
-    V8<double> nx, nr;
-#pragma unroll
-    for (int j = 0; j < kBlock; j++) {
-      nx.v[j] = fma(alpha[j], vp.v[j], vx.v[j]);
-      nr.v[j] = fma(-alpha[j], vy.v[j], vr.v[j]);
-      acc[j] = fma(nr.v[j], nr.v[j], acc[j]);
-    }
-    st8(x + o, nx);
-    st8(r + o, nr);
+  const double2 alpha = reinterpret_cast<const double2*>(sc + B_ALPHA * kBlock)[threadIdx.x & (kPairs - 1)];
+  const double2 *vp = reinterpret_cast<const double2*>(p), *vy = reinterpret_cast<const double2*>(y);
+  double2 *vx = reinterpret_cast<double2*>(x), *vr = reinterpret_cast<double2*>(r), *vo = reinterpret_cast<double2*>(rold);
+  const int64_t pairs = (int64_t)n * kPairs;
+  double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 2
+  for (int64_t q = (int64_t)blockIdx.x * kBT + threadIdx.x; q < pairs; q += (int64_t)kBG * kBT) {
+    const double2 rr = vr[q], pp = vp[q], xx = vx[q], yy = vy[q];
+    if (rold) vo[q] = rr;
+    vx[q] = make_double2(fma(alpha.x, pp.x, xx.x), fma(alpha.y, pp.y, xx.y));
+    const double2 nr = make_double2(fma(-alpha.x, yy.x, rr.x), fma(-alpha.y, yy.y, rr.y));
+    vr[q] = nr;
+    acc.x = fma(nr.x, nr.x, acc.x);
+    acc.y = fma(nr.y, nr.y, acc.y);
   }
-  block_sum8(acc, sh);
-  if (threadIdx.x == 0)
-    for (int j = 0; j < kBlock; j++) partial[j * kBG + blockIdx.x] = acc[j];
+  block_columns(acc, sh, partial + blockIdx.x * kBlock);
   if (!last_block(counter)) return;
-  double t[kBlock];
-  column_totals(partial, t, sh);
-  if (threadIdx.x == 0) {
-    const double it = sc[G_IT] + 1.0;
-    sc[G_IT] = it;
-    double any = 0.0;
-    for (int j = 0; j < kBlock; j++) {
-      sc[B_NR * kBlock + j] = t[j];
-      if (sc[B_ACTIVE * kBlock + j] == 0.0) continue;
+  const double t = column_total(partial, sh);
+  __shared__ int s_any;
+  if (threadIdx.x == 0) s_any = 0;
+  __syncthreads();
+  const int j = threadIdx.x;
+  const double it = sc[G_IT] + 1.0;
+  if (j < kBlock) {
+    sc[B_NR * kBlock + j] = t;
+    if (sc[B_ACTIVE * kBlock + j] != 0.0) {
       sc[B_ITS * kBlock + j] = it;
       const double bn = sqrt(sc[B_BN * kBlock + j]);
-      const double nr = sqrt(t[j]);
+      const double nr = sqrt(t);
       if (!isfinite(nr)) {
         sc[B_FLAG * kBlock + j] = 1.0;
         sc[B_ACTIVE * kBlock + j] = 0.0;
       } else if (nr / (bn > 0.0 ? bn : 1.0) <= sc[G_TOL]) {
         sc[B_ACTIVE * kBlock + j] = 0.0;
       } else {
-        any = 1.0;
+        s_any = 1;
       }
     }
-    sc[G_ANY] = (any != 0.0 && it < sc[G_MAXIT]) ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  if (j == 0) {
+    sc[G_IT] = it;
+    sc[G_ANY] = (s_any && it < sc[G_MAXIT]) ? 1.0 : 0.0;
     *counter = 0u;
   }
 }
 
 // ---- V-cycle kernels (hierarchy precision T) ------------------------------------------------
+// C neighbouring columns of a block row.
+template <class T, int C>
+struct __align__(C * sizeof(T)) Cols {
+  T v[C];
+};
+template <class T>
+using Pair = Cols<T, 2>;
+
+// An in-partition entry in shared memory: its value and the byte offset of the x row it reads.
+template <class T>
+struct __align__(2 * sizeof(T)) BlkEntry {
+  T v;
+  int off;
+};
+
 template <class T>
 __global__ void blk_cast_in_kernel(int64_t m, const double* __restrict__ in, T* __restrict__ out) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -358,36 +386,241 @@ __device__ __forceinline__ T relax1(T x, T b, T sax, T d, T dinv, T w) {
   return x + (w * t) * dinv;
 }
 
-// Partition-block weighted Jacobi on one group of consecutive partitions per CTA (rows
-// [grows[g], grows[g + 1])), all eight columns at once: the group's x double-buffered in
-// shared memory (m x 8), the right-hand side b (pre) or b - A_out x_in (post) staged
-// beside it.  In-partition entries are used for all eight columns: with STAGED they are
-// copied once (coalesced) into shared memory with group-local 16-bit columns, otherwise
-// they are read from global memory (L2) in every sweep.  Pre (POST == false):
-// x0 = w b / d, `inner` sweeps, then x and r = b - A_in x - d x.  Post: `inner` sweeps
-// from x_in.
-template <class T, bool POST, bool STAGED>
-__global__ void __launch_bounds__(512) blk_smooth_kernel(
+// Partition-block weighted Jacobi on one group of consecutive partitions (rows
+// [grows[g], grows[g + 1]), at most kBlkRows of them) and C LPR of the eight columns per CTA:
+// LPR lanes per row with C columns each, times EL lanes that share the row's entries, and up
+// to LPR EL rows per thread.  The group's x is double-buffered in shared memory, its
+// in-partition entries are staged there once (eight loads in flight); a row's bounds,
+// diagonal, right-hand side and x stay in registers.  Pre (POST == false): x0 = w b / d,
+// `inner` sweeps, then x and r = b - A_in x - d x; with b64 the right-hand side is read in
+// FP64, rounded, and kept in b_store for the post relax.  Post: b - A_out x_in, `inner` sweeps
+// from x_in; with z64 the result is written there in FP64.  With EL = 1 row sums run in entry
+// order, else lane j adds entries j, j + EL, ... and the lanes' sums are added by shuffles.
+// Bound by shared-memory instructions and their latency on full levels, by staging and
+// barriers on small ones.  64^3, pre relaxes of the levels of 708, 32 and 2 groups:
+// 95 -> 68, 65 -> 25, 85 -> 27 us (before: all eight columns by one thread per row, bounds
+// and diagonal from global memory in every sweep).
+constexpr int kBlkRows = 512;
+constexpr int kBlkThreads = 512;
+
+template <class T, bool POST, int C, int LPR, int EL>
+__global__ void __launch_bounds__(kBlkThreads, sizeof(T) == 4 ? 2 : 1) blk_smooth_kernel(
     const int32_t* __restrict__ grows, const int32_t* __restrict__ irp, const int32_t* __restrict__ ici,
     const T* __restrict__ iv, const int32_t* __restrict__ orp, const int32_t* __restrict__ oci,
-    const T* __restrict__ ov, const T* __restrict__ diag, const T* __restrict__ dinv, const T* __restrict__ b, T w,
-    int inner, const T* __restrict__ x_in, T* __restrict__ x_out, T* __restrict__ r_out, int mcap, int ecap) {
+    const T* __restrict__ ov, const T* __restrict__ diag, const T* __restrict__ dinv, const T* __restrict__ b,
+    const double* __restrict__ b64, T* __restrict__ b_store, T w, int inner, const T* __restrict__ x_in,
+    T* __restrict__ x_out, double* __restrict__ z64, T* __restrict__ r_out, int mcap) {
+  using V = Cols<T, C>;
+  constexpr int SPLIT = kBlock / (C * LPR);  // CTAs per group
+  constexpr int RV = kBlock / C;             // vectors per block row in global memory
+  constexpr int RP = LPR * EL;               // rows per thread, lanes per row
+  constexpr int RB = C * LPR * sizeof(T);    // bytes of a row of x in shared memory
+  extern __shared__ __align__(16) unsigned char sm[];
+  unsigned char* const x0b = sm;
+  unsigned char* const x1b = sm + (size_t)mcap * RB;
+  BlkEntry<T>* const ent = reinterpret_cast<BlkEntry<T>*>(x1b + (size_t)mcap * RB);
+  const int g = blockIdx.x / SPLIT;
+  const int rs = grows[g], m = grows[g + 1] - rs;
+  const int es = irp[rs], ne = irp[rs + m] - es;
+  const int per = blockDim.x / RP, lr = threadIdx.x / RP;
+  const int lp = threadIdx.x % LPR, el = (threadIdx.x / LPR) % EL;
+  const int vec = (blockIdx.x % SPLIT) * LPR + lp;  // of the row's vectors in global memory
+  for (int q0 = threadIdx.x; q0 < ne; q0 += 8 * blockDim.x) {
+    T v[8];
+    int c[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int q = q0 + k * blockDim.x;
+      v[k] = q < ne ? iv[es + q] : (T)0;
+      c[k] = q < ne ? ici[es + q] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int q = q0 + k * blockDim.x;
+      if (q < ne) {
+        BlkEntry<T> e;
+        e.v = v[k];
+        e.off = (c[k] - rs) * RB;
+        ent[q] = e;
+      }
+    }
+  }
+  const V* xin = reinterpret_cast<const V*>(x_in);
+  V x[RP], bb[RP];
+  T d[RP], di[RP];
+  int e0[RP], e1[RP];
+#pragma unroll
+  for (int u = 0; u < RP; u++) {
+    const int t = u * per + lr, row = rs + t;
+    const bool live = t < m;
+    e0[u] = e1[u] = 0;
+    d[u] = di[u] = (T)1;
+#pragma unroll
+    for (int k = 0; k < C; k++) x[u].v[k] = bb[u].v[k] = (T)0;
+    const int64_t at = (int64_t)row * RV + vec;
+    int o0 = 0, o1 = 0;
+    if (live) {
+      e0[u] = irp[row] - es;
+      e1[u] = irp[row + 1] - es;
+      d[u] = diag[row];
+      di[u] = dinv[row];
+      if (!POST && b64) {
+        const Cols<double, 2>* src = reinterpret_cast<const Cols<double, 2>*>(b64 + at * C);
+#pragma unroll
+        for (int k = 0; k < C / 2; k++) {
+          const Cols<double, 2> v = src[k];
+          bb[u].v[2 * k] = (T)v.v[0];
+          bb[u].v[2 * k + 1] = (T)v.v[1];
+        }
+        if (el == 0) reinterpret_cast<V*>(b_store)[at] = bb[u];
+      } else {
+        bb[u] = reinterpret_cast<const V*>(b)[at];
+      }
+      if (POST) {
+        x[u] = xin[at];
+        o0 = orp[row];
+        o1 = orp[row + 1];
+      } else {
+#pragma unroll
+        for (int k = 0; k < C; k++) x[u].v[k] = (w * bb[u].v[k]) * di[u];
+      }
+    }
+    if (POST) {
+      V so;  // EL > 1: this lane's share of A_out x
+#pragma unroll
+      for (int k = 0; k < C; k++) so.v[k] = (T)0;
+      for (int o = o0 + el; o < o1; o += 4 * EL) {
+        int c[4];
+        T a[4];
+        V xo[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          c[q] = o + q * EL < o1 ? oci[o + q * EL] : row;
+          a[q] = o + q * EL < o1 ? ov[o + q * EL] : (T)0;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) xo[q] = xin[(int64_t)c[q] * RV + vec];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          if (o + q * EL < o1) {
+#pragma unroll
+            for (int k = 0; k < C; k++) {
+              if (EL == 1) bb[u].v[k] = bb[u].v[k] - a[q] * xo[q].v[k];
+              else so.v[k] = fma(a[q], xo[q].v[k], so.v[k]);
+            }
+          }
+      }
+      if (EL > 1) {
+#pragma unroll
+        for (int k = 0; k < C; k++) {
+#pragma unroll
+          for (int f = LPR; f < RP; f <<= 1) so.v[k] = so.v[k] + __shfl_xor_sync(kAll, so.v[k], f);
+          bb[u].v[k] = bb[u].v[k] - so.v[k];
+        }
+      }
+    }
+    if (live && el == 0) reinterpret_cast<V*>(x0b + (size_t)t * RB)[lp] = x[u];
+  }
+  __syncthreads();
+  // every lane of the warp calls it (with EL > 1 the lanes' sums are exchanged)
+  auto row_sum = [&](const unsigned char* cur, int a, int z) {
+    const unsigned char* base = cur + lp * sizeof(V);
+    V s;
+#pragma unroll
+    for (int k = 0; k < C; k++) s.v[k] = (T)0;
+    int e = a + el;
+    for (; e + EL < z; e += 2 * EL) {
+      const BlkEntry<T> p = ent[e], q = ent[e + EL];
+      const V xp = *reinterpret_cast<const V*>(base + p.off), xq = *reinterpret_cast<const V*>(base + q.off);
+#pragma unroll
+      for (int k = 0; k < C; k++) s.v[k] = fma(p.v, xp.v[k], s.v[k]);
+#pragma unroll
+      for (int k = 0; k < C; k++) s.v[k] = fma(q.v, xq.v[k], s.v[k]);
+    }
+    if (e < z) {
+      const BlkEntry<T> p = ent[e];
+      const V xp = *reinterpret_cast<const V*>(base + p.off);
+#pragma unroll
+      for (int k = 0; k < C; k++) s.v[k] = fma(p.v, xp.v[k], s.v[k]);
+    }
+    if (EL > 1) {
+#pragma unroll
+      for (int k = 0; k < C; k++)
+#pragma unroll
+        for (int f = LPR; f < RP; f <<= 1) s.v[k] = s.v[k] + __shfl_xor_sync(kAll, s.v[k], f);
+    }
+    return s;
+  };
+  unsigned char* cur = x0b;
+  unsigned char* nxt = x1b;
+  for (int it = 0; it < inner; it++) {
+#pragma unroll
+    for (int u = 0; u < RP; u++) {
+      const int t = u * per + lr;
+      const V s = row_sum(cur, e0[u], e1[u]);
+#pragma unroll
+      for (int k = 0; k < C; k++) x[u].v[k] = relax1(x[u].v[k], bb[u].v[k], s.v[k], d[u], di[u], w);
+      if (t < m && el == 0) reinterpret_cast<V*>(nxt + (size_t)t * RB)[lp] = x[u];
+    }
+    __syncthreads();
+    unsigned char* tmp = cur;
+    cur = nxt;
+    nxt = tmp;
+  }
+#pragma unroll
+  for (int u = 0; u < RP; u++) {
+    const int t = u * per + lr;
+    const int64_t at = (int64_t)(rs + t) * RV + vec;
+    const bool mine = t < m && el == 0;
+    if (mine) {
+      if (POST && z64) {
+#pragma unroll
+        for (int k = 0; k < C / 2; k++) {
+          Cols<double, 2> z;
+          z.v[0] = (double)x[u].v[2 * k];
+          z.v[1] = (double)x[u].v[2 * k + 1];
+          reinterpret_cast<Cols<double, 2>*>(z64 + at * C)[k] = z;
+        }
+      } else {
+        reinterpret_cast<V*>(x_out)[at] = x[u];
+      }
+    }
+    if (!POST) {
+      const V s = row_sum(cur, e0[u], e1[u]);
+      V r;
+#pragma unroll
+      for (int k = 0; k < C; k++) r.v[k] = (bb[u].v[k] - s.v[k]) - d[u] * x[u].v[k];
+      if (mine) reinterpret_cast<V*>(r_out)[at] = r;
+    }
+  }
+}
+
+// The same relaxes for groups that blk_smooth_kernel does not take (more than kBlkRows rows,
+// or entries that do not fit beside x): one CTA per group, a thread per row with all eight
+// columns, the entries read from global memory in every sweep.
+template <class T, bool POST>
+__global__ void __launch_bounds__(512) blk_smooth_large_kernel(
+    const int32_t* __restrict__ grows, const int32_t* __restrict__ irp, const int32_t* __restrict__ ici,
+    const T* __restrict__ iv, const int32_t* __restrict__ orp, const int32_t* __restrict__ oci,
+    const T* __restrict__ ov, const T* __restrict__ diag, const T* __restrict__ dinv, const T* __restrict__ b,
+    const double* __restrict__ b64, T* __restrict__ b_store, T w, int inner, const T* __restrict__ x_in,
+    T* __restrict__ x_out, double* __restrict__ z64, T* __restrict__ r_out, int mcap) {
   extern __shared__ __align__(16) unsigned char sm[];
   T* xa = reinterpret_cast<T*>(sm);
   T* xb = xa + (int64_t)mcap * kBlock;
   T* sb = xb + (int64_t)mcap * kBlock;
-  T* sv = sb + (int64_t)mcap * kBlock;
-  uint16_t* sc16 = reinterpret_cast<uint16_t*>(sv + ecap);
   const int rs = grows[blockIdx.x], m = grows[blockIdx.x + 1] - rs;
-  const int es = irp[rs];
-  if (STAGED)
-    for (int q = threadIdx.x; q < irp[rs + m] - es; q += blockDim.x) {
-      sv[q] = iv[es + q];
-      sc16[q] = (uint16_t)(ici[es + q] - rs);
-    }
   for (int t = threadIdx.x; t < m; t += blockDim.x) {
     const int row = rs + t;
-    V8<T> bb = ld8(b + (int64_t)row * kBlock), x0;
+    V8<T> bb, x0;
+    if (!POST && b64) {
+      const V8<double> v = ld8(b64 + (int64_t)row * kBlock);
+#pragma unroll
+      for (int j = 0; j < kBlock; j++) bb.v[j] = (T)v.v[j];
+      st8(b_store + (int64_t)row * kBlock, bb);
+    } else {
+      bb = ld8(b + (int64_t)row * kBlock);
+    }
     if (POST) {
       x0 = ld8(x_in + (int64_t)row * kBlock);
       for (int e = orp[row]; e < orp[row + 1]; e++) {
@@ -410,9 +643,8 @@ __global__ void __launch_bounds__(512) blk_smooth_kernel(
 #pragma unroll
     for (int j = 0; j < kBlock; j++) s.v[j] = (T)0;
     for (int e = irp[row]; e < irp[row + 1]; e++) {
-      const T a = STAGED ? sv[e - es] : iv[e];
-      const int col = STAGED ? (int)sc16[e - es] : ici[e] - rs;
-      const V8<T> xv = ld8(cur + (int64_t)col * kBlock);
+      const T a = iv[e];
+      const V8<T> xv = ld8(cur + (int64_t)(ici[e] - rs) * kBlock);
 #pragma unroll
       for (int j = 0; j < kBlock; j++) s.v[j] = fma(a, xv.v[j], s.v[j]);
     }
@@ -438,7 +670,14 @@ __global__ void __launch_bounds__(512) blk_smooth_kernel(
   for (int t = threadIdx.x; t < m; t += blockDim.x) {
     const int row = rs + t;
     const V8<T> xc = ld8(cur + (int64_t)t * kBlock);
-    st8(x_out + (int64_t)row * kBlock, xc);
+    if (POST && z64) {
+      V8<double> z;
+#pragma unroll
+      for (int j = 0; j < kBlock; j++) z.v[j] = (double)xc.v[j];
+      st8(z64 + (int64_t)row * kBlock, z);
+    } else {
+      st8(x_out + (int64_t)row * kBlock, xc);
+    }
     if (!POST) {
       const V8<T> s = row_sum(cur, row), bb = ld8(sb + (int64_t)t * kBlock);
       const T d = diag[row];
@@ -450,48 +689,59 @@ __global__ void __launch_bounds__(512) blk_smooth_kernel(
   }
 }
 
-// r -= A_out x (preAout_kernel, gauss_seidel.cu:1977-2015), eight columns.
-template <class T>
-__global__ void blk_aout_kernel(int n, const int32_t* __restrict__ orp, const int32_t* __restrict__ oci,
-                                const T* __restrict__ ov, const T* __restrict__ x, T* __restrict__ r) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  V8<T> s;
-#pragma unroll
-  for (int j = 0; j < kBlock; j++) s.v[j] = (T)0;
-  for (int e = orp[i]; e < orp[i + 1]; e++) {
-    const T a = ov[e];
-    const V8<T> xv = ld8(x + (int64_t)oci[e] * kBlock);
-#pragma unroll
-    for (int j = 0; j < kBlock; j++) s.v[j] = fma(a, xv.v[j], s.v[j]);
-  }
-  V8<T> ri = ld8(r + (int64_t)i * kBlock);
-#pragma unroll
-  for (int j = 0; j < kBlock; j++) ri.v[j] = ri.v[j] - s.v[j];
-  st8(r + (int64_t)i * kBlock, ri);
-}
+// M x on the block: y = M x (restriction), y += M x (prolongation) or y -= M x (the
+// cross-partition part of the residual, preAout_kernel, gauss_seidel.cu:1977-2015).  Four
+// lanes share a row's eight columns and G such quadruples its entries (every G-th, four in
+// flight); the quadruples' sums are added by shuffles.  G grows with the average row
+// (spmm_groups): a thread per row left the restrictions, rows of 26 to 250 entries on few
+// rows, without parallelism.  64^3, restrictions of levels 0, 1, 2: 82 -> 13, 147 -> 15,
+// 83 -> 12 us.
+enum SpmmMode { SPMM_SET, SPMM_ADD, SPMM_SUB };
 
-// y = M x (accumulate = 0) or y += M x, eight columns (restriction, prolongation).
-template <class T>
-__global__ void blk_spmm_kernel(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                                const T* __restrict__ v, const T* __restrict__ x, T* __restrict__ y, int accumulate) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  V8<T> s;
+template <class T, int MODE, int G>
+__global__ void __launch_bounds__(128) blk_spmm_kernel(int n, const int32_t* __restrict__ rp,
+                                                       const int32_t* __restrict__ ci, const T* __restrict__ v,
+                                                       const T* __restrict__ x, T* __restrict__ y) {
+  constexpr int LANES = kPairs * G;
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / LANES);
+  const int t = threadIdx.x & (kPairs - 1), gr = (threadIdx.x / kPairs) & (G - 1);
+  const bool live = i < n;
+  const Pair<T>* x2 = reinterpret_cast<const Pair<T>*>(x);
+  Pair<T> s;
+  s.v[0] = s.v[1] = (T)0;
+  const int e1 = live ? rp[i + 1] : 0;
+  for (int e = live ? rp[i] + gr : 0; e < e1; e += 4 * G) {
+    int c[4];
+    T a[4];
+    Pair<T> xv[4];
 #pragma unroll
-  for (int j = 0; j < kBlock; j++) s.v[j] = (T)0;
-  for (int e = rp[i]; e < rp[i + 1]; e++) {
-    const T a = v[e];
-    const V8<T> xv = ld8(x + (int64_t)ci[e] * kBlock);
+    for (int k = 0; k < 4; k++) {
+      c[k] = e + k * G < e1 ? ci[e + k * G] : -1;
+      a[k] = e + k * G < e1 ? v[e + k * G] : (T)0;
+    }
 #pragma unroll
-    for (int j = 0; j < kBlock; j++) s.v[j] = fma(a, xv.v[j], s.v[j]);
+    for (int k = 0; k < 4; k++)
+      if (c[k] >= 0) xv[k] = x2[(int64_t)c[k] * kPairs + t];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (c[k] >= 0) {
+        s.v[0] = fma(a[k], xv[k].v[0], s.v[0]);
+        s.v[1] = fma(a[k], xv[k].v[1], s.v[1]);
+      }
   }
-  if (accumulate) {
-    const V8<T> yi = ld8(y + (int64_t)i * kBlock);
 #pragma unroll
-    for (int j = 0; j < kBlock; j++) s.v[j] = yi.v[j] + s.v[j];
+  for (int o = kPairs; o < LANES; o <<= 1) {
+    s.v[0] = s.v[0] + __shfl_xor_sync(kAll, s.v[0], o);
+    s.v[1] = s.v[1] + __shfl_xor_sync(kAll, s.v[1], o);
   }
-  st8(y + (int64_t)i * kBlock, s);
+  if (!live || gr != 0) return;
+  Pair<T>* out = reinterpret_cast<Pair<T>*>(y) + (int64_t)i * kPairs + t;
+  if (MODE != SPMM_SET) {
+    const Pair<T> o = *out;
+    s.v[0] = MODE == SPMM_ADD ? o.v[0] + s.v[0] : o.v[0] - s.v[0];
+    s.v[1] = MODE == SPMM_ADD ? o.v[1] + s.v[1] : o.v[1] - s.v[1];
+  }
+  *out = s;
 }
 
 // Coarsest level, X = Ainv B for the eight columns on the FP64 tensor cores: warp w forms
@@ -549,41 +799,94 @@ __global__ void blk_check_kernel(const double* sc, cudaGraphConditionalHandle lo
   cudaGraphSetConditional(loop, sc[G_ANY] != 0.0 ? 1u : 0u);
 }
 
-// Shared memory of blk_smooth_kernel: x twice and the right-hand side (m x 8 each), plus
-// the staged entries (values and 16-bit columns) when `ecap` > 0.
+// Shared memory of blk_smooth_large_kernel: x twice and the right-hand side (m x 8 each).
 template <class T>
-size_t blk_smooth_smem(int mcap, int ecap = 0) {
-  return (size_t)mcap * kBlock * sizeof(T) * 3 + (size_t)ecap * (sizeof(T) + 2);
+size_t blk_large_smem(int mcap) {
+  return (size_t)mcap * kBlock * sizeof(T) * 3;
 }
 
-// Entries are staged in shared memory when they fit beside the vectors.
+// Shared memory of blk_smooth_kernel for `cols` columns: x twice and the staged entries.
+template <class T>
+size_t blk_smooth_smem(const Level<T>& L, int cols) {
+  return (size_t)L.max_group_rows * cols * sizeof(T) * 2 + (size_t)L.max_group_ents * sizeof(BlkEntry<T>);
+}
+
+// Columns per CTA of blk_smooth_kernel: all eight while the groups fill the SMs twice over,
+// two otherwise (four CTAs per group); 0 when the level's groups do not fit it.
+// 64^3, level of 32 groups, pre relax: 65 us with all eight columns in a CTA (before), 35 us
+// with two, 25 us with two and four lanes per row's entries.
 constexpr size_t kBlockStageLimit = 200 * 1024;
 template <class T>
-bool blk_staged(const Level<T>& L) {
-  return L.max_group_rows < 65536 && blk_smooth_smem<T>(L.max_group_rows, L.max_group_ents) <= kBlockStageLimit;
+int blk_columns(const Level<T>& L) {
+  if (L.max_group_rows > kBlkRows) return 0;
+  if (L.ngroups >= 2 * 152 && blk_smooth_smem(L, kBlock) <= (sizeof(T) == 4 ? kBlockStageLimit / 2 : kBlockStageLimit))
+    return kBlock;
+  return blk_smooth_smem(L, 2) <= kBlockStageLimit ? 2 : 0;
+}
+
+template <class T, bool POST, int C, int LPR, int EL>
+void launch_blk_smooth_as(cudaStream_t s, const Level<T>& L, const T* b, const double* b64, T* b_store, T w, int inner,
+                          const T* x_in, T* x_out, double* z64, T* r_out) {
+  const int thr = std::min(kBlkThreads, (L.max_group_rows * LPR * EL + 31) / 32 * 32);
+  const size_t smem = blk_smooth_smem(L, C * LPR);
+  ensure_smem(blk_smooth_kernel<T, POST, C, LPR, EL>, smem);
+  FG_LAUNCH((blk_smooth_kernel<T, POST, C, LPR, EL>), L.ngroups * (kBlock / (C * LPR)), thr, smem, s, L.grows.p,
+            L.Ain.rp.p, L.Ain.ci.p, L.Ain.v.p, L.Aout.rp.p, L.Aout.ci.p, L.Aout.v.p, L.diag.p, L.dinv.p, b, b64,
+            b_store, w, inner, x_in, x_out, z64, r_out, L.max_group_rows);
 }
 
 template <class T, bool POST>
-void launch_blk_smooth(cudaStream_t s, const Level<T>& L, const T* b, T w, int inner, const T* x_in, T* x_out,
-                       T* r_out) {
-  const int thr = std::min(512, std::max(32, (L.max_group_rows + 31) / 32 * 32));
-  if (blk_staged(L)) {
-    const size_t smem = blk_smooth_smem<T>(L.max_group_rows, L.max_group_ents);
-    ensure_smem(blk_smooth_kernel<T, POST, true>, smem);
-    FG_LAUNCH((blk_smooth_kernel<T, POST, true>), L.ngroups, thr, smem, s, L.grows.p, L.Ain.rp.p, L.Ain.ci.p,
-              L.Ain.v.p, L.Aout.rp.p, L.Aout.ci.p, L.Aout.v.p, L.diag.p, L.dinv.p, b, w, inner, x_in, x_out, r_out,
-              L.max_group_rows, L.max_group_ents);
-  } else {
-    const size_t smem = blk_smooth_smem<T>(L.max_group_rows);
-    ensure_smem(blk_smooth_kernel<T, POST, false>, smem);
-    FG_LAUNCH((blk_smooth_kernel<T, POST, false>), L.ngroups, thr, smem, s, L.grows.p, L.Ain.rp.p, L.Ain.ci.p,
-              L.Ain.v.p, L.Aout.rp.p, L.Aout.ci.p, L.Aout.v.p, L.diag.p, L.dinv.p, b, w, inner, x_in, x_out, r_out,
-              L.max_group_rows, 0);
+void launch_blk_smooth(cudaStream_t s, const Level<T>& L, const T* b, const double* b64, T* b_store, T w, int inner,
+                       const T* x_in, T* x_out, double* z64, T* r_out) {
+  constexpr int C = 16 / (int)sizeof(T);  // 16-byte reads of x
+  const int cols = blk_columns(L);
+  if (cols == kBlock) {
+    launch_blk_smooth_as<T, POST, C, kBlock / C, 1>(s, L, b, b64, b_store, w, inner, x_in, x_out, z64, r_out);
+    return;
   }
+  if (cols == 2) {
+    // rows of 16 entries and more are shared by four lanes
+    if (L.Ain.nnz >= 16 * (int64_t)L.n)
+      launch_blk_smooth_as<T, POST, 2, 1, 4>(s, L, b, b64, b_store, w, inner, x_in, x_out, z64, r_out);
+    else
+      launch_blk_smooth_as<T, POST, 2, 1, 1>(s, L, b, b64, b_store, w, inner, x_in, x_out, z64, r_out);
+    return;
+  }
+  const int thr = std::min(512, std::max(32, (L.max_group_rows + 31) / 32 * 32));
+  const size_t smem = blk_large_smem<T>(L.max_group_rows);
+  ensure_smem(blk_smooth_large_kernel<T, POST>, smem);
+  FG_LAUNCH((blk_smooth_large_kernel<T, POST>), L.ngroups, thr, smem, s, L.grows.p, L.Ain.rp.p, L.Ain.ci.p, L.Ain.v.p,
+            L.Aout.rp.p, L.Aout.ci.p, L.Aout.v.p, L.diag.p, L.dinv.p, b, b64, b_store, w, inner, x_in, x_out, z64,
+            r_out, L.max_group_rows);
 }
 
+// Quadruples of lanes per row of blk_spmm_kernel: each takes about eight entries of an
+// average row (two rounds of its four loads in flight).
 template <class T>
-void block_vcycle(Ctx& c, Hierarchy<T>& H, BlockState<T>& S, int l, T* b_in, T* x_out) {
+int spmm_groups(const DCsr<T>& M) {
+  const double avg = M.n > 0 ? (double)M.nnz / M.n : 0.0;
+  return avg <= 8.0 ? 1 : avg <= 16.0 ? 2 : avg <= 32.0 ? 4 : 8;
+}
+
+template <class T, int MODE>
+void launch_blk_spmm(cudaStream_t s, const DCsr<T>& M, const T* x, T* y) {
+  const int G = spmm_groups(M);
+  const int g = grid_for((int64_t)M.n * kPairs * G, 128);
+#define FG_SPMM(GG) FG_LAUNCH((blk_spmm_kernel<T, MODE, GG>), g, 128, 0, s, M.n, M.rp.p, M.ci.p, M.v.p, x, y)
+  switch (G) {
+    case 1: FG_SPMM(1); break;
+    case 2: FG_SPMM(2); break;
+    case 4: FG_SPMM(4); break;
+    default: FG_SPMM(8); break;
+  }
+#undef FG_SPMM
+}
+
+// b_in -> x_out; at level 0 with r64 the right-hand side is read from r64 in FP64 (and its
+// rounded copy kept in b_in), with z64 the result goes there in FP64.
+template <class T>
+void block_vcycle(Ctx& c, Hierarchy<T>& H, BlockState<T>& S, int l, T* b_in, T* x_out, const double* r64 = nullptr,
+                  double* z64 = nullptr) {
   cudaStream_t s = c.stream;
   Level<T>& L = *H.L[l];
   const int n = L.A.n;
@@ -594,21 +897,27 @@ void block_vcycle(Ctx& c, Hierarchy<T>& H, BlockState<T>& S, int l, T* b_in, T* 
   BlockLevel<T>& W = S.lv[l];
   const T w = (T)c.cfg.smootherWeight;
   // pre relax: x, r = b - A_in x - d x, then r -= A_out x
-  launch_blk_smooth<T, false>(s, L, b_in, w, c.cfg.preInnerIters, (const T*)nullptr, W.x.p, W.r.p);
-  FG_LAUNCH(blk_aout_kernel<T>, grid_for(n, 128), 128, 0, s, n, L.Aout.rp.p, L.Aout.ci.p, L.Aout.v.p, W.x.p, W.r.p);
+  launch_blk_smooth<T, false>(s, L, b_in, r64, b_in, w, c.cfg.preInnerIters, (const T*)nullptr, W.x.p,
+                              (double*)nullptr, W.r.p);
+  launch_blk_spmm<T, SPMM_SUB>(s, L.Aout, W.x.p, W.r.p);
   BlockLevel<T>& NW = S.lv[l + 1];
-  FG_LAUNCH(blk_spmm_kernel<T>, grid_for(L.R.n, 128), 128, 0, s, L.R.n, L.R.rp.p, L.R.ci.p, L.R.v.p, W.r.p, NW.t.p,
-            0);
+  launch_blk_spmm<T, SPMM_SET>(s, L.R, W.r.p, NW.t.p);
   block_vcycle(c, H, S, l + 1, NW.t.p, NW.xo.p);
-  FG_LAUNCH(blk_spmm_kernel<T>, grid_for(n, 128), 128, 0, s, n, L.P.rp.p, L.P.ci.p, L.P.v.p, NW.xo.p, W.x.p, 1);
+  launch_blk_spmm<T, SPMM_ADD>(s, L.P, NW.xo.p, W.x.p);
   T* src = W.x.p;
   for (int rl = 0; rl < c.cfg.postRelaxes; rl++) {
-    T* dst = (rl + 1 == c.cfg.postRelaxes) ? x_out : (src == W.x.p ? W.r.p : W.x.p);
-    launch_blk_smooth<T, true>(s, L, b_in, w, c.cfg.postInnerIters, src, dst, (T*)nullptr);
+    const bool last = rl + 1 == c.cfg.postRelaxes;
+    T* dst = last ? x_out : (src == W.x.p ? W.r.p : W.x.p);
+    launch_blk_smooth<T, true>(s, L, b_in, (const double*)nullptr, (T*)nullptr, w, c.cfg.postInnerIters, src, dst,
+                               last ? z64 : (double*)nullptr, (T*)nullptr);
     src = dst;
   }
-  if (c.cfg.postRelaxes == 0)
-    FG_CUDA(cudaMemcpyAsync(x_out, W.x.p, (size_t)n * kBlock * sizeof(T), cudaMemcpyDeviceToDevice, s));
+  if (c.cfg.postRelaxes == 0) {
+    if (z64)
+      FG_LAUNCH(blk_cast_out_kernel<T>, grid_for((int64_t)n * kBlock, 256), 256, 0, s, (int64_t)n * kBlock, W.x.p, z64);
+    else
+      FG_CUDA(cudaMemcpyAsync(x_out, W.x.p, (size_t)n * kBlock * sizeof(T), cudaMemcpyDeviceToDevice, s));
+  }
 }
 
 template <class T>
@@ -630,7 +939,7 @@ BlockState<T>& block_state(Ctx& c, Hierarchy<T>& H) {
       W.t.alloc(m, s);
       if (!L.coarsest) {
         W.r.alloc(m, s);
-        const size_t smem = blk_smooth_smem<T>(L.max_group_rows);
+        const size_t smem = blk_large_smem<T>(L.max_group_rows);
         FG_REQUIRE(smem <= 227 * 1024, FEMGPU_ERR_LIMIT,
                    "a smoother group is too large for the multi-right-hand-side smoother's shared memory");
       }
@@ -655,10 +964,12 @@ void block_precondition(Ctx& c, Hierarchy<T>& H, BlockState<T>& S, const double*
   BlockLevel<T>& W = S.lv[0];
   if constexpr (std::is_same<T, double>::value) {
     block_vcycle(c, H, S, 0, const_cast<double*>(r), z);  // the V-cycle only reads its input
-  } else {
+  } else if (H.L[0]->coarsest) {
     FG_LAUNCH(blk_cast_in_kernel<T>, grid_for(m, 256), 256, 0, s, m, r, W.b.p);
     block_vcycle(c, H, S, 0, W.b.p, W.xo.p);
     FG_LAUNCH(blk_cast_out_kernel<T>, grid_for(m, 256), 256, 0, s, m, W.xo.p, z);
+  } else {
+    block_vcycle(c, H, S, 0, W.b.p, W.xo.p, r, z);  // level 0 reads r and writes z itself
   }
 }
 
@@ -683,8 +994,8 @@ void block_solve_columns(Ctx& c, Hierarchy<T>& H, int kc, const double* B, int64
   FG_CUDA(cudaMemsetAsync(S.vp.p, 0, S.vp.n * sizeof(double), s));
   FG_LAUNCH(blk_dot_kernel, kBG, kBT, 0, s, n, S.vb.p, S.vb.p, (const double*)nullptr, part, sc, (int)B_BN, 0,
             S.cnt.p);
-  FG_LAUNCH(blk_spmv_kernel, grid_for(n, 128), 128, 0, s, n, off, rp, ci, v, S.vx.p, S.vy.p);
-  FG_LAUNCH(blk_sub_kernel, grid_for(n, 256), 256, 0, s, n, S.vb.p, S.vy.p, S.vr.p);
+  FG_LAUNCH(blk_spmv_kernel, grid_for((int64_t)n * kPairs, 256), 256, 0, s, n, off, rp, ci, v, S.vx.p, S.vy.p);
+  FG_LAUNCH(blk_sub_kernel, grid_for((int64_t)n * kPairs, 256), 256, 0, s, n, S.vb.p, S.vy.p, S.vr.p);
   FG_LAUNCH(blk_dot_kernel, kBG, kBT, 0, s, n, S.vr.p, S.vr.p, (const double*)nullptr, part, sc, (int)B_NR, 0,
             S.cnt.p);
   FG_CUDA(cudaMemcpyAsync(S.h_sc, sc, G_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -711,7 +1022,7 @@ void block_solve_columns(Ctx& c, Hierarchy<T>& H, int kc, const double* B, int64
     FG_LAUNCH(blk_dot_kernel, kBG, kBT, 0, s, n, S.vz.p, S.vr.p, flexible ? (const double*)S.vrold.p : nullptr, part,
               sc, (int)B_RZNEW, (int)B_ZROLD, S.cnt.p);
     FG_LAUNCH(blk_beta_kernel, 1, kBlock, 0, s, sc);
-    FG_LAUNCH(blk_pupdate_kernel, grid_for(n, 256), 256, 0, s, n, sc, S.vz.p, S.vp.p);
+    FG_LAUNCH(blk_pupdate_kernel, grid_for((int64_t)n * kPairs, 256), 256, 0, s, n, sc, S.vz.p, S.vp.p);
     FG_LAUNCH(blk_spmv_dot_kernel, kBG, kBT, 0, s, n, off, rp, ci, v, S.vp.p, S.vy.p, part, sc, S.cnt.p + 1);
     FG_LAUNCH(blk_update_kernel, kBG, kBT, 0, s, n, sc, S.vp.p, S.vy.p, S.vx.p, S.vr.p,
               flexible ? S.vrold.p : nullptr, part, S.cnt.p + 2);
