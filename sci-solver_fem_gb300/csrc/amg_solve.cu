@@ -39,8 +39,17 @@ thread_local bool t_pdl_scope = false;
 
 namespace {
 
-constexpr int kRedBlocks = 608;  // 4 x 152 SMs: fixed grid for deterministic reductions
+constexpr int kRedBlocks = 608;  // 4 x 152 SMs: largest grid of the reductions
 constexpr int kRedThreads = 256;
+
+// Blocks of the reduction kernels for n elements: the largest grid, or a thread per element
+// where that is less.  Blocks past the last element would only add zeros (the same bits), but
+// each costs a block sum and a ticket: 2,744 rows, 608 -> 11 blocks, product with its dot
+// 10.2 -> @RG1@ us, update 8.5 -> @RG2@ us.
+inline int red_blocks(int n) {
+  const int g = (n + kRedThreads - 1) / kRedThreads;
+  return g < 1 ? 1 : g < kRedBlocks ? g : kRedBlocks;
+}
 
 // device scalar slots in Ctx::red (after the partials)
 enum Slot {
@@ -814,6 +823,8 @@ __device__ double ordered_total(const double* partial, int nparts, double* sh) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   // a warp stands in for up to 4 virtual warps per pass; their first partials are
   // loaded together (one L2 round trip) before the adds and butterflies
+  // (virtual warps past the last partial sum to 0: their butterflies, 5 double-precision adds
+  // of 64 cycles each, are left out)
   for (int vw0 = w; vw0 < 32; vw0 += 4 * nw) {
     double v[4];
 #pragma unroll
@@ -825,9 +836,11 @@ __device__ double ordered_total(const double* partial, int nparts, double* sh) {
     for (int m = 0; m < 4; m++) {
       const int vw = vw0 + m * nw;
       if (vw < 32) {
-        for (int q = vw * 32 + lane + 1024; q < nparts; q += 1024) v[m] += partial[q];
+        if (vw * 32 < nparts) {
+          for (int q = vw * 32 + lane + 1024; q < nparts; q += 1024) v[m] += partial[q];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[m] += __shfl_xor_sync(0xffffffffu, v[m], o);
+          for (int o = 16; o > 0; o >>= 1) v[m] += __shfl_xor_sync(0xffffffffu, v[m], o);
+        }
         if (lane == 0) sh[vw] = v[m];
       }
     }
@@ -877,10 +890,24 @@ __global__ void residual_kernel(int n, const double* __restrict__ b, const doubl
 
 
 
-// x += alpha p; r -= alpha y (rold = r first when flexible); partial ||r||^2
+// The device-side PCG loop after an iteration: counts it and stops the loop on convergence (the host's test:
+// sqrt(r.r) / |b| <= tol), breakdown, a non-finite residual, a smoother copy that timed out,
+// or maxIters.
+__device__ __forceinline__ void pcg_check(double* sc, cudaGraphConditionalHandle loop) {
+  const double it = sc[S_IT] + 1.0;
+  sc[S_IT] = it;
+  const double nr = sqrt(sc[S_NR]);
+  const bool stop = sc[S_FLAG] != 0.0 || sc[S_KERR] != 0.0 || !isfinite(nr) || nr / sc[S_BNORM] <= sc[S_TOL] ||
+                    it >= sc[S_MAXIT];
+  cudaGraphSetConditional(loop, stop ? 0u : 1u);
+}
+
+// x += alpha p; r -= alpha y (rold = r first when flexible); partial ||r||^2; in a device-side
+// loop (in_loop) the last block also decides whether another iteration runs.
 __global__ void update_kernel(int n, double* __restrict__ sc, const double* __restrict__ p,
                               const double* __restrict__ y, double* __restrict__ x, double* __restrict__ r,
-                              double* __restrict__ rold, double* partial, unsigned* counter) {
+                              double* __restrict__ rold, double* partial, unsigned* counter, int in_loop,
+                              cudaGraphConditionalHandle loop) {
   pdl_enter();
   __shared__ double sh[32];
   const double alpha = sc[S_ALPHA];
@@ -922,6 +949,7 @@ __global__ void update_kernel(int n, double* __restrict__ sc, const double* __re
   if (threadIdx.x == 0) {
     sc[S_NR] = nr;
     *counter = 0u;
+    if (in_loop) pcg_check(sc, loop);
   }
 }
 
@@ -1071,19 +1099,6 @@ __global__ void dot_beta_kernel(int n, const double* __restrict__ z, const doubl
     beta_update(sc, flexible);
     *counter = 0u;
   }
-}
-
-// Continue the device-side PCG loop?  Stops on convergence (the host's test:
-// sqrt(r.r) / |b| <= tol), breakdown, a non-finite residual, a smoother copy that
-// timed out, or maxIters.
-__global__ void pcg_check_kernel(double* sc, cudaGraphConditionalHandle loop) {
-  pdl_enter();
-  const double it = sc[S_IT] + 1.0;
-  sc[S_IT] = it;
-  const double nr = sqrt(sc[S_NR]);
-  const bool stop = sc[S_FLAG] != 0.0 || sc[S_KERR] != 0.0 || !isfinite(nr) || nr / sc[S_BNORM] <= sc[S_TOL] ||
-                    it >= sc[S_MAXIT];
-  cudaGraphSetConditional(loop, stop ? 0u : 1u);
 }
 
 __global__ void set_slot_kernel(double* sc, int slot, double v) { sc[slot] = v; }
@@ -2002,16 +2017,14 @@ void amg_vcycle_device(Ctx& c, const double* d_r, double* d_z) {
 
 namespace {
 
-// One PCG iteration after the residual check: z = M r, beta, p = z + beta p,
-// y = A p, alpha, x += alpha p, r -= alpha y, ||r||^2, scalars to the host.
 // y = A0p p with p.y and alpha.
 void launch_spmv_dot(Ctx& c, int n, const double* p, double* y) {
   const DCsr<double>& A = c.A0p;
   if (c.sliced)
-    FG_LAUNCH_PDL(spmv_dot_sliced_kernel, kRedBlocks, kRedThreads, 0, c.stream, n, c.s_off.p, c.s_ci.p, c.s_v.p, p, y,
+    FG_LAUNCH_PDL(spmv_dot_sliced_kernel, red_blocks(n), kRedThreads, 0, c.stream, n, c.s_off.p, c.s_ci.p, c.s_v.p, p, y,
               c.red.p, c.red.p + 2 * kRedBlocks, c.rcount.p + 1);
   else
-    FG_LAUNCH_PDL(spmv_dot_kernel, kRedBlocks, kRedThreads, 0, c.stream, n, A.rp.p, A.ci.p, A.v.p, p, y, c.red.p,
+    FG_LAUNCH_PDL(spmv_dot_kernel, red_blocks(n), kRedThreads, 0, c.stream, n, A.rp.p, A.ci.p, A.v.p, p, y, c.red.p,
               c.red.p + 2 * kRedBlocks, c.rcount.p + 1);
 }
 
@@ -2024,7 +2037,11 @@ void launch_spmv_a0(Ctx& c, int n, const double* x, double* y) {
     FG_LAUNCH(spmv_kernel, grid_for(n, 256), 256, 0, c.stream, n, A.rp.p, A.ci.p, A.v.p, x, y);
 }
 
-void pcg_iteration_body(Ctx& c, int n, int flexible, bool to_host) {
+// One PCG iteration after the residual check: z = M r, beta, p = z + beta p, y = A p, alpha,
+// x += alpha p, r -= alpha y, ||r||^2; then the scalars go to the host, or (with loop) the
+// device decides whether another iteration runs.
+void pcg_iteration_body(Ctx& c, int n, int flexible, const cudaGraphConditionalHandle* loop) {
+  const PdlScope pdl_scope(n <= kPdlLevelRows);  // the vector kernels of small problems, as their V-cycle's
   cudaStream_t s = c.stream;
   double* part = c.red.p;
   double* part2 = c.red.p + kRedBlocks;
@@ -2043,20 +2060,20 @@ void pcg_iteration_body(Ctx& c, int n, int flexible, bool to_host) {
   }
   c.zdot = nullptr;
   if (!zd.done)  // else z.r (z.r_old) and beta came from the smoother that wrote z
-    FG_LAUNCH_PDL(dot_beta_kernel, kRedBlocks, kRedThreads, 0, s, n, c.vz.p, c.vr.p, flexible ? c.vrold.p : nullptr,
+    FG_LAUNCH_PDL(dot_beta_kernel, red_blocks(n), kRedThreads, 0, s, n, c.vz.p, c.vr.p, flexible ? c.vrold.p : nullptr,
               part, part2, sc, flexible, cnt);
-  FG_LAUNCH_PDL(pupdate_kernel, kRedBlocks, kRedThreads, 0, s, n, sc, c.vz.p, c.vp.p);
+  FG_LAUNCH_PDL(pupdate_kernel, red_blocks(n), kRedThreads, 0, s, n, sc, c.vz.p, c.vp.p);
   launch_spmv_dot(c, n, c.vp.p, c.vy.p);
-  FG_LAUNCH_PDL(update_kernel, kRedBlocks, kRedThreads, 0, s, n, sc, c.vp.p, c.vy.p, c.vx.p, c.vr.p,
-            flexible ? c.vrold.p : nullptr, part, cnt + 2);
-  if (to_host) FG_CUDA(cudaMemcpyAsync(c.h_scalars, sc, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s));
+  FG_LAUNCH_PDL(update_kernel, red_blocks(n), kRedThreads, 0, s, n, sc, c.vp.p, c.vy.p, c.vx.p, c.vr.p,
+            flexible ? c.vrold.p : nullptr, part, cnt + 2, loop ? 1 : 0, loop ? *loop : cudaGraphConditionalHandle());
+  if (!loop) FG_CUDA(cudaMemcpyAsync(c.h_scalars, sc, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s));
 }
 
 // Captures the whole PCG loop once per hierarchy as a CUDA graph: a conditional while
-// node whose body is one iteration followed by pcg_check_kernel, so the iterations
-// run back to back on the device with no host round trip.
+// node whose body is one iteration, whose last kernel decides about the next, so the
+// iterations run back to back on the device with no host round trip.
 // Adds to `g` a while node on `loop` after `deps` and captures its body on c.stream: one
-// PCG iteration followed by pcg_check_kernel.  Returns the node, or null when a graph call
+// PCG iteration.  Returns the node, or null when a graph call
 // or the capture failed (the capture is ended either way).
 cudaGraphNode_t add_pcg_loop(Ctx& c, int n, int flexible, cudaGraph_t g, cudaGraphConditionalHandle loop,
                              const cudaGraphNode_t* deps, size_t ndeps) {
@@ -2072,8 +2089,7 @@ cudaGraphNode_t add_pcg_loop(Ctx& c, int n, int flexible, cudaGraph_t g, cudaGra
   if (cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
     return nullptr;
   try {
-    pcg_iteration_body(c, n, flexible, false);
-    FG_LAUNCH_PDL(pcg_check_kernel, 1, 1, 0, s, c.red.p + 2 * kRedBlocks, loop);
+    pcg_iteration_body(c, n, flexible, &loop);
   } catch (...) {
     cudaGraph_t dummy = nullptr;
     cudaStreamEndCapture(s, &dummy);
@@ -2139,10 +2155,10 @@ SolveResult amg_solve_device(Ctx& c, const double* d_b, double* d_x) {
     precondition_any(c, c.vb.p, c.vx.p);
     FG_LAUNCH(perm_vec_out_kernel, grid_for(n, 256), 256, 0, s, n, c.perm0.p, c.vx.p, d_x);
     launch_spmv_a0(c, n, c.vx.p, c.vy.p);
-    FG_LAUNCH(residual_kernel, kRedBlocks, kRedThreads, 0, s, n, c.vb.p, c.vy.p, c.vr.p, part);
-    FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, kRedBlocks, sc + S_NR);
-    FG_LAUNCH(dot_kernel, kRedBlocks, kRedThreads, 0, s, n, c.vb.p, c.vb.p, nullptr, part, nullptr);
-    FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, kRedBlocks, sc + S_BN);
+    FG_LAUNCH(residual_kernel, red_blocks(n), kRedThreads, 0, s, n, c.vb.p, c.vy.p, c.vr.p, part);
+    FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, red_blocks(n), sc + S_NR);
+    FG_LAUNCH(dot_kernel, red_blocks(n), kRedThreads, 0, s, n, c.vb.p, c.vb.p, nullptr, part, nullptr);
+    FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, red_blocks(n), sc + S_BN);
     FG_CUDA(cudaMemcpyAsync(c.h_scalars, sc, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s));
     FG_CUDA(cudaStreamSynchronize(s));
     double bn = sqrt(c.h_scalars[S_BN]);
@@ -2151,11 +2167,11 @@ SolveResult amg_solve_device(Ctx& c, const double* d_b, double* d_x) {
     return res;
   }
   const int flexible = c.cfg.flexibleCG;
-  FG_LAUNCH(dot_kernel, kRedBlocks, kRedThreads, 0, s, n, c.vb.p, c.vb.p, nullptr, part, nullptr);
-  FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, kRedBlocks, sc + S_BN);
+  FG_LAUNCH(dot_kernel, red_blocks(n), kRedThreads, 0, s, n, c.vb.p, c.vb.p, nullptr, part, nullptr);
+  FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, red_blocks(n), sc + S_BN);
   launch_spmv_a0(c, n, c.vx.p, c.vy.p);
-  FG_LAUNCH(residual_kernel, kRedBlocks, kRedThreads, 0, s, n, c.vb.p, c.vy.p, c.vr.p, part);
-  FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, kRedBlocks, sc + S_NR);
+  FG_LAUNCH(residual_kernel, red_blocks(n), kRedThreads, 0, s, n, c.vb.p, c.vy.p, c.vr.p, part);
+  FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, red_blocks(n), sc + S_NR);
   FG_LAUNCH(set_slot_kernel, 1, 1, 0, s, sc, S_FLAG, 0.0);
   FG_LAUNCH(set_slot_kernel, 1, 1, 0, s, sc, S_FIRST, 1.0);
   FG_LAUNCH(set_slot_kernel, 1, 1, 0, s, sc, S_KERR, 0.0);
@@ -2177,7 +2193,7 @@ SolveResult amg_solve_device(Ctx& c, const double* d_b, double* d_x) {
     // which profilers can list kernel by kernel
     const bool graph = c.cfg.maxIters > 0 && !getenv("FEMGPU_HOST_LOOP") && capture_iteration(c, n, flexible);
     if (graph) {
-      // the device runs the iterations until pcg_check_kernel stops the loop
+      // the device runs the iterations until pcg_check stops the loop
       FG_LAUNCH(set_slot_kernel, 1, 1, 0, s, sc, S_IT, 0.0);
       FG_LAUNCH(set_slot_kernel, 1, 1, 0, s, sc, S_BNORM, bnorm);
       FG_LAUNCH(set_slot_kernel, 1, 1, 0, s, sc, S_TOL, tol);
@@ -2193,7 +2209,7 @@ SolveResult amg_solve_device(Ctx& c, const double* d_b, double* d_x) {
       else if (nr / bnorm <= tol) res.status = FEMGPU_OK;
     } else {
       while (it < c.cfg.maxIters) {
-        pcg_iteration_body(c, n, flexible, true);
+        pcg_iteration_body(c, n, flexible, nullptr);
         FG_CUDA(cudaStreamSynchronize(s));
         it++;
         nr = sqrt(c.h_scalars[S_NR]);
@@ -2262,11 +2278,11 @@ bool add_batch_branch(Ctx& c, cudaGraph_t g, int64_t* body_kernels, int64_t* fix
   try {
     FG_LAUNCH(perm_vec_in_kernel, grid_for(n, 256), 256, 0, s, n, c.perm0.p, c.bat_b.p, c.vb.p);
     FG_LAUNCH(perm_vec_in_kernel, grid_for(n, 256), 256, 0, s, n, c.perm0.p, c.bat_x.p, c.vx.p);
-    FG_LAUNCH(dot_kernel, kRedBlocks, kRedThreads, 0, s, n, c.vb.p, c.vb.p, nullptr, part, nullptr);
-    FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, kRedBlocks, sc + S_BN);
+    FG_LAUNCH(dot_kernel, red_blocks(n), kRedThreads, 0, s, n, c.vb.p, c.vb.p, nullptr, part, nullptr);
+    FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, red_blocks(n), sc + S_BN);
     launch_spmv_a0(c, n, c.vx.p, c.vy.p);
-    FG_LAUNCH(residual_kernel, kRedBlocks, kRedThreads, 0, s, n, c.vb.p, c.vy.p, c.vr.p, part);
-    FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, kRedBlocks, sc + S_NR);
+    FG_LAUNCH(residual_kernel, red_blocks(n), kRedThreads, 0, s, n, c.vb.p, c.vy.p, c.vr.p, part);
+    FG_LAUNCH(finalize_kernel, 1, 1024, 0, s, part, red_blocks(n), sc + S_NR);
     FG_LAUNCH(set_slot_kernel, 1, 1, 0, s, sc, S_FLAG, 0.0);
     FG_LAUNCH(set_slot_kernel, 1, 1, 0, s, sc, S_FIRST, 1.0);
     FG_LAUNCH(set_slot_kernel, 1, 1, 0, s, sc, S_KERR, 0.0);
@@ -2450,7 +2466,7 @@ void profile_level0(Ctx& c, Hierarchy<T>& H, int which, int reps, double* ms, do
         }
         c.zdot = nullptr;
         if (!zd.done)
-          FG_LAUNCH_PDL(dot_beta_kernel, kRedBlocks, kRedThreads, 0, s, n, c.vz.p, c.vr.p, c.vrold.p, c.red.p,
+          FG_LAUNCH_PDL(dot_beta_kernel, red_blocks(n), kRedThreads, 0, s, n, c.vz.p, c.vr.p, c.vrold.p, c.red.p,
                     c.red.p + kRedBlocks, c.red.p + 2 * kRedBlocks, 1, c.rcount.p);
         break;
       }
