@@ -111,6 +111,7 @@ struct Level {
   // shared-memory smoother plan: lanes per row, CTAs per cluster (one cluster per
   // group), rows and entries of the largest CTA row slice, launch shape
   int smooth_lanes = 1, cluster = 1, slice_rows = 0, slice_ents = 0, smooth_threads = 0, smooth_grid = 0;
+  int split = 1;     // register smoother: CTAs per group (a cluster) when greater than 1
   int smooth_k = 0;  // entries per lane of the register-resident cluster smoother (0: not used)
   bool smooth_staged = false;
   size_t smooth_smem = 0;
