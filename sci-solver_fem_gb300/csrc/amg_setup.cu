@@ -200,7 +200,7 @@ void random_mis(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int k, D
       FG_LAUNCH(mis_iterate_kernel, grid_for(n, 256), 256, 0, s, n, ki, ko, xadj, adj, mis.p, flag.p, it == k - 1);
       std::swap(ki, ko);
     }
-    if (ki != k0.p) std::swap(k0.p, k1.p);  // keep k0 as the next round's input
+    if (ki != k0.p) std::swap(k0, k1);  // keep k0 as the next round's input
     if ((round + 1) % batch != 0) continue;
     if (read_scalar(flag.p, s) == 0) break;
     pt.mark("mis rounds");
@@ -794,7 +794,7 @@ void aggregate_small(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int
   if (h[0] == AGG_LOOP_CAP) throw Error(FEMGPU_ERR_LIMIT, "aggregation did not complete");
   if (h[0] == AGG_RESTRICT_CAP) throw Error(FEMGPU_ERR_LIMIT, "partition size restriction did not converge");
   if (h[0] == AGG_STALLED) throw_stalled();
-  if (h[3]) std::swap(part.p, pout.p);
+  if (h[3]) std::swap(part, pout);
   *count = h[1];
   *labels = h[2];
 }
@@ -831,7 +831,7 @@ int aggregate(Ctx& c, int n, int64_t edges, const int32_t* xadj, const int32_t* 
       counters.zero();
       FG_LAUNCH(allocate_kernel, grid_for(n, 256), 256, 0, s, n, xadj, adj, part.p, pout.p, aggregated.p,
                 counters.p);
-      std::swap(part.p, pout.p);
+      std::swap(part, pout);
     }
     int32_t h[2];
     counters.download(h, 2);
@@ -3186,6 +3186,7 @@ __global__ void identity_kernel(int n, int32_t* p) {
 std::atomic<int64_t> g_kernel_launches{0};
 std::atomic<int64_t> g_host_syncs{0};
 thread_local cudaMemPool_t g_alloc_pool = nullptr;
+thread_local BlockCache* g_alloc_cache = nullptr;
 
 // Values of perm(A) on its (sorted) pattern: row i' and column j' of the permuted
 // matrix are row iperm[i'] and column iperm[j'] of A, found by binary search.

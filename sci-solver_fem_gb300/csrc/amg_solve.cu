@@ -1682,7 +1682,7 @@ void l1_sweeps(Ctx& c, Level<T>& L, const T* b, int sweeps) {
   for (int it = 0; it < sweeps; it++) {
     FG_LAUNCH_PDL(l1_sweep_kernel<T>, grid_for(L.n, 256), 256, 0, c.stream, L.n, L.Ap.rp.p, L.Ap.ci.p, L.Ap.v.p, b,
               L.l1inv.p, w, L.x.p, L.r.p);
-    std::swap(L.x.p, L.r.p);
+    std::swap(L.x, L.r);
   }
 }
 
@@ -1760,7 +1760,7 @@ void vcycle(Ctx& c, Hierarchy<T>& H, int l, T* b_in, T* x_out, double* z_out = n
     double* z64 = (l == 0 && z_out && last) ? z_out : nullptr;
     T* dst = (l > 0 && last) ? x_out : L.r.p;
     smooth<T>(c, L, true, b, L.x.p, dst, nullptr, nullptr, nullptr, z64);
-    if (dst == L.r.p) std::swap(L.x.p, L.r.p);  // r is free after the restriction: the ping-pong buffer
+    if (dst == L.r.p) std::swap(L.x, L.r);  // r is free after the restriction: the ping-pong buffer
     z_done = z64 != nullptr;
     out_done = dst == x_out;
   }

@@ -21,11 +21,18 @@ namespace {
 
 thread_local std::string g_last_global_error;
 
-// Routes the handle's allocations to its pool for the duration of one call.
+// Routes the handle's allocations to its pool and cache for the duration of one call.
 struct PoolScope {
   cudaMemPool_t saved;
-  explicit PoolScope(femgpu_handle h) : saved(g_alloc_pool) { g_alloc_pool = h ? h->pool : nullptr; }
-  ~PoolScope() { g_alloc_pool = saved; }
+  BlockCache* saved_cache;
+  explicit PoolScope(femgpu_handle h) : saved(g_alloc_pool), saved_cache(g_alloc_cache) {
+    g_alloc_pool = h ? h->pool : nullptr;
+    g_alloc_cache = h ? &h->cache : nullptr;
+  }
+  ~PoolScope() {
+    g_alloc_pool = saved;
+    g_alloc_cache = saved_cache;
+  }
 };
 
 // Runs fn for an entry point: the handle's memory pool and device, exceptions turned into
@@ -220,6 +227,7 @@ femgpu_status femgpu_create(femgpu_handle* out, const femgpu_config* cfg) {
       FG_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
       h->own_stream = true;
     }
+    h->cache.stream = h->stream;
     if (h->cfg.mem_pool) {
       h->pool = (cudaMemPool_t)h->cfg.mem_pool;
     } else {

@@ -62,21 +62,68 @@ struct Error : std::runtime_error {
 // C ABI around each call); null = the device's current pool.
 extern thread_local cudaMemPool_t g_alloc_pool;
 
+// Small freed buffers of one handle, kept by size class (powers of two up to 1 MB, at most
+// 32 MB in all) for its next allocations on its stream: a setup makes about 100 short-lived
+// buffers per level, and each trip to the driver's pool costs the host 0.5-1 us, as much as
+// a launch.  Stream order makes the reuse safe (one stream, one thread at a time per handle).
+// Given back with the handle, and before an allocation is allowed to fail.
+struct BlockCache {
+  static constexpr size_t kLargest = size_t(1) << 20, kMost = size_t(32) << 20;
+  static constexpr int kClasses = 13;  // 256 B .. 1 MB
+  cudaStream_t stream = 0;
+  std::vector<void*> kept[kClasses];
+  size_t bytes = 0;
+  static int class_of(size_t b) {
+    int c = 0;
+    while ((size_t(256) << c) < b) c++;
+    return c;
+  }
+  static size_t class_bytes(int c) { return size_t(256) << c; }
+  void* take(int c) {
+    if (kept[c].empty()) return nullptr;
+    void* p = kept[c].back();
+    kept[c].pop_back();
+    bytes -= class_bytes(c);
+    return p;
+  }
+  void give(void* p, int c) {
+    if (bytes + class_bytes(c) > kMost) {
+      cudaFreeAsync(p, stream);
+      return;
+    }
+    kept[c].push_back(p);
+    bytes += class_bytes(c);
+  }
+  void release() {
+    for (auto& k : kept) {
+      for (void* p : k) cudaFreeAsync(p, stream);
+      k.clear();
+    }
+    bytes = 0;
+  }
+  ~BlockCache() { release(); }
+};
+
+// Cache of the handle whose entry point is running on this thread (set with g_alloc_pool).
+extern thread_local BlockCache* g_alloc_cache;
+
 // Stream-ordered device buffer.
 template <class T>
 struct DBuf {
   T* p = nullptr;
   size_t n = 0;
   cudaStream_t s = 0;
+  BlockCache* cache = nullptr;  // where a small buffer goes back to (its handle's, which outlives it)
+  int cls = 0;
   DBuf() = default;
   DBuf(size_t count, cudaStream_t st) { alloc(count, st); }
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
-  DBuf(DBuf&& o) noexcept : p(o.p), n(o.n), s(o.s) { o.p = nullptr; o.n = 0; }
+  DBuf(DBuf&& o) noexcept : p(o.p), n(o.n), s(o.s), cache(o.cache), cls(o.cls) { o.p = nullptr; o.n = 0; }
   DBuf& operator=(DBuf&& o) noexcept {
     if (this != &o) {
       release();
-      p = o.p; n = o.n; s = o.s;
+      p = o.p; n = o.n; s = o.s; cache = o.cache; cls = o.cls;
       o.p = nullptr; o.n = 0;
     }
     return *this;
@@ -86,19 +133,36 @@ struct DBuf {
     release();
     s = st;
     n = count;
-    if (count) {
-      cudaError_t e = g_alloc_pool ? cudaMallocFromPoolAsync((void**)&p, count * sizeof(T), g_alloc_pool, st)
-                                   : cudaMallocAsync((void**)&p, count * sizeof(T), st);
-      if (e != cudaSuccess) {
-        p = nullptr;
-        n = 0;
-        (void)cudaGetLastError();
-        throw Error(FEMGPU_ERR_ALLOC, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
-      }
+    if (!count) return;
+    const size_t bytes = count * sizeof(T);
+    cache = g_alloc_cache && g_alloc_cache->stream == st && bytes <= BlockCache::kLargest ? g_alloc_cache : nullptr;
+    if (cache) {
+      cls = BlockCache::class_of(bytes);
+      if ((p = static_cast<T*>(cache->take(cls)))) return;
+    }
+    cudaError_t e = from_pool(cache ? BlockCache::class_bytes(cls) : bytes);
+    if (e != cudaSuccess && g_alloc_cache) {  // give the kept buffers back and ask for the bare size
+      (void)cudaGetLastError();
+      g_alloc_cache->release();
+      cache = nullptr;
+      e = from_pool(bytes);
+    }
+    if (e != cudaSuccess) {
+      p = nullptr;
+      n = 0;
+      (void)cudaGetLastError();
+      throw Error(FEMGPU_ERR_ALLOC, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
     }
   }
+  cudaError_t from_pool(size_t bytes) {
+    return g_alloc_pool ? cudaMallocFromPoolAsync((void**)&p, bytes, g_alloc_pool, s)
+                        : cudaMallocAsync((void**)&p, bytes, s);
+  }
   void release() {
-    if (p) cudaFreeAsync(p, s);
+    if (p) {
+      if (cache) cache->give(p, cls);
+      else cudaFreeAsync(p, s);
+    }
     p = nullptr;
     n = 0;
   }

@@ -179,6 +179,7 @@ struct BlockStateBase {
 };
 
 struct Ctx {
+  BlockCache cache;  // first member: its buffers' owners below go before it
   femgpu_config cfg{};
   int device = 0;
   cudaStream_t stream = 0;
