@@ -22,6 +22,7 @@
 #include <cstdlib>
 #include <cmath>
 #include <limits>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -455,6 +456,13 @@ constexpr int64_t kClusterAggEdges = 600000;
 
 enum AggStatus { AGG_OK = 0, AGG_MIS_CAP, AGG_LOOP_CAP, AGG_RESTRICT_CAP, AGG_STALLED };
 
+// The order of the next level (what old_mis forms from the partitions), for the weighted
+// graph's kernel to write: the graph's nodes are aggregates, with their member nodes.
+struct OrderArgs {
+  const int32_t *astart, *members;  // members of aggregate a: members[astart[a] .. astart[a + 1])
+  int32_t *part_idx, *old_of, *new_id, *agg_idx, *xadj_out, *adj_out, *iperm, *perm, *agg_of, *part_of_row;
+};
+
 struct AggArgs {
   int n;
   const int32_t *xadj, *adj, *w;  // w: node weights (weighted graph), else null
@@ -464,6 +472,7 @@ struct AggArgs {
   unsigned long long *k0, *k1;  // n each; k0 also holds the partitions' best moves
   int32_t *mis, *part, *pout, *sizes, *map, *to;  // n each
   int32_t* res;  // status, parts after the removals, largest label + 1, 1 when the labels are in pout
+  OrderArgs o;   // weighted graph: part_idx and the rest, else null pointers
 };
 
 // Exchanges one value per CTA; v[r] = CTA r's value on return.  Two buffers: a value is
@@ -516,7 +525,8 @@ __device__ __forceinline__ int agg_block_max(int v, int* sh) {
   __syncthreads();
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  return __reduce_max_sync(0xffffffffu, sh[threadIdx.x & 31]);
+  const int l = threadIdx.x & 31;
+  return __reduce_max_sync(0xffffffffu, l < (int)(blockDim.x >> 5) ? sh[l] : INT32_MIN);
 }
 // Inclusive prefix of a flag over the block, in thread order; *total gets the block's count.
 __device__ __forceinline__ int agg_block_rank(bool flag, int* sh, int* total) {
@@ -529,6 +539,24 @@ __device__ __forceinline__ int agg_block_rank(bool flag, int* sh, int* total) {
   *total = (int)__reduce_add_sync(0xffffffffu, mine);
   const int below = (int)__reduce_add_sync(0xffffffffu, lane < warp ? mine : 0);
   return below + __popc(m & (0xffffffffu >> (31 - lane)));
+}
+
+// Exclusive prefix of one value per thread over the block; *total gets the block's sum.
+__device__ __forceinline__ int agg_block_scan(int v, int* sh, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  __syncthreads();
+  if (lane == 31) sh[warp] = x;
+  __syncthreads();
+  const int mine = sh[lane];
+  *total = (int)__reduce_add_sync(0xffffffffu, mine);
+  const int below = (int)__reduce_add_sync(0xffffffffu, lane < warp ? mine : 0);
+  return below + x - v;
 }
 
 // Arrays that other CTAs write are read from L2 (__ldcg): a line of this SM's L1 may be old.
@@ -731,6 +759,90 @@ __global__ void __launch_bounds__(kAggThreads) aggregate_cluster_kernel(AggArgs 
   int m = -1;
   for (int i = lo + tid; i < hi; i += kAggThreads) m = max(m, __ldcg(pin + i));
   m = x.max(cl, agg_block_max(m, sh));
+  if (a.o.part_idx && status == AGG_OK) {
+    // ---- aggregates ordered by (partition, id), their graph and their nodes renumbered
+    const OrderArgs& o = a.o;
+    const int npart = m + 1;
+    const int pper = (npart + x.C - 1) / x.C, plo = min(npart, x.me * pper), phi = min(npart, plo + pper);
+    const int warp = x.me * (kAggThreads / 32) + (tid >> 5), nwarps = x.C * (kAggThreads / 32), lane = tid & 31;
+    for (int p = plo + tid; p < phi; p += kAggThreads) a.sizes[p] = a.map[p] = 0;
+    cl.sync();
+    for (int i = lo + tid; i < hi; i += kAggThreads) atomicAdd(&a.sizes[__ldcg(pin + i)], 1);
+    cl.sync();
+    {
+      int mine = 0;
+      for (int p = plo + tid; p < phi; p += kAggThreads) mine += __ldcg(a.sizes + p);
+      int base = x.prefix(cl, agg_block_sum(mine, sh)).x;
+      for (int p0 = plo; p0 < phi; p0 += kAggThreads) {
+        const int p = p0 + tid;
+        int total;
+        const int before = agg_block_scan(p < phi ? __ldcg(a.sizes + p) : 0, sh, &total);
+        if (p < phi) o.part_idx[p] = base + before;
+        base += total;
+      }
+      if (x.me == 0 && tid == 0) o.part_idx[npart] = n;
+    }
+    cl.sync();
+    for (int i = lo + tid; i < hi; i += kAggThreads) {
+      const int p = __ldcg(pin + i);
+      a.to[__ldcg(o.part_idx + p) + atomicAdd(&a.map[p], 1)] = i;
+    }
+    cl.sync();
+    // a partition's aggregates in ascending order: each is placed by counting the smaller ones
+    for (int p = warp; p < npart; p += nwarps) {
+      const int b = __ldcg(o.part_idx + p), e = __ldcg(o.part_idx + p + 1);
+      for (int q = b + lane; q < e; q += 32) {
+        const int v = __ldcg(a.to + q);
+        int rank = 0;
+#pragma unroll 8
+        for (int t = b; t < e; t++) rank += __ldcg(a.to + t) < v;
+        o.old_of[b + rank] = v;
+        o.new_id[v] = b + rank;
+      }
+    }
+    cl.sync();
+    {
+      int nodes = 0, edges = 0;
+      for (int q = lo + tid; q < hi; q += kAggThreads) {
+        const int v = __ldcg(o.old_of + q);
+        nodes += o.astart[v + 1] - o.astart[v];
+        edges += xadj[v + 1] - xadj[v];
+      }
+      const int2 pn = x.prefix(cl, agg_block_sum(nodes, sh)), pe = x.prefix(cl, agg_block_sum(edges, sh));
+      int bn = pn.x, be = pe.x;
+      for (int q0 = lo; q0 < hi; q0 += kAggThreads) {
+        const int q = q0 + tid;
+        const int v = q < hi ? __ldcg(o.old_of + q) : 0;
+        int tn, te;
+        const int sn = agg_block_scan(q < hi ? o.astart[v + 1] - o.astart[v] : 0, sh, &tn);
+        const int se = agg_block_scan(q < hi ? xadj[v + 1] - xadj[v] : 0, sh, &te);
+        if (q < hi) {
+          o.agg_idx[q] = bn + sn;
+          o.xadj_out[q] = be + se;
+        }
+        bn += tn;
+        be += te;
+      }
+      if (x.me == 0 && tid == 0) {
+        o.agg_idx[n] = pn.y;
+        o.xadj_out[n] = pe.y;
+      }
+    }
+    cl.sync();
+    for (int q = warp; q < n; q += nwarps) {
+      const int v = __ldcg(o.old_of + q), p = __ldcg(pin + v);
+      const int e0 = xadj[v], e1 = xadj[v + 1], eo = __ldcg(o.xadj_out + q);
+      for (int e = e0 + lane; e < e1; e += 32) o.adj_out[eo + (e - e0)] = __ldcg(o.new_id + adj[e]);
+      const int t0 = o.astart[v], t1 = o.astart[v + 1], no = __ldcg(o.agg_idx + q);
+      for (int t = t0 + lane; t < t1; t += 32) {
+        const int node = o.members[t], at = no + (t - t0);
+        o.iperm[at] = node;
+        o.perm[node] = at;
+        o.agg_of[at] = q;
+        o.part_of_row[at] = p;
+      }
+    }
+  }
   if (x.me == 0 && tid == 0) {
     a.res[0] = status;
     a.res[1] = count;
@@ -743,7 +855,8 @@ __global__ void __launch_bounds__(kAggThreads) aggregate_cluster_kernel(AggArgs 
 // Runs aggregate_cluster_kernel: the labels in `part`, (parts after the removals, largest
 // label + 1) in count and labels.
 void aggregate_small(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int depth, int min_size, int max_size,
-                     int full_size, const int32_t* weights, DBuf<int32_t>& part, int* count, int* labels) {
+                     int full_size, const int32_t* weights, DBuf<int32_t>& part, int* count, int* labels,
+                     const OrderArgs* order) {
   cudaStream_t s = c.stream;
   PhaseTimer pt(s, -4);
   DBuf<unsigned long long> keys((size_t)2 * n, s);
@@ -770,6 +883,7 @@ void aggregate_small(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int
   a.sizes = a.mis + n;
   a.map = a.sizes + n;
   a.to = a.map + n;
+  if (order) a.o = *order;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(kAggThreads);
   cfg.stream = s;
@@ -802,13 +916,17 @@ void aggregate_small(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int
 // aggregateGraph / aggregateWeightedGraph (misHelpers.cu:513-677).  Returns the number
 // of parts (the largest label + 1: the partition restriction of the weighted graph may
 // empty a part).
+// order (weighted graph only, or null): written too when the graph is aggregated by one
+// kernel; *ordered tells.
 int aggregate(Ctx& c, int n, int64_t edges, const int32_t* xadj, const int32_t* adj, int depth, bool weighted,
-              int min_size, int max_size, int full_size, const int32_t* weights, DBuf<int32_t>& part) {
+              int min_size, int max_size, int full_size, const int32_t* weights, DBuf<int32_t>& part,
+              const OrderArgs* order = nullptr, bool* ordered = nullptr) {
   cudaStream_t s = c.stream;
   if (edges <= kClusterAggEdges && n <= kClusterAggEdges / 4 && depth > 0) {
     int count = 0, labels = 0;
     aggregate_small(c, n, xadj, adj, depth, min_size, max_size, full_size, weighted ? weights : nullptr, part, &count,
-                    &labels);
+                    &labels, order);
+    if (ordered) *ordered = order != nullptr;
     return weighted ? labels : count;
   }
   PhaseTimer pt(s, -4);
@@ -1111,43 +1229,47 @@ void old_mis(Ctx& c, int n, int64_t edges, const int32_t* xadj, const int32_t* a
               iadj.p);
   }
   pt.mark("induced");
-  // partitions of aggregates (aggregateWeightedGraph, weights = aggregate sizes)
-  DBuf<int32_t> coarse;
-  const int npart =
-      aggregate(c, nagg, induced_nnz, ixadj.p, iadj.p, coarse_depth, true, 0, c.cfg.partitionMaxSize, n, acount.p, coarse);
-  pt.mark("partitions");
-  // new aggregate ids: order (partition, old id)
-  DBuf<int32_t> pcount(npart + 1, s), pcur(npart, s), old_of(nagg, s), new_id(nagg, s);
-  pcount.zero();
-  FG_LAUNCH(histogram_kernel, grid_for(nagg, 256), 256, 0, s, nagg, coarse.p, nullptr, pcount.p);
-  o.part_idx.alloc(npart + 1, s);
-  exclusive_scan_async(pcount.p, o.part_idx.p, npart, s);
-  pcur.zero();
-  FG_LAUNCH(scatter_bucket_kernel, grid_for(nagg, 256), 256, 0, s, nagg, coarse.p, o.part_idx.p, pcur.p, old_of.p);
-  segmented_sort_i32(old_of.p, o.part_idx.p, npart, nullptr, s);
-  FG_LAUNCH(invert_kernel, grid_for(nagg, 256), 256, 0, s, nagg, old_of.p, new_id.p);
-  // next-level graph (remapInducedGraph, misHelpers.cu:1258-1280): rows in new order,
-  // entries kept in their order and renamed
-  DBuf<int32_t> rlen(nagg + 1, s);
-  FG_LAUNCH(gather_len_kernel, grid_for(nagg, 256), 256, 0, s, nagg, old_of.p, ixadj.p, rlen.p);
+  // partitions of aggregates (aggregateWeightedGraph, weights = aggregate sizes), then the
+  // order of the next level: aggregates by (partition, old id), their graph with its rows in
+  // that order and its entries renamed in place (remapInducedGraph, misHelpers.cu:1258-1280),
+  // nodes by aggregate, members ascending.  Small graphs do it in the kernel that
+  // partitions them (11 launches fewer).
+  DBuf<int32_t> coarse, old_of(nagg, s), new_id(nagg, s);
+  o.part_idx.alloc(nagg + 1, s);
   o.xadj_out.alloc(nagg + 1, s);
-  exclusive_scan_async(rlen.p, o.xadj_out.p, nagg, s);
   o.nnz_out = induced_nnz;  // the same rows, reordered
   o.adj_out.alloc(o.nnz_out > 0 ? o.nnz_out : 1, s);
-  FG_LAUNCH(remap_graph_kernel, grid_for(nagg, 256), 256, 0, s, nagg, old_of.p, ixadj.p, iadj.p, new_id.p,
-            o.xadj_out.p, o.adj_out.p);
-  // node order: aggregates in new order, members ascending
-  DBuf<int32_t> asz(nagg + 1, s);
-  FG_LAUNCH(gather_len_kernel, grid_for(nagg, 256), 256, 0, s, nagg, old_of.p, astart.p, asz.p);
   o.agg_idx.alloc(nagg + 1, s);
-  exclusive_scan_async(asz.p, o.agg_idx.p, nagg, s);
   o.iperm.alloc(n, s);
   o.perm.alloc(n, s);
   o.agg_of.alloc(n, s);
   o.part_of_row.alloc(n, s);
-  FG_LAUNCH(node_order_kernel, grid_for(nagg, 256), 256, 0, s, nagg, old_of.p, astart.p, members.p, o.agg_idx.p,
-            coarse.p, o.iperm.p, o.agg_of.p, o.part_of_row.p);
-  FG_LAUNCH(invert_kernel, grid_for(n, 256), 256, 0, s, n, o.iperm.p, o.perm.p);
+  OrderArgs order{astart.p, members.p, o.part_idx.p, old_of.p, new_id.p, o.agg_idx.p, o.xadj_out.p,
+                  o.adj_out.p, o.iperm.p, o.perm.p, o.agg_of.p, o.part_of_row.p};
+  bool ordered = false;
+  const int npart = aggregate(c, nagg, induced_nnz, ixadj.p, iadj.p, coarse_depth, true, 0, c.cfg.partitionMaxSize, n,
+                              acount.p, coarse, &order, &ordered);
+  o.part_idx.n = (size_t)npart + 1;  // (allocated for a partition per aggregate)
+  pt.mark("partitions");
+  if (!ordered) {
+    DBuf<int32_t> pcount(npart + 1, s), pcur(npart, s), rlen(nagg + 1, s), asz(nagg + 1, s);
+    pcount.zero();
+    FG_LAUNCH(histogram_kernel, grid_for(nagg, 256), 256, 0, s, nagg, coarse.p, nullptr, pcount.p);
+    exclusive_scan_async(pcount.p, o.part_idx.p, npart, s);
+    pcur.zero();
+    FG_LAUNCH(scatter_bucket_kernel, grid_for(nagg, 256), 256, 0, s, nagg, coarse.p, o.part_idx.p, pcur.p, old_of.p);
+    segmented_sort_i32(old_of.p, o.part_idx.p, npart, nullptr, s);
+    FG_LAUNCH(invert_kernel, grid_for(nagg, 256), 256, 0, s, nagg, old_of.p, new_id.p);
+    FG_LAUNCH(gather_len_kernel, grid_for(nagg, 256), 256, 0, s, nagg, old_of.p, ixadj.p, rlen.p);
+    exclusive_scan_async(rlen.p, o.xadj_out.p, nagg, s);
+    FG_LAUNCH(remap_graph_kernel, grid_for(nagg, 256), 256, 0, s, nagg, old_of.p, ixadj.p, iadj.p, new_id.p,
+              o.xadj_out.p, o.adj_out.p);
+    FG_LAUNCH(gather_len_kernel, grid_for(nagg, 256), 256, 0, s, nagg, old_of.p, astart.p, asz.p);
+    exclusive_scan_async(asz.p, o.agg_idx.p, nagg, s);
+    FG_LAUNCH(node_order_kernel, grid_for(nagg, 256), 256, 0, s, nagg, old_of.p, astart.p, members.p, o.agg_idx.p,
+              coarse.p, o.iperm.p, o.agg_of.p, o.part_of_row.p);
+    FG_LAUNCH(invert_kernel, grid_for(n, 256), 256, 0, s, n, o.iperm.p, o.perm.p);
+  }
   pt.mark("order");
   o.nagg = nagg;
   o.npart = npart;
@@ -1190,6 +1312,7 @@ struct EscArgs {
   int32_t* overflow;
   int thread_cap;        // rows with at most this many items use the thread tier
   int64_t known_nnz;     // PERMUTE: the input's entry count (every entry is kept), else 0
+  int max_items;         // bound on a row's items when known, else 0
 };
 
 constexpr int kEscWarpCap = 1024;
@@ -1337,8 +1460,16 @@ __global__ void collect_big_rows_kernel(int n, const int32_t* items, int cap, in
   if (i < n && items[i] > cap && items[i] <= hard_cap) list[atomicAdd(nlist, 1)] = i;
 }
 
+// Rows of more than thread_cap and at most kEscWarpCap items, one warp each.  A warp looks at
+// `look` rows' item counts at a time: 32 on large levels (one row at a time, 2.1 M rows with
+// none to sort took 0.4 ms per pass), few on small ones, whose rows need all the warps.  Items of a permuted row have distinct columns: up to
+// kRankCap of them are placed by counting the smaller ones (a broadcast read and a compare per
+// item and lane, no barriers) instead of a bitonic network: 80,338 rows of 100 items 406 ->
+// 191 us.
+constexpr int kRankCap = 256;
+
 template <class T, int MODE, bool WRITE>
-__global__ void esc_warp_kernel(EscArgs<T> a, const int32_t* items) {
+__global__ void esc_warp_kernel(EscArgs<T> a, const int32_t* __restrict__ items, int look) {
   extern __shared__ unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem_raw) + (size_t)w * kEscWarpCap;
@@ -1346,19 +1477,63 @@ __global__ void esc_warp_kernel(EscArgs<T> a, const int32_t* items) {
             (size_t)w * kEscWarpCap;
   __shared__ int s_scan[kEscWarps][32];
   __shared__ int s_cnt[kEscWarps];
-  for (int i = blockIdx.x * kEscWarps + w; i < a.n; i += gridDim.x * kEscWarps) {
-    int len = items[i];
-    if (len > kEscWarpCap || len <= a.thread_cap) continue;
-    esc_generate<T, MODE>(a, i, keys, vals, lane, 32, s_scan[w], WarpSync());
-    int np2 = next_pow2(len < 2 ? 2 : len);
-    for (int p = len + lane; p < np2; p += 32) keys[p] = ~0ull;
-    __syncwarp();
-    bitonic_sort_shared(keys, np2, lane, 32, WarpSync());
-    int out = WRITE ? a.orp[i] : 0;
-    int cnt = esc_reduce<T>(keys, vals, len, lane, 32, &s_cnt[w], WRITE ? a.oci + out : nullptr,
-                            WRITE ? a.ov + out : nullptr, WRITE, WarpSync());
-    if (!WRITE && lane == 0) a.counts[i] = cnt;
-    __syncwarp();
+  for (int i0 = (blockIdx.x * kEscWarps + w) * look; i0 < a.n; i0 += gridDim.x * kEscWarps * look) {
+    const int mylen = lane < look && i0 + lane < a.n ? items[i0 + lane] : 0;
+    unsigned todo = __ballot_sync(0xffffffffu, mylen > a.thread_cap && mylen <= kEscWarpCap);
+    while (todo) {
+      const int src = __ffs(todo) - 1, i = i0 + src;
+      todo &= todo - 1;
+      const int len = __shfl_sync(0xffffffffu, mylen, src);
+      if (MODE == ESC_PERMUTE && WRITE && len <= kRankCap) {
+        const int r = esc_input_row<T, MODE>(a, i), rb = a.arp[r], out = a.orp[i];
+        int32_t* col = reinterpret_cast<int32_t*>(keys);
+        int32_t c[kRankCap / 32];
+        int rank[kRankCap / 32];
+#pragma unroll
+        for (int q = 0; q < kRankCap / 32; q++) {
+          const int g = lane + 32 * q;
+          c[q] = INT32_MAX;
+          rank[q] = 0;
+          if (g < len) {
+            const int j = a.aci[rb + g];
+            c[q] = a.perm ? a.perm[j] : j;
+          }
+          col[g] = c[q];  // past the end INT32_MAX: never smaller
+        }
+        __syncwarp();
+        auto count = [&](auto nq) {  // nq registers of 32 items cover the row
+          for (int t = 0; t < len; t += 4) {
+            const int4 o = *reinterpret_cast<const int4*>(col + t);
+#pragma unroll
+            for (int q = 0; q < decltype(nq)::value; q++)
+              rank[q] += (o.x < c[q]) + (o.y < c[q]) + (o.z < c[q]) + (o.w < c[q]);
+          }
+        };
+        if (len <= 64) count(std::integral_constant<int, 2>());
+        else if (len <= 128) count(std::integral_constant<int, 4>());
+        else count(std::integral_constant<int, 8>());
+#pragma unroll
+        for (int q = 0; q < kRankCap / 32; q++) {
+          const int g = lane + 32 * q;
+          if (g < len) {
+            a.oci[out + rank[q]] = c[q];
+            a.ov[out + rank[q]] = a.av[rb + g];
+          }
+        }
+        __syncwarp();
+        continue;
+      }
+      esc_generate<T, MODE>(a, i, keys, vals, lane, 32, s_scan[w], WarpSync());
+      int np2 = next_pow2(len < 2 ? 2 : len);
+      for (int p = len + lane; p < np2; p += 32) keys[p] = ~0ull;
+      __syncwarp();
+      bitonic_sort_shared(keys, np2, lane, 32, WarpSync());
+      int out = WRITE ? a.orp[i] : 0;
+      int cnt = esc_reduce<T>(keys, vals, len, lane, 32, &s_cnt[w], WRITE ? a.oci + out : nullptr,
+                              WRITE ? a.ov + out : nullptr, WRITE, WarpSync());
+      if (!WRITE && lane == 0) a.counts[i] = cnt;
+      __syncwarp();
+    }
   }
 }
 
@@ -1573,21 +1748,31 @@ template <class T, int MODE>
 void run_esc_sort(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>& out) {
   cudaStream_t s = c.stream;
   a.n = nrows_out;
-  DBuf<int32_t> items(nrows_out + 1, s), ucnt(nrows_out + 1, s), big(nrows_out + 1, s), nbig(1, s);
-  DBuf<int32_t> dense(nrows_out + 1, s), ndense(1, s);
-  nbig.zero();
-  ndense.zero();
+  DBuf<int32_t> items(nrows_out + 1, s), ucnt, big, nbig, dense, ndense;
+  if (MODE != ESC_PERMUTE) ucnt.alloc(nrows_out + 1, s);
   a.counts = items.p;
   FG_LAUNCH((esc_count_items_kernel<T, MODE>), grid_for(nrows_out, 256), 256, 0, s, a);
-  FG_LAUNCH(collect_big_rows_kernel, grid_for(nrows_out, 256), 256, 0, s, nrows_out, items.p, kEscWarpCap,
-            kEscBlockCap, big.p, nbig.p);
-  FG_LAUNCH(collect_dense_rows_kernel, grid_for(nrows_out, 256), 256, 0, s, nrows_out, items.p, kEscBlockCap,
-            dense.p, ndense.p);
-  int32_t h_big = 0, h_dense = 0;  // both counts in one round trip
-  FG_CUDA(cudaMemcpyAsync(&h_big, nbig.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  FG_CUDA(cudaMemcpyAsync(&h_dense, ndense.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  FG_CUDA(cudaStreamSynchronize(s));
-  g_host_syncs.fetch_add(1, std::memory_order_relaxed);
+  // tiers above the thread's (warp, block, dense accumulator) run only where the longest
+  // row's items, when the caller knows a bound, can reach them
+  const bool warp_tier = a.max_items == 0 || a.max_items > kThreadRowCap;
+  int32_t h_big = 0, h_dense = 0;
+  if (a.max_items == 0 || a.max_items > kEscWarpCap) {
+    big.alloc(nrows_out + 1, s);
+    dense.alloc(nrows_out + 1, s);
+    nbig.alloc(1, s);
+    ndense.alloc(1, s);
+    nbig.zero();
+    ndense.zero();
+    FG_LAUNCH(collect_big_rows_kernel, grid_for(nrows_out, 256), 256, 0, s, nrows_out, items.p, kEscWarpCap,
+              kEscBlockCap, big.p, nbig.p);
+    FG_LAUNCH(collect_dense_rows_kernel, grid_for(nrows_out, 256), 256, 0, s, nrows_out, items.p, kEscBlockCap,
+              dense.p, ndense.p);
+    // both counts in one round trip
+    FG_CUDA(cudaMemcpyAsync(&h_big, nbig.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    FG_CUDA(cudaMemcpyAsync(&h_dense, ndense.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    FG_CUDA(cudaStreamSynchronize(s));
+    g_host_syncs.fetch_add(1, std::memory_order_relaxed);
+  }
   a.nbig = h_big;
   a.big_rows = big.p;
   EscArgs<T> ad = a;  // dense tier: rows with more items than the sort capacity
@@ -1618,14 +1803,15 @@ void run_esc_sort(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>& o
     ensure_smem(esc_block_kernel<T, MODE, true>, bsm);
     attr_set = true;
   }
-  const int wgrid = std::min<int64_t>((nrows_out + kEscWarps - 1) / kEscWarps, 152 * 64);
+  const int look = std::max(1, std::min(32, nrows_out / (152 * 64)));
+  const int wgrid = (int)std::min<int64_t>(((int64_t)nrows_out + look * kEscWarps - 1) / (look * kEscWarps), 152 * 64);
   a.counts = ucnt.p;
   a.thread_cap = kThreadRowCap;
   // a permuted row has no repeated column: its output length is its item count, so the
   // counting pass is needed only for the prolongator
   if (MODE != ESC_PERMUTE) {
     FG_LAUNCH((esc_thread_kernel<T, MODE, false>), grid_for(nrows_out, 128), 128, 0, s, a, items.p);
-    FG_LAUNCH((esc_warp_kernel<T, MODE, false>), wgrid, 32 * kEscWarps, wsm, s, a, items.p);
+    if (warp_tier) FG_LAUNCH((esc_warp_kernel<T, MODE, false>), wgrid, 32 * kEscWarps, wsm, s, a, items.p, look);
     if (a.nbig > 0)
       FG_LAUNCH((esc_block_kernel<T, MODE, false>), std::min(a.nbig, 152 * 2), kEscBlockThreads, bsm, s, a,
                 items.p);
@@ -1650,7 +1836,7 @@ void run_esc_sort(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>& o
   a.oci = out.ci.p;
   a.ov = out.v.p;
   FG_LAUNCH((esc_thread_kernel<T, MODE, true>), grid_for(nrows_out, 128), 128, 0, s, a, items.p);
-  FG_LAUNCH((esc_warp_kernel<T, MODE, true>), wgrid, 32 * kEscWarps, wsm, s, a, items.p);
+  if (warp_tier) FG_LAUNCH((esc_warp_kernel<T, MODE, true>), wgrid, 32 * kEscWarps, wsm, s, a, items.p, look);
   if (a.nbig > 0)
     FG_LAUNCH((esc_block_kernel<T, MODE, true>), std::min(a.nbig, 152 * 2), kEscBlockThreads, bsm, s, a, items.p);
   if (ad.nbig > 0) {
@@ -2081,7 +2267,7 @@ __global__ void spgemm_dense_warp_kernel(EscArgs<T> a, int ncols, const int32_t*
     for (int t = nt + lane; t < np2; t += 32) list[t] = INT32_MAX;
     __syncwarp();
     bitonic_sort_shared(list, np2, lane, 32, WarpSync());
-    const int o = toff[i];
+    const int o = toff ? toff[i] : i * ncols;  // without offsets a row's slots are a whole row
     for (int t = lane; t < nt; t += 32) {
       const int col = list[t];
       tci[o + t] = col;
@@ -2101,11 +2287,11 @@ __global__ void spgemm_capacity_kernel(int n, const int32_t* items, int ncols, i
 // Rows from their capacity-spaced temporary slots to the compact CSR: G lanes per row
 // (G near the average row length, so short rows do not leave most of a warp idle).
 template <class T, int G>
-__global__ void compact_rows_copy_kernel(int n, const int32_t* toff, const int32_t* tci, const T* tv,
+__global__ void compact_rows_copy_kernel(int n, const int32_t* toff, int stride, const int32_t* tci, const T* tv,
                                          const int32_t* orp, int32_t* oci, T* ov) {
   const int lane = threadIdx.x & (G - 1);
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) / G; i < n; i += (gridDim.x * blockDim.x) / G) {
-    const int o = orp[i], len = orp[i + 1] - o, src = toff[i];
+    const int o = orp[i], len = orp[i + 1] - o, src = toff ? toff[i] : i * stride;
     for (int t = lane; t < len; t += G) {
       oci[o + t] = tci[src + t];
       ov[o + t] = tv[src + t];
@@ -2114,10 +2300,76 @@ __global__ void compact_rows_copy_kernel(int n, const int32_t* toff, const int32
 }
 
 template <class T>
-void run_spgemm_hash(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>& out) {
+void compact_rows(cudaStream_t s, int n, double avg, const int32_t* toff, int stride, const int32_t* tci, const T* tv,
+                  DCsr<T>& out) {
+  const int G = avg <= 6.0 ? 4 : avg <= 12.0 ? 8 : avg <= 24.0 ? 16 : 32;
+  const int cgrid = grid_for((int64_t)n * G, 256);
+#define FG_COMPACT(GG)                                                                                            \
+  FG_LAUNCH((compact_rows_copy_kernel<T, GG>), cgrid, 256, 0, s, n, toff, stride, tci, tv, out.rp.p, out.ci.p, \
+            out.v.p)
+  switch (G) {
+    case 4: FG_COMPACT(4); break;
+    case 8: FG_COMPACT(8); break;
+    case 16: FG_COMPACT(16); break;
+    default: FG_COMPACT(32); break;
+  }
+#undef FG_COMPACT
+}
+
+// Narrow products whose rows fit this many temporary entries as whole rows (n x ncols) take
+// their slots there at once: no count of the products, no scan of the counts and no look at
+// their total (two launches and a host read of 10-15 us before a kernel of 10-20 us).
+constexpr int64_t kDirectSlots = 1 << 21;
+
+// C = A B.  max_row (or null) receives the longest row of C, read back with its size.  With
+// on_device a product that takes direct slots is not read back at all: its arrays have room
+// for every slot and C.nnz is that bound (for a product that only the next product reads).
+template <class T>
+void run_spgemm_hash(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>& out, int* max_row, bool on_device) {
   cudaStream_t s = c.stream;
   PhaseTimer pt(s, -2);
   a.n = nrows_out;
+  const size_t dper = dense_warp_smem<T>(ncols_out);
+  const bool narrow = nrows_out < 65536 && ncols_out <= kDenseCols;
+  DBuf<int32_t> mx(1, s);
+  out.n = nrows_out;
+  out.m = ncols_out;
+  auto dense_rows = [&](const int32_t* toff, int32_t* tci, T* tv, int32_t* cnt) {
+    const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)(200 * 1024) / dper));
+    const size_t dsm = (size_t)wpb * dper;
+    if (dsm > 48 * 1024) ensure_smem(spgemm_dense_warp_kernel<T>, dsm);
+    FG_LAUNCH(spgemm_dense_warp_kernel<T>, (int)std::min<int64_t>((nrows_out + wpb - 1) / wpb, 152 * 4), 32 * wpb,
+              dsm, s, a, ncols_out, toff, tci, tv, cnt);
+  };
+  if (narrow && (int64_t)nrows_out * ncols_out <= kDirectSlots) {
+    const int64_t slots = (int64_t)nrows_out * ncols_out;
+    DBuf<int32_t> cnt(nrows_out + 1, s), tci(slots, s);
+    DBuf<T> tv(slots, s);
+    dense_rows(nullptr, tci.p, tv.p, cnt.p);
+    pt.mark("sp rows");
+    out.rp.alloc(nrows_out + 1, s);
+    exclusive_scan_async(cnt.p, out.rp.p, nrows_out, s);
+    out.nnz = slots;
+    double avg = 16.0;
+    if (!on_device) {
+      int32_t h_tot = 0, h_max = 0;
+      if (max_row) {
+        reduce_max_async(cnt.p, nrows_out, mx.p, s);
+        FG_CUDA(cudaMemcpyAsync(&h_max, mx.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+      }
+      FG_CUDA(cudaMemcpyAsync(&h_tot, out.rp.p + nrows_out, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+      FG_CUDA(cudaStreamSynchronize(s));
+      g_host_syncs.fetch_add(1, std::memory_order_relaxed);
+      out.nnz = h_tot;
+      if (max_row) *max_row = h_max;
+      avg = nrows_out > 0 ? (double)out.nnz / nrows_out : 0.0;
+    }
+    out.ci.alloc(out.nnz > 0 ? out.nnz : 1, s);
+    out.v.alloc(out.nnz > 0 ? out.nnz : 1, s);
+    compact_rows<T>(s, nrows_out, avg, nullptr, ncols_out, tci.p, tv.p, out);
+    pt.mark("sp out");
+    return;
+  }
   DBuf<int32_t> items(nrows_out + 1, s), capv(nrows_out + 1, s), toff(nrows_out + 1, s), cnt(nrows_out + 1, s);
   a.counts = items.p;
   FG_LAUNCH((esc_count_items_kernel<T, ESC_SPGEMM>), grid_for(nrows_out, 256), 256, 0, s, a);
@@ -2131,14 +2383,8 @@ void run_spgemm_hash(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>
   nover1.zero();
   nover2.zero();
   const int wgrid = std::min<int64_t>((nrows_out + kHashWarps - 1) / kHashWarps, 152 * 32);
-  const size_t dper = dense_warp_smem<T>(ncols_out);
-  if (nrows_out < 65536 && ncols_out <= kDenseCols) {
-    // a narrow product: every row on the dense accumulator tier (no overflow rows)
-    const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)(200 * 1024) / dper));
-    const size_t dsm = (size_t)wpb * dper;
-    if (dsm > 48 * 1024) ensure_smem(spgemm_dense_warp_kernel<T>, dsm);
-    FG_LAUNCH(spgemm_dense_warp_kernel<T>, (int)std::min<int64_t>((nrows_out + wpb - 1) / wpb, 152 * 4), 32 * wpb,
-              dsm, s, a, ncols_out, toff.p, tci.p, tv.p, cnt.p);
+  if (narrow) {
+    dense_rows(toff.p, tci.p, tv.p, cnt.p);  // every row on the dense accumulator tier (no overflow rows)
   } else if (nrows_out >= 65536 && tcap <= (int64_t)nrows_out * 128) {
     // short rows on average: thread-per-row tier first, its overflow rows to the warp tier
     DBuf<int32_t> over0(nrows_out + 1, s), nover0(1, s);
@@ -2154,11 +2400,13 @@ void run_spgemm_hash(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>
   pt.mark("sp rows");
   // the output offsets are scanned before the overflow count is read, so when no row
   // overflowed (the usual case) both come back in one round trip
-  out.n = nrows_out;
-  out.m = ncols_out;
   out.rp.alloc(nrows_out + 1, s);
   exclusive_scan_async(cnt.p, out.rp.p, nrows_out, s);
-  int32_t h_n1 = 0, h_tot = 0;
+  int32_t h_n1 = 0, h_tot = 0, h_max = 0;
+  if (max_row) {
+    reduce_max_async(cnt.p, nrows_out, mx.p, s);
+    FG_CUDA(cudaMemcpyAsync(&h_max, mx.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  }
   FG_CUDA(cudaMemcpyAsync(&h_n1, nover1.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   FG_CUDA(cudaMemcpyAsync(&h_tot, out.rp.p + nrows_out, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   FG_CUDA(cudaStreamSynchronize(s));
@@ -2192,64 +2440,50 @@ void run_spgemm_hash(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>
                 nullptr);
     }
     out.nnz = exclusive_scan(cnt.p, out.rp.p, nrows_out, s);  // the overflow rows' counts are in now
+    if (max_row) h_max = reduce_max(cnt.p, nrows_out, s);
   }
   pt.mark("sp big");
   out.ci.alloc(out.nnz > 0 ? out.nnz : 1, s);
   out.v.alloc(out.nnz > 0 ? out.nnz : 1, s);
-  {
-    const double avg = nrows_out > 0 ? (double)out.nnz / nrows_out : 0.0;
-    const int G = avg <= 6.0 ? 4 : avg <= 12.0 ? 8 : avg <= 24.0 ? 16 : 32;
-    const int cgrid = grid_for((int64_t)nrows_out * G, 256);
-#define FG_COMPACT(GG)                                                                                    \
-  FG_LAUNCH((compact_rows_copy_kernel<T, GG>), cgrid, 256, 0, s, nrows_out, toff.p, tci.p, tv.p, out.rp.p, \
-            out.ci.p, out.v.p)
-    switch (G) {
-      case 4: FG_COMPACT(4); break;
-      case 8: FG_COMPACT(8); break;
-      case 16: FG_COMPACT(16); break;
-      default: FG_COMPACT(32); break;
-    }
-#undef FG_COMPACT
-  }
+  if (max_row) *max_row = h_max;
+  compact_rows<T>(s, nrows_out, nrows_out > 0 ? (double)out.nnz / nrows_out : 0.0, toff.p, 0, tci.p, tv.p, out);
   pt.mark("sp out");
 }
 
-template <class T, int MODE>
-void run_esc(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>& out) {
-  if (MODE == ESC_SPGEMM) run_spgemm_hash<T>(c, a, nrows_out, ncols_out, out);
-  else run_esc_sort<T, MODE>(c, a, nrows_out, ncols_out, out);
-}
-
 // ---- level matrices -----------------------------------------------------------------
+// Diagonal of the sorted rows and its reciprocal.
 template <class T>
-__global__ void diag_kernel(int n, const int32_t* rp, const int32_t* ci, const T* v, T* d) {
+__global__ void diag_kernel(int n, const int32_t* rp, const int32_t* ci, const T* v, T* d, T* dinv) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     int s = lower_bound_i32(ci, rp[i], rp[i + 1], i);
-    d[i] = (s < rp[i + 1] && ci[s] == i) ? v[s] : (T)0;
+    const T x = (s < rp[i + 1] && ci[s] == i) ? v[s] : (T)0;
+    d[i] = x;
+    dinv[i] = (T)1 / x;
   }
 }
 
-template <class T>
-__global__ void reciprocal_kernel(int n, const T* d, T* dinv) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dinv[i] = (T)1 / d[i];
-}
-
+// In- and out-of-partition entries of every row, and the longest in-partition row in *longest
+// (zero before).
 template <class T>
 __global__ void split_count_kernel(int n, const int32_t* rp, const int32_t* ci, const int32_t* part, int32_t* cin,
-                                   int32_t* cout) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int pi = part[i], a = 0, b = 0;
-  for (int e = rp[i]; e < rp[i + 1]; e++) {
-    int j = ci[e];
-    if (j == i) continue;
-    if (part[j] == pi) a++;
-    else b++;
+                                   int32_t* cout, int32_t* longest) {
+  __shared__ int sh[32];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int a = 0, b = 0;
+  if (i < n) {
+    const int pi = part[i];
+    for (int e = rp[i]; e < rp[i + 1]; e++) {
+      const int j = ci[e];
+      if (j == i) continue;
+      if (part[j] == pi) a++;
+      else b++;
+    }
+    cin[i] = a;
+    cout[i] = b;
   }
-  cin[i] = a;
-  cout[i] = b;
+  const int m = agg_block_max(a, sh);
+  if (threadIdx.x == 0 && m > 0) atomicMax(longest, m);
 }
 
 template <class T>
@@ -2740,26 +2974,28 @@ __global__ void dense_inverse_kernel(int n, const double* __restrict__ F, const 
   for (int i = threadIdx.x; i < n; i += blockDim.x) inv[(int64_t)i * n + j] = sb[i];
 }
 
-__global__ void partition_rows_kernel(int npart, const int32_t* part_idx, const int32_t* agg_idx, int32_t* rows) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < npart) rows[p] = agg_idx[part_idx[p + 1]] - agg_idx[part_idx[p]];
-}
-
-// In-partition entries per partition (the shared-memory footprint of the smoother).
-__global__ void partition_entries_kernel(int npart, const int32_t* part_idx, const int32_t* agg_idx,
-                                         const int32_t* irp, int32_t* ent) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < npart) ent[p] = irp[agg_idx[part_idx[p + 1]]] - irp[agg_idx[part_idx[p]]];
-}
-
-// First row and first in-partition entry of partitions 0..npart (npart = the end).
-__global__ void partition_starts_kernel(int npart, const int32_t* part_idx, const int32_t* agg_idx,
-                                        const int32_t* irp, int32_t* row0, int32_t* ent0) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p <= npart) {
-    const int r = agg_idx[part_idx[p]];
+// First row and first in-partition entry of partitions 0..npart (npart = the end), and the
+// largest partition's rows and in-partition entries (mx[0], mx[1]); one block.
+__global__ void __launch_bounds__(1024) partition_starts_kernel(int npart, const int32_t* part_idx,
+                                                                const int32_t* agg_idx, const int32_t* irp,
+                                                                int32_t* row0, int32_t* ent0, int32_t* mx) {
+  __shared__ int sh[32];
+  int rows = 0, ents = 0;
+  for (int p = threadIdx.x; p <= npart; p += 1024) {
+    const int r = agg_idx[part_idx[p]], e = irp[r];
     row0[p] = r;
-    ent0[p] = irp[r];
+    ent0[p] = e;
+    if (p < npart) {
+      const int r1 = agg_idx[part_idx[p + 1]];
+      rows = max(rows, r1 - r);
+      ents = max(ents, irp[r1] - e);
+    }
+  }
+  rows = agg_block_max(rows, sh);
+  ents = agg_block_max(ents, sh);
+  if (threadIdx.x == 0) {
+    mx[0] = rows;
+    mx[1] = ents;
   }
 }
 
@@ -2835,17 +3071,11 @@ __global__ void __launch_bounds__(512) jds_build_kernel(const int32_t* __restric
 
 // Smoother work groups: consecutive partitions packed greedily into one CTA while
 // the group stays within `max_rows` rows and `max_ents` in-partition entries.
+// hr, he: first row and first in-partition entry of partitions 0..npart.
 template <class T>
-void build_smoother_groups(Ctx& c, Level<T>& L, int max_rows, int max_ents) {
+void build_smoother_groups(Ctx& c, Level<T>& L, int max_rows, int max_ents, const std::vector<int32_t>& hr,
+                           const std::vector<int32_t>& he) {
   cudaStream_t s = c.stream;
-  DBuf<int32_t> row0(L.npart + 1, s), ent0(L.npart + 1, s);
-  FG_LAUNCH(partition_starts_kernel, grid_for(L.npart + 1, 256), 256, 0, s, L.npart, L.part_idx.p, L.agg_idx.p,
-            L.Ain.rp.p, row0.p, ent0.p);
-  std::vector<int32_t> hr(L.npart + 1), he(L.npart + 1);
-  row0.download(hr.data(), L.npart + 1);
-  ent0.download(he.data(), L.npart + 1);
-  FG_CUDA(cudaStreamSynchronize(s));
-  g_host_syncs.fetch_add(1, std::memory_order_relaxed);
   std::vector<int32_t> g{hr[0]};
   int gp = 0, mx = 0, mxe = 0;
   for (int p = 1; p <= L.npart; p++) {
@@ -2908,6 +3138,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
     FG_CUDA(cudaMemcpyAsync(L0->A.ci.p, c.A.ci.p, c.A.nnz * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
     FG_LAUNCH(cast_kernel<T>, grid_for(c.A.nnz, 256), 256, 0, s, c.A.nnz, c.A.v.p, L0->A.v.p);
     L0->gnnz = c.graph_nnz;
+    L0->max_row = c.A_max_row;
     L0->gxadj.alloc(n0 + 1, s);
     L0->gadj.alloc(c.graph_nnz > 0 ? c.graph_nnz : 1, s);
     FG_CUDA(cudaMemcpyAsync(L0->gxadj.p, c.gxadj.p, (n0 + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
@@ -2970,34 +3201,36 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
       a.perm = L.perm.p;
       a.iperm = L.iperm.p;
       a.known_nnz = L.A.nnz;
-      run_esc<T, ESC_PERMUTE>(c, a, N, N, L.Ap);
+      a.max_items = L.max_row;
+      run_esc_sort<T, ESC_PERMUTE>(c, a, N, N, L.Ap);
     }
     pt.mark("permute");
     L.diag.alloc(N, s);
-    FG_LAUNCH(diag_kernel<T>, grid_for(N, 256), 256, 0, s, N, L.Ap.rp.p, L.Ap.ci.p, L.Ap.v.p, L.diag.p);
     L.dinv.alloc(N, s);
-    FG_LAUNCH(reciprocal_kernel<T>, grid_for(N, 256), 256, 0, s, N, L.diag.p, L.dinv.p);
-    // in/out-of-partition split; the two entry counts and the three maxima the smoother
-    // plan needs come back in one round trip
+    FG_LAUNCH(diag_kernel<T>, grid_for(N, 256), 256, 0, s, N, L.Ap.rp.p, L.Ap.ci.p, L.Ap.v.p, L.diag.p, L.dinv.p);
+    // in/out-of-partition split; the two entry counts, the three maxima and the partition
+    // starts the smoother plan needs come back in one round trip
+    std::vector<int32_t> hr, he;
     {
-      DBuf<int32_t> cin(N + 1, s), cout(N + 1, s), prow(L.npart + 1, s), pent(L.npart + 1, s), mx(3, s);
+      DBuf<int32_t> cin(N + 1, s), cout(N + 1, s), row0(L.npart + 1, s), ent0(L.npart + 1, s), mx(3, s);
+      mx.zero();
       FG_LAUNCH(split_count_kernel<T>, grid_for(N, 256), 256, 0, s, N, L.Ap.rp.p, L.Ap.ci.p, o.part_of_row.p, cin.p,
-                cout.p);
+                cout.p, mx.p + 2);
       L.Ain.n = L.Ain.m = L.Aout.n = L.Aout.m = N;
       L.Ain.rp.alloc(N + 1, s);
       L.Aout.rp.alloc(N + 1, s);
-      reduce_max_async(cin.p, N, mx.p + 2, s);  // longest in-partition row
       exclusive_scan_async(cin.p, L.Ain.rp.p, N, s);
       exclusive_scan_async(cout.p, L.Aout.rp.p, N, s);
-      FG_LAUNCH(partition_rows_kernel, grid_for(L.npart, 256), 256, 0, s, L.npart, L.part_idx.p, L.agg_idx.p, prow.p);
-      reduce_max_async(prow.p, L.npart, mx.p, s);
-      FG_LAUNCH(partition_entries_kernel, grid_for(L.npart, 256), 256, 0, s, L.npart, L.part_idx.p, L.agg_idx.p,
-                L.Ain.rp.p, pent.p);
-      reduce_max_async(pent.p, L.npart, mx.p + 1, s);
+      FG_LAUNCH(partition_starts_kernel, 1, 1024, 0, s, L.npart, L.part_idx.p, L.agg_idx.p, L.Ain.rp.p, row0.p,
+                ent0.p, mx.p);
       int32_t h_in = 0, h_out = 0, h_mx[3] = {0, 0, 0};
+      hr.resize(L.npart + 1);
+      he.resize(L.npart + 1);
       FG_CUDA(cudaMemcpyAsync(&h_in, L.Ain.rp.p + N, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
       FG_CUDA(cudaMemcpyAsync(&h_out, L.Aout.rp.p + N, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
       FG_CUDA(cudaMemcpyAsync(h_mx, mx.p, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+      row0.download(hr.data(), L.npart + 1);
+      ent0.download(he.data(), L.npart + 1);
       FG_CUDA(cudaStreamSynchronize(s));
       g_host_syncs.fetch_add(1, std::memory_order_relaxed);
       L.Ain.nnz = h_in;
@@ -3016,7 +3249,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
     {
       pt.mark("split rows");
       if (smoother_in_registers(L.max_in_row, L.max_part_rows)) {
-        build_smoother_groups(c, L, kRegGroupRows, std::numeric_limits<int>::max());
+        build_smoother_groups(c, L, kRegGroupRows, std::numeric_limits<int>::max(), hr, he);
         L.jv.alloc(L.Ain.nnz + 16, s);
         L.jv.zero();
         L.jc16.alloc(L.Ain.nnz + 16, s);
@@ -3026,7 +3259,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
           FG_LAUNCH(jds_build_kernel<T>, L.ngroups, kRegGroupRows, 0, s, L.grows.p, L.Ain.rp.p, L.Ain.ci.p,
                     L.Ain.v.p, L.jv.p, L.jc16.p, L.jrow.p);
       } else
-        build_smoother_groups(c, L, L.max_part_rows, L.max_part_entries);
+        build_smoother_groups(c, L, L.max_part_rows, L.max_part_entries, hr, he);
       pt.mark("groups");
       plan_smoother(c, L);
       pt.mark("plan");
@@ -3051,7 +3284,8 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
       a.agg_of = L.agg_of.p;
       a.diag = L.diag.p;
       a.neg_omega = -(T)c.cfg.proOmega;
-      run_esc<T, ESC_PROLONG>(c, a, N, L.nagg, L.P);
+      a.max_items = L.max_row > 0 ? L.max_row + 1 : 0;
+      run_esc_sort<T, ESC_PROLONG>(c, a, N, L.nagg, L.P);
     }
     {
       pt.mark("P");
@@ -3074,7 +3308,8 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
       a.aci = Ru.ci.p;
       a.av = Ru.v.p;
       a.known_nnz = L.P.nnz;
-      run_esc<T, ESC_PERMUTE>(c, a, L.nagg, N, L.R);
+      a.max_items = N <= kEscWarpCap ? N : 0;  // a row of R has at most N entries
+      run_esc_sort<T, ESC_PERMUTE>(c, a, L.nagg, N, L.R);
     }
     // Galerkin product A_next = R (Ap P)
     auto nx = std::make_unique<Level<T>>();
@@ -3093,7 +3328,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
       a.brp = L.P.rp.p;
       a.bci = L.P.ci.p;
       a.bv = pv.p;
-      run_esc<double, ESC_SPGEMM>(c, a, N, L.nagg, AP);
+      run_spgemm_hash<double>(c, a, N, L.nagg, AP, nullptr, true);
       EscArgs<double> r{};
       r.arp = L.R.rp.p;
       r.aci = L.R.ci.p;
@@ -3101,7 +3336,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
       r.brp = AP.rp.p;
       r.bci = AP.ci.p;
       r.bv = AP.v.p;
-      run_esc<double, ESC_SPGEMM>(c, r, L.nagg, L.nagg, A64);
+      run_spgemm_hash<double>(c, r, L.nagg, L.nagg, A64, &nx->max_row, false);
       nx->A.n = A64.n;
       nx->A.m = A64.m;
       nx->A.nnz = A64.nnz;
@@ -3121,7 +3356,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
       a.bci = L.P.ci.p;
       a.bv = L.P.v.p;
       pt.mark("R");
-      run_esc<T, ESC_SPGEMM>(c, a, N, L.nagg, AP);
+      run_spgemm_hash<T>(c, a, N, L.nagg, AP, nullptr, true);
       pt.mark("AP");
       EscArgs<T> r{};
       r.arp = L.R.rp.p;
@@ -3130,7 +3365,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
       r.brp = AP.rp.p;
       r.bci = AP.ci.p;
       r.bv = AP.v.p;
-      run_esc<T, ESC_SPGEMM>(c, r, L.nagg, L.nagg, nx->A);
+      run_spgemm_hash<T>(c, r, L.nagg, L.nagg, nx->A, &nx->max_row, false);
       pt.mark("RAP");
     }
     nx->n = L.nagg;

@@ -375,8 +375,10 @@ femgpu_status femgpu_set_matrix_csr(femgpu_handle h, int64_t n, const int32_t* r
     FG_REQUIRE(n < INT32_MAX, FEMGPU_ERR_LIMIT, "matrix exceeds int32 indexing");
     int64_t nnz = rowptr[n];
     FG_REQUIRE(nnz >= 0 && (nnz == 0 || (cols && vals)), FEMGPU_ERR_INVALID, "bad CSR arrays");
+    int32_t longest = 0;
     for (int64_t i = 0; i < n; i++) {
       FG_REQUIRE(rowptr[i] <= rowptr[i + 1], FEMGPU_ERR_INVALID, "row offsets not monotone");
+      longest = std::max(longest, rowptr[i + 1] - rowptr[i]);
       for (int64_t e = rowptr[i]; e < rowptr[i + 1]; e++) {
         FG_REQUIRE(cols[e] >= 0 && cols[e] < n, FEMGPU_ERR_INVALID, "column index out of range");
         FG_REQUIRE(e == rowptr[i] || cols[e] > cols[e - 1], FEMGPU_ERR_INVALID, "columns must be sorted and unique");
@@ -388,6 +390,7 @@ femgpu_status femgpu_set_matrix_csr(femgpu_handle h, int64_t n, const int32_t* r
     DCsr<double>& A = h->A;
     A.n = A.m = (int)n;
     A.nnz = nnz;
+    h->A_max_row = longest;
     A.rp.alloc(n + 1, s);
     A.rp.upload(rowptr, n + 1);
     A.ci.alloc(nnz > 0 ? nnz : 1, s);

@@ -83,6 +83,7 @@ constexpr int kSlotRowMax = 32;
 template <class T>
 struct Level {
   int n = 0, nagg = 0, npart = 0;
+  int max_row = 0;  // entries of A's longest row (0: not known), used while the level is built
   bool coarsest = false;
   DCsr<T> A;
   DBuf<int32_t> gxadj, gadj;  // aggregation graph of this level
@@ -195,6 +196,7 @@ struct Ctx {
   DBuf<uint8_t> dmask;           // Dirichlet mask of the last femgpu_set_dirichlet (empty: none)
   bool assembled_from_mesh = false;
   DCsr<double> A;                // level-0 operator, original numbering, FP64
+  int A_max_row = 0;             // entries of its longest row
   DBuf<int32_t> gxadj, gadj;     // level-0 aggregation graph
   int64_t graph_nnz = 0;
   bool has_matrix = false;

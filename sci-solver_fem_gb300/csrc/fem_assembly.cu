@@ -600,7 +600,8 @@ void build_mesh_pattern(Ctx& c) {
   FG_LAUNCH(compact_rows_kernel, grid_for((int64_t)nv * 32, 256), 256, 0, s, cand.p, coff.p, c.A.rp.p, nv, c.A.ci.p);
   // slot map for the assembly's row gather, when every row fits its shared-memory sums
   M.slot.release();
-  if (reduce_max_row_length(c) <= kSlotRowMax) {
+  c.A_max_row = reduce_max_row_length(c);
+  if (c.A_max_row <= kSlotRowMax) {
     M.slot.alloc((size_t)nslots * k, s);
     DBuf<int32_t> bad2(1, s);
     bad2.zero();

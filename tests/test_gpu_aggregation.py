@@ -39,3 +39,34 @@ def test_square_sizes(n):
     (21, dict(partitionMaxSize=450, seed=7)), (21, dict(randMisParameters=50102))])
 def test_cube_options(n, opts):
     check(*meshes.kuhn_cube(n), **opts)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("half", [2, 7, 8, 31, 32, 63, 64, 100])
+def test_banded_hierarchies(half, precision):
+    # rows of 5, 15, 17, 63, 65, 127, 129 and 201 entries: the row tiers of the permuted operator
+    # and the prolongator (16, 64, 128, 256), products with and without direct slots
+    n = 4000
+    rng = np.random.default_rng(half)
+    i = np.arange(n)
+    lo, hi = np.maximum(0, i - half), np.minimum(n, i + half + 1)
+    rp = np.zeros(n + 1, np.int32)
+    np.cumsum(hi - lo, out=rp[1:])
+    rows = np.repeat(i, hi - lo)
+    ci = (np.arange(rp[-1]) - np.repeat(rp[:-1], hi - lo) + np.repeat(lo, hi - lo)).astype(np.int32)
+    w = rng.uniform(0.5, 1.0, (n, half + 1))
+    v = np.where(ci == rows, 0.0, -w[np.minimum(rows, ci), np.abs(rows - ci)])
+    v[ci == rows] = 1.0 - np.bincount(rows, weights=v, minlength=n)
+    gx, ga = meshes.adjacency_from_pattern(rp, ci)
+    part = 512 if 7 <= half < 60 else 1024
+    orc = O.OracleAMG(rp, ci, v, gx, ga, seed=1, fp64_hierarchy=precision, max_levels=2, partition_max=part)
+    with femgpu.Solver(precision=precision, maxLevels=2, partitionMaxSize=part) as s:
+        s.set_matrix_csr(rp, ci, v)
+        s.setup()
+        assert s.num_levels == orc.num_levels
+        for l in range(orc.num_levels):
+            got, want = s.level(l), orc.level(l)
+            for key in want:
+                assert np.array_equal(got[key], want[key]), (l, key)
+        r = rng.standard_normal(n)
+        assert np.array_equal(s.vcycle(r), orc.vcycle(r))
