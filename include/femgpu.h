@@ -72,10 +72,10 @@ typedef struct {
   void* mem_pool;           /* cudaMemPool_t for device buffers; NULL = a pool owned by the handle
                                that keeps freed memory for reuse until femgpu_destroy */
   int autotune;             /* 1 (default): at setup, time each level's result-neutral launch
-                               choices (cross-partition lanes per row, cluster smoother CTAs per
-                               group) once per device and level shape and keep the fastest; the
-                               choices are cached for the process, and in the file named by the
-                               environment variable FEMGPU_TUNE_CACHE when set.  0: fixed rules */
+                               choice (cross-partition lanes per row) once per device and level
+                               shape and keep the fastest; the choices are cached for the
+                               process, and in the file named by the environment variable
+                               FEMGPU_TUNE_CACHE when set.  0: fixed rules */
   int smoother;             /* 0 (default): the reference's partition-block weighted Jacobi
                                (gauss_seidel.cu dsType 0); 1: l1-Jacobi on every level's whole
                                operator, x += w (b - A x) / l1 with l1_i = sum_j |a_ij|,

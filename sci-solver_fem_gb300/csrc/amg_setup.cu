@@ -2999,6 +2999,54 @@ __global__ void __launch_bounds__(1024) partition_starts_kernel(int npart, const
   }
 }
 
+// Rank of a lane's row in its 32-row block: by decreasing length, ties by row.
+__device__ __forceinline__ int block_rank(bool live, int len, int lane) {
+  const unsigned key = live ? ((unsigned)(len + 1) << 5) | (unsigned)(31 - lane) : 0u;
+  int rank = 0;
+  for (int j = 0; j < 32; j++) rank += __shfl_sync(0xffffffffu, key, j) > key;
+  return rank;
+}
+
+// The copy of x that a lane's column a reads (a < 0: none), the warp's lanes reading together;
+// load: per bank, the distinct columns that have chosen it (the warp's scratch).
+template <class T, int NC>
+__device__ __forceinline__ int choose_copies(int a, int* load) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int NB = sizeof(T) == 4 ? 32 : 16;  // bank slots of one element size
+  constexpr int SHIFT = NB / kXCopies;          // bank slots between copies
+  if (NC == 1) return 0;
+  const int lane = threadIdx.x & 31;
+  const unsigned same = __match_any_sync(kAll, a);
+  const int leader = __ffs(same) - 1;
+  bool choosing = a >= 0 && leader == lane;
+  int copy = 0;
+  if (lane < NB) load[lane] = 0;
+  __syncwarp();
+  while (__any_sync(kAll, choosing)) {
+    int bank = -1 - lane;
+    if (choosing) {
+      int best = 0;
+#pragma unroll
+      for (int c = 0; c < NC; c++) {
+        const int lb = load[(a + c * SHIFT) % NB];
+        if (c == 0 || lb < best) {
+          best = lb;
+          copy = c;
+        }
+      }
+      bank = (a + copy * SHIFT) % NB;
+    }
+    const unsigned rivals = __match_any_sync(kAll, bank);
+    __syncwarp();
+    if (choosing && __ffs(rivals) - 1 == lane) {
+      load[bank]++;
+      choosing = false;
+    }
+    __syncwarp();
+  }
+  return __shfl_sync(kAll, copy, leader);
+}
+
 // The register smoother's entry layout, one CTA of 512 threads per group, warp w taking
 // the group's rows [rs + 32w, rs + 32w + 32) (a block):
 // * the block's rows are ranked by decreasing in-partition length (ties: lower row
@@ -3021,7 +3069,6 @@ __global__ void __launch_bounds__(512) jds_build_kernel(const int32_t* __restric
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int CS = xcopy_stride<T>();
   constexpr int NB = sizeof(T) == 4 ? 32 : 16;  // bank slots of one element size
-  constexpr int SHIFT = NB / kXCopies;          // bank slots between copies
   const int rs = grows[blockIdx.x], re = grows[blockIdx.x + 1];
   const int lane = threadIdx.x & 31;
   const int r0 = rs + (threadIdx.x & ~31);
@@ -3029,9 +3076,7 @@ __global__ void __launch_bounds__(512) jds_build_kernel(const int32_t* __restric
   const int row = r0 + lane;
   const bool live = row < re;
   const int len = live ? irp[row + 1] - irp[row] : 0;
-  const unsigned key = live ? ((unsigned)(len + 1) << 5) | (unsigned)(31 - lane) : 0u;
-  int rank = 0;
-  for (int j = 0; j < 32; j++) rank += __shfl_sync(kAll, key, j) > key;
+  const int rank = block_rank(live, len, lane);
   if (live) jrow[r0 + rank] = (uint8_t)lane;
   const int eb = irp[r0];
   const int mine = live ? irp[row] : 0;
@@ -3043,41 +3088,63 @@ __global__ void __launch_bounds__(512) jds_build_kernel(const int32_t* __restric
     const unsigned am = __ballot_sync(kAll, act);
     if (!am) break;
     const int a = act ? ici[mine + k] - rs : -1;
-    const unsigned same = __match_any_sync(kAll, a);
-    const int leader = __ffs(same) - 1;
-    bool choosing = act && leader == lane;
-    int copy = 0;
-    if (lane < NB) load[lane] = 0;
-    __syncwarp();
-    while (__any_sync(kAll, choosing)) {
-      int bank = -1 - lane;
-      if (choosing) {
-        int best = 0;
-#pragma unroll
-        for (int c = 0; c < kXCopies; c++) {
-          const int lb = load[(a + c * SHIFT) % NB];
-          if (c == 0 || lb < best) {
-            best = lb;
-            copy = c;
-          }
-        }
-        bank = (a + copy * SHIFT) % NB;
-      }
-      const unsigned rivals = __match_any_sync(kAll, bank);
-      __syncwarp();
-      if (choosing && __ffs(rivals) - 1 == lane) {
-        load[bank]++;
-        choosing = false;
-      }
-      __syncwarp();
-    }
-    copy = __shfl_sync(kAll, copy, leader);
+    const int copy = choose_copies<T, kXCopies>(a, load);
     if (act) {
       const int dst = eb + dk + rank;
       jv[dst] = iv[mine + k];
       jc[dst] = (uint16_t)(a + copy * CS);
     }
     dk += __popc(am);
+  }
+}
+
+// Padded row lengths of the row smoother's layout: whole quads.
+__global__ void quad_len_kernel(int n, const int32_t* __restrict__ irp, int32_t* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = (irp[i + 1] - irp[i] + 3) & ~3;
+}
+
+// The row smoother's entry layout: blocks, ranks and copies as in jds_build_kernel, but four
+// consecutive entries of a row stay together (one 128-bit load of FP32 values, one 64-bit load
+// of columns).  Quad q of the row ranked p starts at qrp[block's first row] + 4 (m_0 + ... +
+// m_{q-1} + p), m_q = rows of the block longer than 4 q; a row's last quad is filled with zero
+// values that point at the zero slot kRegGroupRows of copy 0.  qrp: exclusive scan of
+// quad_len_kernel's lengths.
+template <class T, int NC>
+__global__ void __launch_bounds__(512) quad_build_kernel(const int32_t* __restrict__ grows,
+                                                         const int32_t* __restrict__ irp,
+                                                         const int32_t* __restrict__ ici, const T* __restrict__ iv,
+                                                         const int32_t* __restrict__ qrp, T* __restrict__ rv,
+                                                         uint16_t* __restrict__ rc, uint8_t* __restrict__ rrow) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int CS = xcopy_stride<T>();
+  const int rs = grows[blockIdx.x], re = grows[blockIdx.x + 1];
+  const int lane = threadIdx.x & 31;
+  const int r0 = rs + (threadIdx.x & ~31);
+  if (r0 >= re) return;  // the whole warp: its block is empty
+  const int row = r0 + lane;
+  const bool live = row < re;
+  const int mine = live ? irp[row] : 0;
+  const int len = live ? irp[row + 1] - mine : 0;
+  const int rank = block_rank(live, len, lane);
+  if (live) rrow[r0 + rank] = (uint8_t)lane;
+  __shared__ int s_load[16][sizeof(T) == 4 ? 32 : 16];
+  int* const load = s_load[threadIdx.x >> 5];
+  int at = qrp[r0] + 4 * rank;
+  for (int q = 0;; q += 4) {
+    const unsigned am = __ballot_sync(kAll, q < len);
+    if (!am) break;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const bool act = q + i < len;
+      const int a = act ? ici[mine + q + i] - rs : -1;
+      const int copy = choose_copies<T, NC>(a, load);
+      if (q < len) {
+        rv[at + i] = act ? iv[mine + q + i] : (T)0;
+        rc[at + i] = (uint16_t)(act ? a + copy * CS : kRegGroupRows);
+      }
+    }
+    at += 4 * __popc(am);
   }
 }
 
@@ -3281,6 +3348,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
                 "slice %d rows / %d entries, %d threads, %zu B shared%s\n",
                 num_levels - 1,
                 smoother_in_registers(L.max_in_row, L.max_part_rows) ? "registers"
+                : L.rows_c > 0                                        ? "rows"
                 : L.smooth_k > 0                                      ? "cluster, entries in registers"
                                                                       : "cluster",
                 L.ngroups, L.max_group_rows, L.smooth_lanes, L.cluster, L.slice_rows, L.slice_ents,
@@ -3581,5 +3649,25 @@ void amg_setup(Ctx& c) {
   c.has_hierarchy = true;
   c.hier_gen++;  // invalidates the captured PCG iteration graph
 }
+
+// The row smoother's layout of a level (quad_build_kernel), with the copies of x spread over the
+// banks or (copies == 1) the plain columns.
+template <class T>
+void build_row_layout(Ctx& c, Level<T>& L, int copies) {
+  cudaStream_t s = c.stream;
+  const size_t cap = (size_t)L.Ain.nnz + 3 * (size_t)L.n + 16;  // padded rows, slack for bulk copies
+  L.rv.alloc(cap, s);
+  L.rc.alloc(cap, s);
+  L.rrow.alloc(L.n, s);
+  L.qrp.alloc((size_t)L.n + 1, s);
+  DBuf<int32_t> len(L.n, s);
+  FG_LAUNCH(quad_len_kernel, grid_for(L.n, 256), 256, 0, s, L.n, L.Ain.rp.p, len.p);
+  exclusive_scan_async(len.p, L.qrp.p, L.n, s);
+  auto k = copies == 1 ? quad_build_kernel<T, 1> : quad_build_kernel<T, kXCopies>;
+  FG_LAUNCH(k, L.ngroups, kRegGroupRows, 0, s, L.grows.p, L.Ain.rp.p, L.Ain.ci.p, L.Ain.v.p, L.qrp.p, L.rv.p, L.rc.p,
+            L.rrow.p);
+}
+template void build_row_layout<float>(Ctx&, Level<float>&, int);
+template void build_row_layout<double>(Ctx&, Level<double>&, int);
 
 }  // namespace femgpu

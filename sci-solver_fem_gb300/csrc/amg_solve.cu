@@ -819,6 +819,206 @@ __global__ void __launch_bounds__(512) smooth_split_kernel(
   cl.sync();  // no CTA leaves while another may still write its copy of x
 }
 
+__device__ __forceinline__ void load_quad(const float* p, float (&v)[4]) {
+  const float4 q = *reinterpret_cast<const float4*>(p);
+  v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+}
+__device__ __forceinline__ void load_quad(const double* p, double (&v)[4]) {
+  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+  v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+
+// Shared memory of the row smoother: the mbarrier, x twice, the staged values and columns of
+// `ecap` entries (filled as 16-byte rounded ranges).
+struct RowSmemLayout {
+  size_t xa, xb, val, col, total;
+};
+
+template <class T>
+__host__ __device__ inline RowSmemLayout row_smem_layout(int ecap) {
+  RowSmemLayout L{};
+  constexpr size_t xbytes = (size_t)(sizeof(T) == 8 ? 1 : kXCopies) * xcopy_stride<T>() * sizeof(T);
+  L.xa = 16;
+  L.xb = L.xa + xbytes;
+  L.val = round16<T>(L.xb + xbytes);
+  L.col = round16<T>(L.val + (size_t)ecap * sizeof(T));
+  L.total = round16<T>(L.col + (size_t)ecap * 2);
+  return L;
+}
+
+// Row smoother, for levels with many groups and rows of any length: a thread per row, a CTA
+// (FP64: a cluster of C CTAs, each with a slice of whole 32-row blocks) per group.  With the
+// lanes of smooth_creg_kernel a level of 267 groups takes 3.5 waves of 2 CTAs per SM, each of
+// which waits for its entries (rows read lane by lane, uncoalesced) and for 6 cluster barriers.
+// Here the entries are laid out at setup (quad_build_kernel: jagged diagonals of quads, columns
+// spread over the copies of x as in smooth_reg_kernel) and arrive in one bulk copy each for
+// values and columns; a sweep reads 4 entries with one 128-bit and one 64-bit load from
+// consecutive addresses plus 4 gathers, all groups of 304 CTAs fit one wave, and a sweep ends
+// with a block barrier.  The S accumulators of a row are those of its S lanes, summed in the
+// butterfly's order: the same x.  Measured per relax (pre, post), FP32: 267 groups 34.3, 32.7 ->
+// 17.4, 15.6 us; 123 groups 33.5, 33.8 -> 12.3, 11.3 us.  FP64, bound by the FP64 units, which
+// spend as long on a warp's 8 live lanes as on 32: 32 groups (4 CTAs each) 36.6, 32.1 -> 29.6,
+// 25.6 us; 123 groups 107, 91 -> 52, 44 us.  One entry at a time (8 loads in flight) instead of
+// quads: 21.7, 19.0 us at 267 groups; a branch per entry instead of selects: 24.5, 21.1 us.
+// A copy that does not land within `wait_limit` polls sets *kerr; the CTA then runs on without
+// entries (its cluster waits for it at every sweep) and leaves when its copies have landed.
+template <class T, bool POST, int S>
+__global__ void __launch_bounds__(512) smooth_rows_kernel(
+    const int32_t* __restrict__ grows, const int32_t* __restrict__ irp, const int32_t* __restrict__ qrp,
+    const uint16_t* __restrict__ rc, const T* __restrict__ rv, const uint8_t* __restrict__ rrow, const T* __restrict__ diag,
+    const T* __restrict__ dinv, const T* __restrict__ b, T w, int inner, const T* __restrict__ x_in,
+    T* __restrict__ x_out, T* __restrict__ r_out, int ecap, double* __restrict__ kerr, int wait_limit) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr bool CL = sizeof(T) == 8;  // groups over clusters, one copy of x
+  constexpr int NC = CL ? 1 : kXCopies;
+  constexpr int CS = xcopy_stride<T>();
+  const RowSmemLayout Ls = row_smem_layout<T>(ecap);
+  uint64_t* const bar = reinterpret_cast<uint64_t*>(sm);
+  T* const xa = reinterpret_cast<T*>(sm + Ls.xa);
+  T* const xb = reinterpret_cast<T*>(sm + Ls.xb);
+  int C = 1, c = 0;
+  if (CL) {
+    C = (int)cg::this_cluster().num_blocks();
+    c = (int)cg::this_cluster().block_rank();
+  }
+  const int g = blockIdx.x / C;
+  const int rs = grows[g], m = grows[g + 1] - rs;
+  const int qs = CL ? ((m + C - 1) / C + 31) / 32 * 32 : m;
+  const int ss = min(m, c * qs), ns = min(m, ss + qs) - ss;  // own slice: group rows [ss, ss + ns)
+  const int es = qrp[rs + ss];  // a multiple of 4, as every block's and row's first entry
+  const int t = threadIdx.x, lane = t & 31;
+  if (t == 0) {
+    mbar_init(bar, 1);
+    const int ee = qrp[rs + ss + ns];
+    const int c0 = es & ~7;
+    const uint32_t vbytes = (uint32_t)((ee - es) * (int)sizeof(T));
+    const uint32_t cbytes = (uint32_t)((((ee + 7) & ~7) - c0) * 2);
+    mbar_arrive_expect_tx(bar, vbytes + cbytes);
+    if (vbytes) bulk_copy_g2s(sm + Ls.val, rv + es, vbytes, bar);
+    if (cbytes) bulk_copy_g2s(sm + Ls.col, rc + c0, cbytes, bar);
+  }
+  __syncthreads();  // the mbarrier is initialised
+  const int wb = rs + ss + (t & ~31);  // first row of this warp's 32-row block
+  const bool live = t < ns;
+  const int eb = (t & ~31) < ns ? qrp[wb] : es;  // the block's first entry
+  const int nrow = rs + ss + t;
+  int jr = 0, ne0 = 0, ne1 = 0;
+  T nd = (T)1, ndi = (T)1, nb = (T)0, nx = (T)0;
+  if (live) {
+    jr = rrow[nrow];
+    ne0 = irp[nrow];
+    ne1 = irp[nrow + 1];
+    nd = diag[nrow];
+    ndi = dinv[nrow];
+  }
+  // everything above reads constant data and writes only this CTA's shared memory
+  pdl_enter();
+  if (live) {
+    nb = b[nrow];
+    if (POST) nx = x_in[nrow];
+  }
+  if (t == 0) xa[kRegGroupRows] = xb[kRegGroupRows] = (T)0;  // the padding's x
+  if (CL)
+    for (int q = t; q < m; q += blockDim.x) {
+      const int r = rs + q;
+      xa[q] = POST ? x_in[r] : (w * b[r]) * dinv[r];
+    }
+  // natural row order to the block's sorted order; every lane executes every shuffle
+  const int row = wb + jr;
+  const int loc = row - rs;
+  const int e0 = __shfl_sync(kAll, ne0, jr), e1 = __shfl_sync(kAll, ne1, jr);
+  const T d = __shfl_sync(kAll, nd, jr), di = __shfl_sync(kAll, ndi, jr);
+  const T bb = __shfl_sync(kAll, nb, jr), xs = __shfl_sync(kAll, nx, jr);
+  T x = POST ? xs : (w * bb) * di;
+  if (!CL && live) {
+#pragma unroll
+    for (int q = 0; q < NC; q++) xa[loc + q * CS] = x;
+  }
+  const bool bad = __syncthreads_or(!mbar_wait_bounded(bar, 0, wait_limit));
+  if (CL) cg::this_cluster().sync();  // every CTA of the cluster is running and holds x0
+  const int len = live && !bad ? e1 - e0 : 0;
+  const int kmax = __shfl_sync(kAll, len, 0);  // lane 0 holds the block's longest row
+  const T* const pv = reinterpret_cast<const T*>(sm + Ls.val) + (eb - es);
+  const uint16_t* const pc = reinterpret_cast<const uint16_t*>(sm + Ls.col) + (eb - (es & ~7));
+  auto rowsum = [&](const T* src) {
+    constexpr int Q = S > 8 ? S / 4 : 2;  // quads per step: whole turns of the S sums
+    constexpr int F = 2;                  // quads in flight
+    T s[S];
+#pragma unroll
+    for (int j = 0; j < S; j++) s[j] = (T)0;
+    int at = 4 * lane;  // this lane's place on the block's quad
+#pragma unroll 1
+    for (int k = 0; k < kmax; k += 4 * Q) {
+#pragma unroll
+      for (int h = 0; h < Q; h += F) {
+        if (h == 0 || k + 4 * h < kmax) {
+          T v[F][4], xv[F][4];
+          // lanes past their row's end read the block's first quad and drop the products:
+          // plain loads and selects, no branches
+#pragma unroll
+          for (int f = 0; f < F; f++) {
+            const bool a = k + 4 * (h + f) < len;
+            const int q = a ? at : 0;
+            at += 4 * __popc(__ballot_sync(kAll, a));
+            load_quad(pv + q, v[f]);
+            const uint2 cc = *reinterpret_cast<const uint2*>(pc + q);
+            xv[f][0] = src[cc.x & 0xffffu];
+            xv[f][1] = src[cc.x >> 16];
+            xv[f][2] = src[cc.y & 0xffffu];
+            xv[f][3] = src[cc.y >> 16];
+          }
+#pragma unroll
+          for (int f = 0; f < F; f++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const int j = (4 * (h + f) + i) % S;
+              const T p = fma(v[f][i], xv[f][i], s[j]);
+              s[j] = k + 4 * (h + f) < len ? p : s[j];
+            }
+        }
+      }
+    }
+#pragma unroll
+    for (int off = S >> 1; off > 0; off >>= 1)
+#pragma unroll
+      for (int j = 0; j < off; j++) s[j] = s[j] + s[j + off];
+    return s[0];
+  };
+  const T* cur = xa;
+  T* nxt = xb;
+#pragma unroll 1
+  for (int it = 0; it < (POST ? inner : inner + 1); it++) {
+    const T sv = rowsum(cur);
+    if (!POST && it == inner) {  // the residual's sum, the one copy of the code kept small
+      if (live) {
+        T u = bb - sv;
+        r_out[row] = u - d * x;
+      }
+      break;
+    }
+    x = relax(x, bb, sv, d, di, w);
+    if (live) {
+      if (CL) {
+        for (int r = 0; r < C; r++) *cg::this_cluster().map_shared_rank(nxt + loc, r) = x;
+      } else {
+#pragma unroll
+        for (int q = 0; q < NC; q++) nxt[loc + q * CS] = x;
+      }
+    }
+    if (CL) cg::this_cluster().sync();  // all copies of the new x written; the old buffer is no longer read
+    else __syncthreads();
+    T* const tmp = const_cast<T*>(cur);
+    cur = nxt;
+    nxt = tmp;
+  }
+  if (live) x_out[row] = x;
+  if (bad && t == 0) {
+    *kerr = 1.0 + g;  // the host reports it; the copies in flight land before the CTA exits
+    (void)mbar_wait_bounded(bar, 0);
+  }
+}
+
 // r -= A_out x (preAout_kernel, gauss_seidel.cu:1977-2015).
 template <class T>
 __global__ void aout_residual_kernel(int n, const int32_t* __restrict__ orp, const int32_t* __restrict__ oci,
@@ -1334,6 +1534,20 @@ CregSmoothFn<T> pick_creg_kernel(bool post, int S, int K) {
   }
 }
 
+template <class T>
+using RowSmoothFn = void (*)(const int32_t*, const int32_t*, const int32_t*, const uint16_t*, const T*, const uint8_t*, const T*,
+                             const T*, const T*, T, int, const T*, T*, T*, int, double*, int);
+
+template <class T>
+RowSmoothFn<T> pick_row_kernel(bool post, int S) {
+  switch (S) {
+    case 2: return post ? smooth_rows_kernel<T, true, 2> : smooth_rows_kernel<T, false, 2>;
+    case 4: return post ? smooth_rows_kernel<T, true, 4> : smooth_rows_kernel<T, false, 4>;
+    case 8: return post ? smooth_rows_kernel<T, true, 8> : smooth_rows_kernel<T, false, 8>;
+    default: return post ? smooth_rows_kernel<T, true, 16> : smooth_rows_kernel<T, false, 16>;
+  }
+}
+
 // Launch with a 1-D thread-block cluster of `cluster` CTAs (counted like FG_LAUNCH).
 template <class... KArgs, class... Args>
 void launch_clustered(void (*k)(KArgs...), int grid, int block, size_t smem, int cluster, cudaStream_t s,
@@ -1522,6 +1736,15 @@ void smooth_sweeps(Ctx& c, Level<T>& L, bool post, const T* b, const T* xin, T* 
               c.red.p + 2 * kRedBlocks + S_KERR, f.b64, f.b_store, f.aout ? L.Aout.rp.p : nullptr,
               f.aout ? L.Aout.ci.p : nullptr, f.aout ? L.Aout.v.p : nullptr, f.z64, f.dot_r, f.dot_o, f.dot_part,
               c.rcount.p + 3, c.red.p + 2 * kRedBlocks, f.dot_o ? 1 : 0, c.copy_wait_limit);
+    return;
+  }
+  if (L.rows_c > 0) {
+    RowSmoothFn<T> k = pick_row_kernel<T>(post, L.smooth_lanes);
+    if (L.smooth_smem > 48 * 1024) ensure_smem(k, L.smooth_smem);
+    launch_clustered(k, L.ngroups * L.rows_c, L.smooth_threads, L.smooth_smem, L.rows_c, s, (const int32_t*)L.grows.p,
+                     (const int32_t*)L.Ain.rp.p, (const int32_t*)L.qrp.p, (const uint16_t*)L.rc.p, (const T*)L.rv.p, (const uint8_t*)L.rrow.p,
+                     (const T*)L.diag.p, (const T*)L.dinv.p, b, w, inner, xin, xout, rout, L.rows_ecap,
+                     c.red.p + 2 * kRedBlocks + S_KERR, c.copy_wait_limit);
     return;
   }
   if (L.smooth_k > 0) {
@@ -1920,10 +2143,54 @@ int split_clusters(int split) {
   return least;
 }
 
+// The row smoother with C CTAs per group: sets the plan and returns true when it fits.
+template <class T>
+bool row_plan(Ctx& c, Level<T>& L, int S, int C) {
+  // (one lane means rows of at most 16 entries in partitions of more than 512 rows)
+  if (S < 2 || S > 16 || L.max_group_rows > kRegGroupRows) return false;
+  const int qs = ((L.max_group_rows + C - 1) / C + 31) / 32 * 32;
+  const int ecap =
+      (int)std::min<int64_t>(L.max_group_ents + 3 * (int64_t)L.max_group_rows, (int64_t)qs * (L.max_in_row + 3)) + 16;
+  const size_t sm = row_smem_layout<T>(ecap).total;
+  if (sm > kSmemOptIn) return false;
+  for (int post = 0; post < 2; post++) {
+    RowSmoothFn<T> k = pick_row_kernel<T>(post != 0, S);
+    if (sm > 48 * 1024) ensure_smem(k, sm);
+    int clusters = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(L.ngroups * C));
+    cfg.blockDim = dim3((unsigned)qs);
+    cfg.dynamicSmemBytes = sm;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)C;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, k, &cfg);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    if (e != cudaSuccess || clusters <= 0) return false;
+  }
+  L.smooth_lanes = S;
+  L.smooth_k = 0;
+  L.cluster = C;
+  L.slice_rows = qs;
+  L.slice_ents = 0;
+  L.smooth_staged = false;
+  L.smooth_smem = sm;
+  L.smooth_threads = qs;
+  L.rows_c = C;
+  L.rows_ecap = ecap;
+  build_row_layout(c, L, sizeof(T) == 8 ? 1 : kXCopies);
+  return true;
+}
+
 template <class T>
 void plan_smoother(Ctx& c, Level<T>& L) {
   cudaStream_t s = c.stream;
   L.split = 1;
+  L.rows_c = 0;
   if (smoother_in_registers(L.max_in_row, L.max_part_rows)) {
     L.smooth_lanes = 1;
     L.cluster = 1;
@@ -1959,14 +2226,33 @@ void plan_smoother(Ctx& c, Level<T>& L) {
   const int mcap = L.max_group_rows;
   L.smooth_lanes = S;
   L.smooth_k = 0;
-  // register-resident entries: at most 16 per lane, one row slice per CTA of <= 1024
-  // threads, 16-bit group-local columns
+  int sms = 0;
+  FG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
+  // Lane smoother: at most 16 entries per lane, one row slice per CTA of <= 1024 threads, 16-bit
+  // group-local columns.  Its time falls with the CTAs per group as long as all CTAs run at once
+  // (FP64, 2 groups of 250 rows: 2 CTAs 25.9 us, 4 17.1, 8 13.5; FP32, 1 CTA 10.0, 2 8.3, 3 to 8
+  // 7.7) and nearly doubles with the second wave (FP32, 32 groups: 4 CTAs 10.2 us, 5 15.4):
+  // the most that do.
   const int per_lane = (L.max_in_row + S - 1) / S;
   const int rows_per_cta = 1024 / S;
-  const int creg_c = (mcap + rows_per_cta - 1) / rows_per_cta;
-  if (per_lane <= kLaneEntries && creg_c <= kMaxCluster && mcap < 65535) {
-    const int K = per_lane <= 8 ? 8 : 16;
-    for (int C = std::max(1, creg_c); C <= kMaxCluster; C++)
+  const int creg_c = std::max(1, (mcap + rows_per_cta - 1) / rows_per_cta);
+  const bool creg = per_lane <= kLaneEntries && creg_c <= kMaxCluster && mcap < 65535;
+  const int K = per_lane <= 8 ? 8 : 16;
+  const int fit = std::max(1, std::min(kMaxCluster, sms / std::max(1, L.ngroups)));  // CTAs per group in one wave
+  // Row smoother instead where the lanes need a second wave (FP32, 41 groups: 17.1 against 11.2
+  // to 12.8 us; 123 groups: 33 against 12; 267 groups: 33 to 40 against 16; 33 groups, one wave:
+  // 8.5 against 9.0 to 10.4), in FP64 where they get fewer than 6 CTAs (32 groups, 4 CTAs: 36
+  // against 28; 11 groups, 8 CTAs: 21 against 25; 123 groups: 99 against 48).
+  if (fit < (sizeof(T) == 8 ? 6 : creg_c)) {
+    int C = 1;
+    if (sizeof(T) == 8)
+      while (C < 4 && 2 * C <= fit) C *= 2;
+    if (row_plan(c, L, S, C)) return;
+  }
+  if (creg) {
+    for (int C = std::max(creg_c, fit); C >= creg_c; C--)
+      if (creg_plan(c, L, S, K, C)) return;
+    for (int C = std::max(creg_c, fit) + 1; C <= kMaxCluster; C++)
       if (creg_plan(c, L, S, K, C)) return;
   }
   int C = (int)std::min<int64_t>(kMaxCluster, ((int64_t)mcap * S + 1023) / 1024);
@@ -2131,27 +2417,6 @@ void autotune_level(Ctx& c, Level<T>& L) {
     }
     L.aout_lanes_tuned = best;
     if (verbose) fprintf(stderr, "[femgpu tune] level n=%d cross-partition lanes %d\n", L.n, best);
-  }
-  // CTAs per cluster of the register-resident cluster smoother
-  if (!smoother_in_registers(L.max_in_row, L.max_part_rows) && L.smooth_k > 0) {
-    const std::string key = dev + "|creg|" + shape;
-    const int S = L.smooth_lanes, K = L.smooth_k, C0 = L.cluster;
-    int best = 0;
-    if (!tune_lookup(key, &best)) {
-      float tbest = 1e30f;
-      for (int C = C0; C <= kMaxCluster; C++) {
-        if (!creg_plan(c, L, S, K, C)) continue;
-        const float t = time_launches(s, [&] { smooth_sweeps<T>(c, L, false, L.b.p, nullptr, L.x.p, L.r.p); });
-        if (t < tbest) {
-          tbest = t;
-          best = C;
-        }
-      }
-      tune_store(key, best);
-    }
-    if (best < C0 || !creg_plan(c, L, S, K, best))
-      FG_REQUIRE(creg_plan(c, L, S, K, C0), FEMGPU_ERR_LIMIT, "no resident configuration for the cluster smoother");
-    if (verbose) fprintf(stderr, "[femgpu tune] level n=%d cluster smoother CTAs per group %d\n", L.n, L.cluster);
   }
 }
 
@@ -2657,8 +2922,8 @@ void profile_level0(Ctx& c, Hierarchy<T>& H, int which, int reps, double* ms, do
   // in-partition entries: value + 16-bit column on the register path (plus one byte per
   // row for its place in its block), value + 32-bit column otherwise
   const bool reg = smoother_in_registers(L.max_in_row, L.max_part_rows);
-  const double ein = reg ? ts + 2 : ts + 4;
-  const double rowb = reg ? 1.0 * n : 0.0;
+  const double ein = reg || L.rows_c > 0 ? ts + 2 : ts + 4;
+  const double rowb = reg || L.rows_c > 0 ? 1.0 * n : 0.0;
   switch (which) {
     case 1:  // entries, row offsets, b, diag, 1/diag in; x, r out
       *bytes = L.Ain.nnz * ein + 4.0 * (n + 1) + 3 * ts * n + 2 * ts * n + rowb;

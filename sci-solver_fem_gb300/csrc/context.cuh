@@ -109,6 +109,14 @@ struct Level {
   DBuf<T> jv;
   DBuf<uint16_t> jc16;
   DBuf<uint8_t> jrow;
+  // row smoother (rows_c > 0: its CTAs per group): in-partition entries in quads of the same
+  // block order (quad_build_kernel), built with the launch plan; qrp: first padded entry per
+  // row, rows_ecap: staged entries per CTA
+  DBuf<T> rv;
+  DBuf<uint16_t> rc;
+  DBuf<uint8_t> rrow;
+  DBuf<int32_t> qrp;
+  int rows_c = 0, rows_ecap = 0;
   // shared-memory smoother plan: lanes per row, CTAs per cluster (one cluster per
   // group), rows and entries of the largest CTA row slice, launch shape
   int smooth_lanes = 1, cluster = 1, slice_rows = 0, slice_ents = 0, smooth_threads = 0, smooth_grid = 0;
@@ -291,8 +299,10 @@ SolveResult amg_solve_device(Ctx& c, const double* d_b, double* d_x);
 // Chooses the smoother's launch plan for a level whose groups are built.
 template <class T>
 void plan_smoother(Ctx& c, Level<T>& L);
-// Times the level's result-neutral launch choices (cross-partition lanes, cluster size) and
-// keeps the fastest (cached per device and level shape); no-op when cfg.autotune is 0.
+template <class T>
+void build_row_layout(Ctx& c, Level<T>& L, int copies);
+// Times the level's result-neutral launch choice (cross-partition lanes) and keeps the
+// fastest (cached per device and level shape); no-op when cfg.autotune is 0.
 template <class T>
 void autotune_level(Ctx& c, Level<T>& L);
 // The PCG solves of several handles (same device, hierarchies built) as one CUDA graph
