@@ -1630,15 +1630,22 @@ __global__ void aout_lanes_kernel(int n, const int32_t* __restrict__ orp, const 
   if (live && j == 0) out[g] = RHS ? acc : acc - sum;
 }
 
-// Lanes per row of the cross-partition kernels: 1 (per-thread gather) below 8 entries
-// per row on average, else a power of two near a quarter of the average row.
+// Lanes per row of the cross-partition kernels (any number gives the same sums).  S lanes
+// shorten a row's chain of dependent loads but multiply the adds, which every lane executes: at
+// most one lane per 1.5 entries of an average row, while all rows' lanes stay near one wave of
+// threads (FP64: a ninth of it and at most 4, an add being 64 cycles of a warp's FP64 unit).
+// Measured, us at S = 1, 2, 4, 8, 16, 32: FP32, 2.1 M rows of 4.2 entries 31, 40, 57, 133, 345,
+// 1001 (rule: 1); 80 k rows of 14.4: 8.8, 7.7, 8.5, 10, 17, 47 (2); 8.8 k of 12.6: 6.6, 5.9, 4.8,
+// 4.7, 5.1, 8.6 (8); 2.8 k of 32: 12.7, 12.1, 7.5, 6.0, 5.2, 5.5 (16).  FP64, 275 k of 4.0: 17, 29,
+// 49, 161, 552, 1826 (1); 10.6 k of 12.4: 11.6, 10.8, 11.2, 14, 29, 102 (2); 1.6 k of 8.9: 9.9, 9.0,
+// 7.9, 8.6, 9.0, 24 (4).
 template <class T>
 int aout_lanes(const Level<T>& L) {
   if (L.aout_lanes_tuned > 0) return L.aout_lanes_tuned;  // chosen by the autotuner (same sums)
-  const double avg = L.n > 0 ? (double)L.Aout.nnz / L.n : 0.0;
-  if (avg < 8.0) return 1;
-  int s = 2;
-  while (s < 32 && s * 4 < avg) s <<= 1;
+  const int most = sizeof(T) == 8 ? 4 : 32;
+  const int64_t threads = sizeof(T) == 8 ? 32768 : 262144;
+  int s = 1;
+  while (s < most && 3 * (int64_t)s * L.n <= L.Aout.nnz && 2 * (int64_t)s * L.n <= threads) s <<= 1;
   return s;
 }
 
@@ -2305,12 +2312,11 @@ template void plan_smoother<float>(Ctx&, Level<float>&);
 template void plan_smoother<double>(Ctx&, Level<double>&);
 
 // ---- autotuner ---------------------------------------------------------------------------
-// Launch shapes that do not change any result are picked per level by timing the level's
-// own kernels once: the lanes per row of the cross-partition products (every lane count
-// adds the products in entry order), and the CTAs per cluster of the register-resident
-// cluster smoother (a row's sums never cross CTAs).  Choices are cached per device and
-// level shape for the life of the process, and in the file named by FEMGPU_TUNE_CACHE
-// when it is set (one "key value" per line).
+// A launch shape that does not change any result is checked per level by timing the level's
+// own kernel once: the lanes per row of the cross-partition products (every lane count adds the
+// products in entry order).  The rule's choice is kept unless half or twice as many lanes take
+// less than 0.9 of its time.  Choices are cached per device and level shape for the life of the
+// process, and in the file named by FEMGPU_TUNE_CACHE when it is set (one "key value" per line).
 namespace {
 
 std::mutex g_tune_mu;
@@ -2355,7 +2361,13 @@ void tune_store(const std::string& key, int value) {
     }
 }
 
+// Name and SM count of a device (its properties take the driver longer than a small kernel:
+// read once per device).
 std::string device_tag(int device) {
+  std::lock_guard<std::mutex> lock(g_tune_mu);
+  static std::map<int, std::string>* tags = new std::map<int, std::string>();
+  std::string& tag = (*tags)[device];
+  if (!tag.empty()) return tag;
   cudaDeviceProp p;
   if (cudaGetDeviceProperties(&p, device) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -2364,60 +2376,67 @@ std::string device_tag(int device) {
   std::string n = p.name;
   for (char& ch : n)
     if (ch == ' ') ch = '_';
-  return n + "_sm" + std::to_string(p.multiProcessorCount);
+  return tag = n + "_sm" + std::to_string(p.multiProcessorCount);
 }
 
-// average time of `reps` launches of fn (after one untimed launch)
+// Shortest of kTimed launches of fn (after one untimed launch), each between two events: a
+// delay of the host between launches lengthens one of them, an average took it for the kernel
+// (2.1 M rows, 3 launches: 4 lanes chosen, 57 us, where 1 takes 31).
+constexpr int kTimed = 5;
 template <class F>
-float time_launches(cudaStream_t s, F&& fn, int reps = 3) {
+float time_launches(cudaStream_t s, F&& fn) {
+  cudaEvent_t e[kTimed + 1];
+  for (cudaEvent_t& x : e) FG_CUDA(cudaEventCreate(&x));
   fn();
-  cudaEvent_t e0, e1;
-  FG_CUDA(cudaEventCreate(&e0));
-  FG_CUDA(cudaEventCreate(&e1));
-  FG_CUDA(cudaEventRecord(e0, s));
-  for (int i = 0; i < reps; i++) fn();
-  FG_CUDA(cudaEventRecord(e1, s));
-  FG_CUDA(cudaEventSynchronize(e1));
-  float ms = 0;
-  FG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  return ms / reps;
+  for (int i = 0; i <= kTimed; i++) {
+    if (i > 0) fn();
+    FG_CUDA(cudaEventRecord(e[i], s));
+  }
+  FG_CUDA(cudaEventSynchronize(e[kTimed]));
+  float best = 1e30f;
+  for (int i = 0; i < kTimed; i++) {
+    float ms = 0;
+    FG_CUDA(cudaEventElapsedTime(&ms, e[i], e[i + 1]));
+    best = std::min(best, ms);
+  }
+  for (cudaEvent_t& x : e) cudaEventDestroy(x);
+  return best;
 }
 
 }  // namespace
 
 template <class T>
 void autotune_level(Ctx& c, Level<T>& L) {
-  if (!c.cfg.autotune || L.coarsest || L.n == 0) return;
+  if (!c.cfg.autotune || L.coarsest || L.n == 0 || L.Aout.nnz == 0) return;
   cudaStream_t s = c.stream;
-  const std::string dev = device_tag(c.device);
-  const std::string shape = std::to_string(sizeof(T)) + "_" + std::to_string(L.n) + "_" + std::to_string(L.Ain.nnz) +
-                            "_" + std::to_string(L.Aout.nnz) + "_" + std::to_string(L.max_group_rows);
-  const bool verbose = getenv("FEMGPU_PROFILE") != nullptr;
-  // inputs of the timed launches: finite values in the level's work vectors
-  FG_CUDA(cudaMemsetAsync(L.x.p, 0, L.x.n * sizeof(T), s));
-  FG_CUDA(cudaMemsetAsync(L.r.p, 0, L.r.n * sizeof(T), s));
-  FG_CUDA(cudaMemsetAsync(L.b.p, 0, L.b.n * sizeof(T), s));
-  // cross-partition lanes
-  if (L.Aout.nnz > 0) {
-    const std::string key = dev + "|aout|" + shape;
-    int best = 0;
-    if (!tune_lookup(key, &best)) {
-      float tbest = 1e30f;
-      for (int S = 1; S <= 32; S <<= 1) {
-        L.aout_lanes_tuned = S;
-        const float t = time_launches(s, [&] { aout_residual<T>(s, L, L.x.p, L.r.p); });
-        if (t < tbest) {
-          tbest = t;
-          best = S;
-        }
+  const std::string key = device_tag(c.device) + "|lanes|" + std::to_string(sizeof(T)) + "_" + std::to_string(L.n) +
+                          "_" + std::to_string(L.Aout.nnz);
+  int best = 0;
+  if (!tune_lookup(key, &best)) {
+    // inputs of the timed launches: finite values in the level's work vectors
+    FG_CUDA(cudaMemsetAsync(L.x.p, 0, L.x.n * sizeof(T), s));
+    FG_CUDA(cudaMemsetAsync(L.r.p, 0, L.r.n * sizeof(T), s));
+    L.aout_lanes_tuned = 0;
+    const int rule = aout_lanes(L);
+    const auto time = [&](int S) {
+      L.aout_lanes_tuned = S;
+      return time_launches(s, [&] { aout_residual<T>(s, L, L.x.p, L.r.p); });
+    };
+    float least = 0.9f * time(rule);
+    best = rule;
+    for (int S : {rule / 2, rule * 2}) {
+      if (S < 1 || S > 32) continue;
+      const float t = time(S);
+      if (t < least) {
+        least = t;
+        best = S;
       }
-      tune_store(key, best);
     }
-    L.aout_lanes_tuned = best;
-    if (verbose) fprintf(stderr, "[femgpu tune] level n=%d cross-partition lanes %d\n", L.n, best);
+    tune_store(key, best);
   }
+  L.aout_lanes_tuned = best;
+  if (getenv("FEMGPU_PROFILE"))
+    fprintf(stderr, "[femgpu tune] level n=%d cross-partition lanes %d\n", L.n, best);
 }
 
 template void autotune_level<float>(Ctx&, Level<float>&);
