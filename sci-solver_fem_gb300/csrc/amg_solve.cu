@@ -360,12 +360,12 @@ __device__ __forceinline__ T gather_row(const int32_t* __restrict__ ci, const T*
   return s;
 }
 
-// Shared memory of the register smoother: two mbarriers, x twice (each buffer holds
-// kXCopies copies of the group's x, xcopy_stride<T>() elements apart), then two staging
-// buffers for a group's in-partition values and 16-bit columns (ecap entries each, filled
+// Shared memory of the register smoother: the mbarrier, x twice (each buffer holds
+// kXCopies copies of the group's x, xcopy_stride<T>() elements apart), then the staging
+// buffer for a group's in-partition values and 16-bit columns (ecap entries, filled
 // as 16-byte rounded ranges).
 struct RegSmemLayout {
-  size_t x0, x1, val0, col0, val1, col1, total;
+  size_t x0, x1, val, col, total;
 };
 
 template <class T>
@@ -379,23 +379,26 @@ __host__ __device__ inline RegSmemLayout reg_smem_layout(int ecap) {
   constexpr size_t xbytes = (size_t)kXCopies * xcopy_stride<T>() * sizeof(T);
   L.x0 = 16;
   L.x1 = L.x0 + xbytes;
-  L.val0 = round16<T>(L.x1 + xbytes);
-  L.col0 = round16<T>(L.val0 + (size_t)ecap * sizeof(T));
-  L.val1 = round16<T>(L.col0 + (size_t)ecap * 2);
-  L.col1 = round16<T>(L.val1 + (size_t)ecap * sizeof(T));
-  L.total = round16<T>(L.col1 + (size_t)ecap * 2);
+  L.val = round16<T>(L.x1 + xbytes);
+  L.col = round16<T>(L.val + (size_t)ecap * sizeof(T));
+  L.total = round16<T>(L.col + (size_t)ecap * 2);
   return L;
 }
 
+// Copies one 32-bit word to shared memory without waiting for it (cp.async.wait_all does).
+__device__ __forceinline__ void copy_word_async(int* smem, const int* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(smem)), "l"(gmem) : "memory");
+}
+
 // One thread (thread 0) starts the bulk copies of a group's values and columns (entries
-// [es, ee) of the jagged-diagonal arrays) into staging buffer `buf`; completion is counted
-// on bar[buf].  A group's entries are one contiguous range (the reordering stays inside
+// [es, ee) of the jagged-diagonal arrays) into the staging buffer; completion is counted
+// on bar.  A group's entries are one contiguous range (the reordering stays inside
 // each 32-row block).  With orp (post relax), the group's cross-partition entries
 // [o0, o1), also one contiguous range, are prefetched into L2 for the b - A_out x that
 // opens the group.
 template <class T>
-__device__ __forceinline__ void stage_group(unsigned char* sm, const RegSmemLayout& Ls, uint64_t* bar, int buf,
-                                            int es, int ee, const uint16_t* __restrict__ jc,
+__device__ __forceinline__ void stage_group(unsigned char* sm, const RegSmemLayout& Ls, uint64_t* bar, int es,
+                                            int ee, const uint16_t* __restrict__ jc,
                                             const T* __restrict__ jv, const int32_t* __restrict__ oci = nullptr,
                                             const T* __restrict__ ov = nullptr, int o0 = 0, int o1 = 0) {
   constexpr int VA = 16 / (int)sizeof(T);
@@ -406,16 +409,20 @@ __device__ __forceinline__ void stage_group(unsigned char* sm, const RegSmemLayo
   const int v0 = es & ~(VA - 1), c0 = es & ~7;
   const uint32_t vbytes = (uint32_t)((((ee + VA - 1) & ~(VA - 1)) - v0) * (int)sizeof(T));
   const uint32_t cbytes = (uint32_t)((((ee + 7) & ~7) - c0) * 2);
-  mbar_arrive_expect_tx(bar + buf, vbytes + cbytes);
-  if (vbytes) bulk_copy_g2s(sm + (buf ? Ls.val1 : Ls.val0), jv + v0, vbytes, bar + buf);
-  if (cbytes) bulk_copy_g2s(sm + (buf ? Ls.col1 : Ls.col0), jc + c0, cbytes, bar + buf);
+  mbar_arrive_expect_tx(bar, vbytes + cbytes);
+  if (vbytes) bulk_copy_g2s(sm + Ls.val, jv + v0, vbytes, bar);
+  if (cbytes) bulk_copy_g2s(sm + Ls.col, jc + c0, cbytes, bar);
 }
 
 // Register-resident smoother for groups of at most 512 rows whose in-partition rows
 // have at most K entries: one thread per row, persistent CTAs walking the groups.
-// A group's values and 16-bit local columns are contiguous in HBM; thread 0 moves the
-// NEXT group's ranges into the other staging buffer with bulk asynchronous copies
-// (TMA) while the CTA smooths the current one.  Lane p of the warp that owns a 32-row
+// A group's values and 16-bit local columns are contiguous in HBM; as soon as the CTA has
+// the current group's in registers, thread 0 moves the NEXT group's over them in the
+// staging buffer with bulk asynchronous copies (TMA), which land while the CTA smooths.
+// One buffer instead of two leaves FP64 (which an SM's 2 FP64 lanes bound: 80% of their rate
+// with one CTA, whose 13 busy warps of 16 load the 4 schedulers unevenly) room for a second
+// CTA per SM and FP32 more L1 for the gathers of b - A_out x: 708 FP64 groups pre 101.8 ->
+// 93.2, post 115.8 -> 104.7 us; 4991 FP32 groups pre 78.3 -> 77.6, post 120.3 -> 113.6 us.  Lane p of the warp that owns a 32-row
 // block smooths the block's row at sorted position p (rows by decreasing length), and
 // the entries are stored diagonal by diagonal, so the lanes read their k-th entries
 // from consecutive shared-memory words.  Each thread keeps its row's entries in
@@ -456,13 +463,12 @@ __global__ void __launch_bounds__(512, 2) smooth_reg_kernel(
   constexpr int VA = 16 / (int)sizeof(T);
   const int t = threadIdx.x, lane = t & 31;
   // Group bounds travel across iterations, so no warp waits on a dependent global load
-  // at a group's start: rows [rs, re) of this group and [rsn, ren) of the next one; thread
-  // 0 also holds the next group's entry range [esn, een) and cross-partition range
-  // [osn, oen) for the staging it starts, and sh_es[buf] is the entry offset where the
-  // group staged into buffer buf begins.
-  __shared__ int sh_es[2];
+  // at a group's start: rows [rs, re) of this group and [rsn, ren) of the next one; sh_next
+  // (thread 0's, filled by asynchronous copies that it waits for one group later) holds the next
+  // group's entry range and cross-partition range for the staging it starts, sh_es is the entry offset where the staged group begins.
+  __shared__ int sh_es, sh_next[4];
   const int g0 = blockIdx.x;
-  int rs = 0, re = 0, rsn = 0, ren = 0, esn = 0, een = 0, osn = 0, oen = 0;
+  int rs = 0, re = 0, rsn = 0, ren = 0;
   if (g0 < ngroups) {
     rs = grows[g0];
     re = grows[g0 + 1];
@@ -473,18 +479,17 @@ __global__ void __launch_bounds__(512, 2) smooth_reg_kernel(
   }
   if (t == 0) {
     mbar_init(bar, 1);
-    mbar_init(bar + 1, 1);
     if (g0 < ngroups) {
       const int es0 = irp[rs];
-      sh_es[0] = es0;
-      stage_group<T>(sm, Ls, bar, 0, es0, irp[re], jc, jv);
+      sh_es = es0;
+      stage_group<T>(sm, Ls, bar, es0, irp[re], jc, jv);
     }
     if (g0 + (int)gridDim.x < ngroups) {
-      esn = irp[rsn];
-      een = irp[ren];
+      sh_next[0] = irp[rsn];
+      sh_next[1] = irp[ren];
       if (orp) {
-        osn = orp[rsn];
-        oen = orp[ren];
+        sh_next[2] = orp[rsn];
+        sh_next[3] = orp[ren];
       }
     }
   }
@@ -494,14 +499,7 @@ __global__ void __launch_bounds__(512, 2) smooth_reg_kernel(
   pdl_enter();
   int i = 0;
   for (int g = g0; g < ngroups; g += gridDim.x, i++) {
-    const int buf = i & 1;
-    const uint32_t parity = (uint32_t)(i >> 1) & 1u;
     const int gn = g + gridDim.x, gn2 = gn + gridDim.x;
-    // buffer buf ^ 1 was last read before the barrier that ended the previous group
-    if (t == 0 && gn < ngroups) {
-      sh_es[buf ^ 1] = esn;
-      stage_group<T>(sm, Ls, bar, buf ^ 1, esn, een, jc, jv, orp ? oci : nullptr, ov, osn, oen);
-    }
     // the bounds of the group after next, used from the next iteration on
     int rsn2 = 0, ren2 = 0;
     if (gn2 < ngroups) {
@@ -577,18 +575,18 @@ __global__ void __launch_bounds__(512, 2) smooth_reg_kernel(
       for (int c = 0; c < kXCopies; c++) xa[loc + c * CS] = x;
     }
     const int kmax = __shfl_sync(0xffffffffu, len, 0);  // lane 0 holds the block's longest row
-    const bool ok = mbar_wait_bounded(bar + buf, parity, wait_limit);
+    const bool ok = mbar_wait_bounded(bar, (uint32_t)i & 1u, wait_limit);
     // Entry k of this lane's row: its value, and the index of the x it reads within an x
     // buffer (group-local column + copy stride: below 2^16), two per register.
     T val[K];
     uint32_t offp[K / 2];
     {
-      const int es = sh_es[buf];
+      const int es = sh_es;
       // the block's entries start where its first row's do (the reordering stays in the
       // block): lane 0 loaded that row's offset
       const int eb = __shfl_sync(0xffffffffu, ne0, 0);
-      const T* sval = reinterpret_cast<const T*>(sm + (buf ? Ls.val1 : Ls.val0)) + (eb - (es & ~(VA - 1)));
-      const uint16_t* scol = reinterpret_cast<const uint16_t*>(sm + (buf ? Ls.col1 : Ls.col0)) + (eb - (es & ~7));
+      const T* sval = reinterpret_cast<const T*>(sm + Ls.val) + (eb - (es & ~(VA - 1)));
+      const uint16_t* scol = reinterpret_cast<const uint16_t*>(sm + Ls.col) + (eb - (es & ~7));
       int dk = lane;  // this lane's position on diagonal k
 #pragma unroll
       for (int k = 0; k < K; k++) {
@@ -601,24 +599,32 @@ __global__ void __launch_bounds__(512, 2) smooth_reg_kernel(
         dk += __popc(m);
       }
     }
-    // thread 0: the entry and cross-partition ranges of the group after next (its row
-    // bounds have arrived by now), for the staging it starts in the next iteration
-    if (t == 0 && gn2 < ngroups) {
-      esn = irp[rsn2];
-      een = irp[ren2];
-      if (orp) {
-        osn = orp[rsn2];
-        oen = orp[ren2];
-      }
-    }
     if (__syncthreads_or(!ok)) {
       if (t == 0) {
         *kerr = 1.0 + g;  // where: the first group whose copy did not land
-        // let the copies in flight land before the CTA exits
-        (void)mbar_wait_bounded(bar + buf, parity);
-        if (gn < ngroups) (void)mbar_wait_bounded(bar + (buf ^ 1), (uint32_t)((i + 1) >> 1) & 1u);
+        (void)mbar_wait_bounded(bar, (uint32_t)i & 1u);  // let it land before the CTA exits
+        asm volatile("cp.async.wait_all;" ::: "memory");
       }
       return;
+    }
+    // every entry of this group is in registers: the next group's are staged over them; then
+    // the ranges of the group after next (its row bounds have arrived by now)
+    if (t == 0) {
+      if (gn < ngroups) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        const int es = sh_next[0];
+        sh_es = es;
+        stage_group<T>(sm, Ls, bar, es, sh_next[1], jc, jv, orp ? oci : nullptr, ov, orp ? sh_next[2] : 0,
+                       orp ? sh_next[3] : 0);
+      }
+      if (gn2 < ngroups) {
+        copy_word_async(sh_next, irp + rsn2);
+        copy_word_async(sh_next + 1, irp + ren2);
+        if (orp) {
+          copy_word_async(sh_next + 2, orp + rsn2);
+          copy_word_async(sh_next + 3, orp + ren2);
+        }
+      }
     }
     // Fused multiply-adds in entry order over the row's entries (lanes past their row's
     // end are predicated off and touch no shared memory).
@@ -663,7 +669,7 @@ __global__ void __launch_bounds__(512, 2) smooth_reg_kernel(
         r_out[row] = u - d * x;
       }
     }
-    __syncthreads();  // x buffers and this staging buffer are free for the next group
+    __syncthreads();  // the x buffers are free for the next group
     rs = rsn;
     re = ren;
     rsn = rsn2;
@@ -1736,8 +1742,7 @@ void smooth_sweeps(Ctx& c, Level<T>& L, bool post, const T* b, const T* xin, T* 
   }
   if (smoother_in_registers(L.max_in_row, L.max_part_rows)) {
     auto k = post ? smooth_reg_kernel<T, true, kRegRow> : smooth_reg_kernel<T, false, kRegRow>;
-    if (L.smooth_smem > 48 * 1024)
-      ensure_smem(k, L.smooth_smem);
+    ensure_smem(k, L.smooth_smem);
     FG_LAUNCH_PDL(k, L.smooth_grid, L.smooth_threads, L.smooth_smem, s, L.ngroups, L.grows.p, L.Ain.rp.p, L.jc16.p,
               L.jv.p, L.jrow.p, L.diag.p, L.dinv.p, b, w, inner, xin, xout, rout, L.max_group_ents + 16,
               c.red.p + 2 * kRedBlocks + S_KERR, f.b64, f.b_store, f.aout ? L.Aout.rp.p : nullptr,
@@ -1747,7 +1752,7 @@ void smooth_sweeps(Ctx& c, Level<T>& L, bool post, const T* b, const T* xin, T* 
   }
   if (L.rows_c > 0) {
     RowSmoothFn<T> k = pick_row_kernel<T>(post, L.smooth_lanes);
-    if (L.smooth_smem > 48 * 1024) ensure_smem(k, L.smooth_smem);
+    ensure_smem(k, L.smooth_smem);
     launch_clustered(k, L.ngroups * L.rows_c, L.smooth_threads, L.smooth_smem, L.rows_c, s, (const int32_t*)L.grows.p,
                      (const int32_t*)L.Ain.rp.p, (const int32_t*)L.qrp.p, (const uint16_t*)L.rc.p, (const T*)L.rv.p, (const uint8_t*)L.rrow.p,
                      (const T*)L.diag.p, (const T*)L.dinv.p, b, w, inner, xin, xout, rout, L.rows_ecap,
@@ -2162,7 +2167,7 @@ bool row_plan(Ctx& c, Level<T>& L, int S, int C) {
   if (sm > kSmemOptIn) return false;
   for (int post = 0; post < 2; post++) {
     RowSmoothFn<T> k = pick_row_kernel<T>(post != 0, S);
-    if (sm > 48 * 1024) ensure_smem(k, sm);
+    ensure_smem(k, sm);
     int clusters = 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(L.ngroups * C));
@@ -2207,8 +2212,7 @@ void plan_smoother(Ctx& c, Level<T>& L) {
     int per_sm = 0;
     for (int post = 0; post < 2; post++) {
       auto k = post ? smooth_reg_kernel<T, true, kRegRow> : smooth_reg_kernel<T, false, kRegRow>;
-      if (L.smooth_smem > 48 * 1024)
-        ensure_smem(k, L.smooth_smem);
+      ensure_smem(k, L.smooth_smem);
       int nb = 0;
       FG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, L.smooth_threads, L.smooth_smem));
       per_sm = post ? std::min(per_sm, nb) : nb;

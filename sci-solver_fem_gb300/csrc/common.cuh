@@ -207,7 +207,8 @@ inline int grid_for(int64_t n, int block) {
 void ensure_dynamic_smem(const void* func, size_t bytes);
 template <class F>
 inline void ensure_smem(F* func, size_t bytes) {
-  if (bytes > 48 * 1024) ensure_dynamic_smem(reinterpret_cast<const void*>(func), bytes);
+  // below the 48 KB that need no permission: a kernel's static arrays count towards them too
+  if (bytes > 40 * 1024) ensure_dynamic_smem(reinterpret_cast<const void*>(func), bytes);
 }
 
 // The largest power-of-two cluster of up to `most` CTAs of `threads` threads (static shared
