@@ -229,8 +229,8 @@ femgpu_status femgpu_spmv_device(femgpu_handle h, const double* d_x, double* d_y
  * time step and cannot allocate there: applications that hand almost all device
  * memory to their own pool at start-up, or run under a fixed per-process memory
  * cap, where a hidden allocation mid-step can fail.
- * The two per-element scratch arrays live in a fixed region built into the
- * library: 2 x FEMGPU_NOALLOC_MAX_ELEMENTS doubles (32 MiB) per device, reserved
+ * The per-element scratch (a pair of values per element) lives in a fixed region built into
+ * the library: 2 x FEMGPU_NOALLOC_MAX_ELEMENTS doubles (32 MiB) per device, reserved
  * when this part of the library is first used under CUDA's lazy module loading (the
  * default since CUDA 12.2; with CUDA_MODULE_LOADING=EAGER, when the library is
  * loaded into a device context).  Meshes with more elements are
