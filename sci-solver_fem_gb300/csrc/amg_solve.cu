@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdio>
 #include <deque>
+#include <limits>
 #include <map>
 #include <mutex>
 #include <string>
@@ -2160,6 +2161,8 @@ template <class T>
 bool row_plan(Ctx& c, Level<T>& L, int S, int C) {
   // (one lane means rows of at most 16 entries in partitions of more than 512 rows)
   if (S < 2 || S > 16 || L.max_group_rows > kRegGroupRows) return false;
+  // padded rows are counted in int32, as the entries are
+  if (L.Ain.nnz + 3 * (int64_t)L.n + 16 > std::numeric_limits<int32_t>::max()) return false;
   const int qs = ((L.max_group_rows + C - 1) / C + 31) / 32 * 32;
   const int ecap =
       (int)std::min<int64_t>(L.max_group_ents + 3 * (int64_t)L.max_group_rows, (int64_t)qs * (L.max_in_row + 3)) + 16;
