@@ -77,6 +77,7 @@ struct Mesh {
   // slot[q * k + b]: position, within the row of incidence q's vertex, of the column of
   // vertex b of q's element (rows of at most kSlotRowMax entries; empty otherwise)
   DBuf<uint8_t> slot;
+  bool repeats = false;  // an element of the slot map names a vertex more than once
 };
 constexpr int kSlotRowMax = 32;
 

@@ -272,11 +272,16 @@ __global__ void __launch_bounds__(128) element2d_kernel(const double* __restrict
 }
 
 // Positions within its row of every (incidence, element vertex) pair, for the gather
-// below (one binary search each, once per mesh).
+// below (one binary search each, once per mesh).  An element that names a vertex more than
+// once has several entries at one position; the second, third and fourth of them carry their
+// turn in the upper two bits, and *repeats is set.
+constexpr int kSlotTurn = 6;  // positions are below kSlotRowMax
+static_assert(kSlotRowMax <= 1 << kSlotTurn, "turns share a byte with the positions");
+
 __global__ void slot_map_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ cols,
                                 const int32_t* __restrict__ vstart, const int32_t* __restrict__ inc,
                                 const int32_t* __restrict__ conn, int nv, int k, uint8_t* __restrict__ slot,
-                                int32_t* bad) {
+                                int32_t* bad, int32_t* repeats) {
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
     const int rb = rowptr[v], re = rowptr[v + 1];
     for (int q = vstart[v]; q < vstart[v + 1]; q++) {
@@ -289,7 +294,10 @@ __global__ void slot_map_kernel(const int32_t* __restrict__ rowptr, const int32_
           slot[(int64_t)q * k + b] = 0;
           continue;
         }
-        slot[(int64_t)q * k + b] = (uint8_t)(s - rb);
+        int turn = 0;
+        for (int o = 0; o < b; o++) turn += conn[(int64_t)e * k + o] == col;
+        if (turn) *repeats = 1;
+        slot[(int64_t)q * k + b] = (uint8_t)((s - rb) | turn << kSlotTurn);
       }
     }
   }
@@ -297,16 +305,17 @@ __global__ void slot_map_kernel(const int32_t* __restrict__ rowptr, const int32_
 
 // Four lanes per row with the row's sums in shared memory (at most kSlotRowMax entries,
 // kSlotRowMax + 1 doubles apart per row): lane b adds entry b of each incident element's
-// row, in element order, at the position the slot map gives (an element's vertices are
-// distinct, so the lanes of a row never meet; an element that repeats a vertex has zero
-// volume and only NaN entries).  Bound by the chain of shared-memory adds, 24 per row of a
-// tetrahedral mesh, so a row's lanes work side by side and the sectors, codes and slots of
-// the next four elements are loaded ahead.  101^3 cells: 335 us (one thread per row,
+// row, in element order, at the position the slot map gives.  The lanes of a row never meet
+// in a mesh whose elements have distinct vertices; with REPEATS lanes at one position add one
+// after the other, in the order of the element's vertices (such an element's volume is only
+// nearly zero after rounding, so its entries are finite).  Bound by the chain of shared-memory
+// adds, 24 per row of a tetrahedral mesh, so a row's lanes work side by side and the sectors,
+// codes and slots of the next four elements are loaded ahead.  101^3 cells: 335 us (one thread per row,
 // entry-major table, four 8-byte reads of as many sectors per incidence: 874 us; one thread
 // per row on this table: 705 us).
 constexpr int kGatherThreads = 256;
 
-template <int K>
+template <int K, bool REPEATS>
 __global__ void __launch_bounds__(kGatherThreads, 6) gather_rows_slot_kernel(
     const int32_t* __restrict__ rowptr, const int32_t* __restrict__ vstart, const int32_t* __restrict__ inc,
     const uint8_t* __restrict__ slot, const double* __restrict__ ev, int nv, double* __restrict__ vals) {
@@ -350,8 +359,15 @@ __global__ void __launch_bounds__(kGatherThreads, 6) gather_rows_slot_kernel(
     load(q + U);
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      if (q + u < q1) acc[at[u]] += w[u];
-      __syncwarp();  // a column's next contribution may come from another lane of the row
+      if (REPEATS) {
+        for (int turn = 0; turn < K; turn++) {
+          if (q + u < q1 && at[u] >> kSlotTurn == turn) acc[at[u] & ((1 << kSlotTurn) - 1)] += w[u];
+          __syncwarp();
+        }
+      } else {
+        if (q + u < q1) acc[at[u]] += w[u];
+        __syncwarp();  // a column's next contribution may come from another lane of the row
+      }
     }
   }
   __syncwarp();
@@ -548,7 +564,8 @@ void gather_rows(Ctx& c, const double* ev, double* vals) {
   cudaStream_t s = c.stream;
   Mesh& M = c.mesh;
   if (M.slot.n) {
-    auto k = M.k == 4 ? gather_rows_slot_kernel<4> : gather_rows_slot_kernel<3>;
+    auto k = M.repeats ? (M.k == 4 ? gather_rows_slot_kernel<4, true> : gather_rows_slot_kernel<3, true>)
+                       : (M.k == 4 ? gather_rows_slot_kernel<4, false> : gather_rows_slot_kernel<3, false>);
     FG_LAUNCH(k, grid_for(M.nv, kGatherThreads / 4), kGatherThreads, 0, s, c.A.rp.p, M.vstart.p, M.inc.p, M.slot.p, ev,
               (int)M.nv, vals);
     return;
@@ -603,11 +620,15 @@ void build_mesh_pattern(Ctx& c) {
   c.A_max_row = reduce_max_row_length(c);
   if (c.A_max_row <= kSlotRowMax) {
     M.slot.alloc((size_t)nslots * k, s);
-    DBuf<int32_t> bad2(1, s);
-    bad2.zero();
+    DBuf<int32_t> found(2, s);
+    found.zero();
     FG_LAUNCH(slot_map_kernel, grid_for(nv, 128), 128, 0, s, c.A.rp.p, c.A.ci.p, M.vstart.p, M.inc.p, M.conn.p, nv,
-              k, M.slot.p, bad2.p);
-    FG_REQUIRE(read_scalar(bad2.p, s) == 0, FEMGPU_ERR_INVALID, "element vertex outside the pattern");
+              k, M.slot.p, found.p, found.p + 1);
+    int32_t h[2];
+    found.download(h, 2);
+    FG_CUDA(cudaStreamSynchronize(s));
+    FG_REQUIRE(h[0] == 0, FEMGPU_ERR_INVALID, "element vertex outside the pattern");
+    M.repeats = h[1] != 0;
   }
   // level-0 aggregation graph: the pattern without self loops
   c.gxadj.alloc(nv + 1, s);
