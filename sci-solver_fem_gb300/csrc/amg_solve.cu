@@ -2726,7 +2726,7 @@ struct BatchGraph {
 
 std::mutex g_batch_mu;
 std::deque<std::unique_ptr<BatchGraph>> g_batch;  // most recently used first
-constexpr size_t kBatchGraphsKept = 4;
+constexpr size_t kBatchGraphsKept = 32;  // a graph holds one part of a batch (6 handles at most)
 
 // One independent branch per mesh: the kernels amg_solve_device runs before its loop (b and
 // x read from c.bat_b and c.bat_x), the PCG while loop, then x back to c.bat_x and the
@@ -2813,8 +2813,10 @@ bool batch_solve_graph(const std::vector<Ctx*>& hs, std::vector<SolveResult>& re
     g_batch.erase(it);
   }
   if (!bg || bg->gens != gens) {
-    // capture the branches again (new hierarchies, new buffers); the executable graph is
-    // updated in place when its topology is unchanged, else instantiated anew
+    // capture the branches again (new hierarchies, new buffers) and instantiate them anew: an
+    // update in place would bring kernel arguments that name the new graph's conditional
+    // handles to while nodes made with the old graph's
+    bg.reset();
     const int64_t before = g_kernel_launches.load();
     cudaGraph_t g = nullptr;
     std::vector<int64_t> body(hs.size(), 0);
@@ -2822,16 +2824,8 @@ bool batch_solve_graph(const std::vector<Ctx*>& hs, std::vector<SolveResult>& re
     bool ok = cudaGraphCreate(&g, 0) == cudaSuccess;
     for (size_t i = 0; ok && i < hs.size(); i++) ok = add_batch_branch(*hs[i], g, &body[i], &fixed);
     g_kernel_launches.store(before);
-    if (ok && bg && bg->exec) {
-      cudaGraphExecUpdateResultInfo info;
-      if (cudaGraphExecUpdate(bg->exec, g, &info) != cudaSuccess) {
-        (void)cudaGetLastError();
-        cudaGraphExecDestroy(bg->exec);
-        bg->exec = nullptr;
-      }
-    }
-    if (ok && (!bg || !bg->exec)) {
-      if (!bg) bg = std::make_unique<BatchGraph>();
+    if (ok) {
+      bg = std::make_unique<BatchGraph>();
       ok = cudaGraphInstantiate(&bg->exec, g, 0) == cudaSuccess;
       if (!ok) bg->exec = nullptr;
     }
