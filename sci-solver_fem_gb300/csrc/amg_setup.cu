@@ -1789,19 +1789,19 @@ void run_esc_sort(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>& o
     gacc.alloc((size_t)dgrid * ncols_out, s);
     gmark.alloc((size_t)dgrid * ncols_out, s);
   }
-  if (ad.nbig > 0 && dense_shared && dsm > 48 * 1024) {
+  if (ad.nbig > 0 && dense_shared) {
     ensure_smem(esc_dense_kernel<T, MODE, false>, dsm);
     ensure_smem(esc_dense_kernel<T, MODE, true>, dsm);
   }
   const size_t wsm = (size_t)kEscWarps * kEscWarpCap * (sizeof(unsigned long long) + sizeof(T));
   const size_t bsm = (size_t)kEscBlockCap * (sizeof(unsigned long long) + sizeof(T));
-  static bool attr_set = false;
-  if (!attr_set) {
+  if (warp_tier) {
     ensure_smem(esc_warp_kernel<T, MODE, false>, wsm);
     ensure_smem(esc_warp_kernel<T, MODE, true>, wsm);
+  }
+  if (a.nbig > 0) {
     ensure_smem(esc_block_kernel<T, MODE, false>, bsm);
     ensure_smem(esc_block_kernel<T, MODE, true>, bsm);
-    attr_set = true;
   }
   const int look = std::max(1, std::min(32, nrows_out / (152 * 64)));
   const int wgrid = (int)std::min<int64_t>(((int64_t)nrows_out + look * kEscWarps - 1) / (look * kEscWarps), 152 * 64);
@@ -2337,7 +2337,7 @@ void run_spgemm_hash(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>
   auto dense_rows = [&](const int32_t* toff, int32_t* tci, T* tv, int32_t* cnt) {
     const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)(200 * 1024) / dper));
     const size_t dsm = (size_t)wpb * dper;
-    if (dsm > 48 * 1024) ensure_smem(spgemm_dense_warp_kernel<T>, dsm);
+    ensure_smem(spgemm_dense_warp_kernel<T>, dsm);
     FG_LAUNCH(spgemm_dense_warp_kernel<T>, (int)std::min<int64_t>((nrows_out + wpb - 1) / wpb, 152 * 4), 32 * wpb,
               dsm, s, a, ncols_out, toff, tci, tv, cnt);
   };
@@ -2426,10 +2426,8 @@ void run_spgemm_hash(Ctx& c, EscArgs<T> a, int nrows_out, int ncols_out, DCsr<T>
       EscArgs<T> ad = a;
       ad.nbig = n2;
       ad.big_rows = over2.p;
-      if (dsm > 48 * 1024) {
-        ensure_smem(esc_dense_kernel<T, ESC_SPGEMM, false>, dsm);
-        ensure_smem(esc_dense_kernel<T, ESC_SPGEMM, true>, dsm);
-      }
+      ensure_smem(esc_dense_kernel<T, ESC_SPGEMM, false>, dsm);
+      ensure_smem(esc_dense_kernel<T, ESC_SPGEMM, true>, dsm);
       ad.counts = cnt.p;
       FG_LAUNCH((esc_dense_kernel<T, ESC_SPGEMM, false>), std::min(n2, 304), 256, dsm, s, ad, ncols_out, nullptr,
                 nullptr);
@@ -3251,7 +3249,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
         FG_LAUNCH(dense_lu_kernel, 1, 1024, 0, s, N, F.p, piv.p, st.p);
         FG_REQUIRE(read_scalar(st.p, s) == 0, FEMGPU_ERR_BREAKDOWN, "coarsest matrix is singular");
         const size_t bbytes = (size_t)N * sizeof(double);
-        if (bbytes > 48 * 1024) ensure_smem(dense_inverse_kernel, bbytes);
+        ensure_smem(dense_inverse_kernel, bbytes);
         FG_LAUNCH(dense_inverse_kernel, N, std::min(1024, std::max(32, (N + 31) / 32 * 32)), bbytes, s, N, F.p, piv.p,
                   L.Ainv.p);
       }

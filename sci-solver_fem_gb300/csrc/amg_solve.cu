@@ -1762,8 +1762,7 @@ void smooth_sweeps(Ctx& c, Level<T>& L, bool post, const T* b, const T* xin, T* 
   }
   if (L.smooth_k > 0) {
     CregSmoothFn<T> k = pick_creg_kernel<T>(post, L.smooth_lanes, L.smooth_k);
-    if (L.smooth_smem > 48 * 1024)
-      ensure_smem(k, L.smooth_smem);
+    ensure_smem(k, L.smooth_smem);
     launch_clustered(k, L.ngroups * L.cluster, L.smooth_threads, L.smooth_smem, L.cluster, s,
                      (const int32_t*)L.grows.p, (const int32_t*)L.Ain.rp.p, (const int32_t*)L.Ain.ci.p,
                      (const T*)L.Ain.v.p, (const T*)L.diag.p, (const T*)L.dinv.p, b, w, inner, xin, xout, rout,
@@ -1772,8 +1771,7 @@ void smooth_sweeps(Ctx& c, Level<T>& L, bool post, const T* b, const T* xin, T* 
   }
   ClusterSmoothFn<T> k = pick_cluster_kernel<T>(post, L.smooth_staged, L.smooth_lanes);
   // the limit is a per-function attribute shared by every handle: set it per launch
-  if (L.smooth_smem > 48 * 1024)
-    ensure_smem(k, L.smooth_smem);
+  ensure_smem(k, L.smooth_smem);
   launch_clustered(k, L.ngroups * L.cluster, L.smooth_threads, L.smooth_smem, L.cluster, s,
                    (const int32_t*)L.grows.p, (const int32_t*)L.Ain.rp.p, (const int32_t*)L.Ain.ci.p,
                    (const T*)L.Ain.v.p, aorp, (const int32_t*)L.Aout.ci.p, (const T*)L.Aout.v.p,
@@ -2103,7 +2101,7 @@ bool creg_plan(Ctx& c, Level<T>& L, int S, int K, int C) {
   const size_t sm = 2 * (size_t)(mcap + 1) * sizeof(T);
   for (int post = 0; post < 2; post++) {
     CregSmoothFn<T> k = pick_creg_kernel<T>(post != 0, S, K);
-    if (sm > 48 * 1024) ensure_smem(k, sm);
+    ensure_smem(k, sm);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(L.ngroups * C));
     cfg.blockDim = dim3((unsigned)thr);
@@ -2285,7 +2283,7 @@ void plan_smoother(Ctx& c, Level<T>& L) {
     bool fits = true;
     for (int post = 0; post < 2 && fits; post++) {
       ClusterSmoothFn<T> k = pick_cluster_kernel<T>(post != 0, st, S);
-      if (sm > 48 * 1024) ensure_smem(k, sm);
+      ensure_smem(k, sm);
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)(L.ngroups * C));
       cfg.blockDim = dim3((unsigned)thr);
