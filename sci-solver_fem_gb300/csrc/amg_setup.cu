@@ -2585,7 +2585,7 @@ __global__ void dense_lu_kernel(int n, double* F, int32_t* piv, int32_t* status)
     int p = s_idx[0];
     double pb = s_best[0];
     __syncthreads();
-    if (pb == 0.0) {
+    if (!(pb > 0.0)) {  // every candidate is zero, or NaN (then no row was chosen and p is n)
       if (threadIdx.x == 0) *status = 1;
       return;
     }
