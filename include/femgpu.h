@@ -277,6 +277,11 @@ femgpu_status femgpu_profile_kernel(femgpu_handle h, int which, int reps, double
  * gives up still waits, with the full limit, for the copies it started, so the context
  * stays usable.  No reference counterpart. */
 femgpu_status femgpu_test_copy_wait_limit(femgpu_handle h, int polls);
+/* Testing of devices that run no large thread-block clusters (a partition of a GPU): the
+ * handle's next setups use clusters of at most `ctas` CTAs for the aggregation and the
+ * coarsest factorisation (below 1: the default again).  The hierarchy keeps its bits.
+ * No reference counterpart. */
+femgpu_status femgpu_test_cluster_limit(femgpu_handle h, int ctas);
 /* Number of kernel launches issued by the library on this handle so far. */
 femgpu_status femgpu_kernel_launches(femgpu_handle h, int64_t* count);
 

@@ -893,7 +893,8 @@ void aggregate_small(Ctx& c, int n, const int32_t* xadj, const int32_t* adj, int
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  const int most = largest_cluster(reinterpret_cast<const void*>(aggregate_cluster_kernel), kAggThreads, kAggCtas);
+  const int most = std::min(c.cluster_limit, largest_cluster(reinterpret_cast<const void*>(aggregate_cluster_kernel),
+                                                             kAggThreads, kAggCtas));
   const int ctas = std::min(most, next_pow2((n + kAggThreads - 1) / kAggThreads));
   at[0].val.clusterDim.x = (unsigned)ctas;
   cfg.gridDim = dim3((unsigned)ctas);
@@ -2911,7 +2912,20 @@ __global__ void __launch_bounds__(32) dense_inverse_warp_kernel(int n, const dou
     if (lane + 32 * r < n) inv[(size_t)(lane + 32 * r) * n + j] = x[r];
 }
 
-// The explicit inverse of a coarsest matrix of at most kLuMax rows; *status is set when it
+// Whether dense_inverse takes a coarsest matrix of n rows: it must fit, and the device must be
+// able to run the cluster (asked for sizes in steps of 56 rows, one panel more per CTA every
+// second step).
+template <class T>
+bool lu_in_cluster(const Ctx& c, int n) {
+  if (n > kLuMax || c.cluster_limit < kLuCluster) return false;
+  constexpr int kStep = 56;
+  static_assert(kLuMax % kStep == 0, "the largest step is kLuMax");
+  const size_t smem = lu_smem_bytes((n + kStep - 1) / kStep * kStep);
+  return largest_cluster(reinterpret_cast<const void*>(dense_lu_cluster_kernel<T>), kLuThreads, kLuCluster, smem) ==
+         kLuCluster;
+}
+
+// The explicit inverse of a coarsest matrix that lu_in_cluster accepts; *status is set when it
 // is singular.
 template <class T>
 void dense_inverse(cudaStream_t s, int n, const int32_t* rp, const int32_t* ci, const T* v, double* F, int32_t* pos,
@@ -3234,7 +3248,7 @@ void build_levels(Ctx& c, Hierarchy<T>& H) {
       DBuf<int32_t> piv(N, s), st(1, s);
       st.zero();
       L.Ainv.alloc((size_t)N * N, s);
-      if (N <= kLuMax) {
+      if (L.A64v.n ? lu_in_cluster<double>(c, N) : lu_in_cluster<T>(c, N)) {
         if (L.A64v.n)  // formed in FP64: the dense factorisation takes those values
           dense_inverse<double>(s, N, L.A.rp.p, L.A.ci.p, L.A64v.p, F.p, piv.p, st.p, L.Ainv.p);
         else

@@ -768,6 +768,12 @@ femgpu_status femgpu_test_copy_wait_limit(femgpu_handle h, int polls) {
   return FEMGPU_OK;
 }
 
+femgpu_status femgpu_test_cluster_limit(femgpu_handle h, int ctas) {
+  if (!h) return FEMGPU_ERR_INVALID;
+  h->cluster_limit = ctas < 1 ? 16 : ctas;
+  return FEMGPU_OK;
+}
+
 femgpu_status femgpu_kernel_launches(femgpu_handle h, int64_t* count) {
   (void)h;
   if (!count) return FEMGPU_ERR_INVALID;

@@ -211,10 +211,11 @@ inline void ensure_smem(F* func, size_t bytes) {
   if (bytes > 40 * 1024) ensure_dynamic_smem(reinterpret_cast<const void*>(func), bytes);
 }
 
-// The largest power-of-two cluster of up to `most` CTAs of `threads` threads (static shared
-// memory only) that the kernel can run on the current device; above 8 CTAs the kernel is
-// allowed the non-portable size.  Asked once per (device, kernel).
-int largest_cluster(const void* func, int threads, int most);
+// The largest power-of-two cluster of up to `most` CTAs of `threads` threads with `smem` bytes
+// of dynamic shared memory that the kernel can run on the current device (a partition of a GPU
+// may not have the SMs side by side); above 8 CTAs the kernel is allowed the non-portable size.
+// Asked once per (device, kernel, smem).
+int largest_cluster(const void* func, int threads, int most, size_t smem = 0);
 
 // Host round trips of the setup (counted for its phase timer).
 extern std::atomic<int64_t> g_host_syncs;

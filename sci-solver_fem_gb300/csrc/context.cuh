@@ -248,6 +248,9 @@ struct Ctx {
   // polls of the register smoother's wait for its staged entries before it gives up
   // (femgpu_test_copy_wait_limit lowers it to exercise the error path)
   int copy_wait_limit = kMbarWaitLimit;
+  // largest thread-block cluster of the setup's kernels (femgpu_test_cluster_limit lowers it to
+  // exercise what a device without such clusters runs)
+  int cluster_limit = 16;
   // block vectors and scalars of the multi-right-hand-side solve, rebuilt with the hierarchy
   std::unique_ptr<BlockStateBase> block;
   // device address of the no-alloc load vector's built-in scratch region, looked up by

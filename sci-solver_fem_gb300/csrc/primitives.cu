@@ -2,6 +2,7 @@
 // (no Thrust/CUB on the product path).
 #include <map>
 #include <mutex>
+#include <tuple>
 
 #include "common.cuh"
 
@@ -20,19 +21,21 @@ void ensure_dynamic_smem(const void* func, size_t bytes) {
 }
 
 
-int largest_cluster(const void* func, int threads, int most) {
+int largest_cluster(const void* func, int threads, int most, size_t smem) {
   static std::mutex mu;
-  static std::map<std::pair<int, const void*>, int> known;
+  static std::map<std::tuple<int, const void*, size_t>, int> known;
   int dev = 0;
   FG_CUDA(cudaGetDevice(&dev));
+  if (smem > 0) ensure_dynamic_smem(func, smem);
   std::lock_guard<std::mutex> lock(mu);
-  int& size = known[{dev, func}];
+  int& size = known[std::make_tuple(dev, func, smem)];
   if (size > 0) return size;
   if (most > 8) FG_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   for (int c = most; c > 1; c >>= 1) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)c);
     cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)c;

@@ -27,7 +27,7 @@ EXPORTS = [
     "femgpu_num_levels", "femgpu_get_level_info", "femgpu_level_get", "femgpu_vcycle", "femgpu_kernel_launches",
     "femgpu_profile_kernel", "femgpu_load_vector_device_noalloc", "femgpu_adjoint_grad",
     "femgpu_adjoint_grad_device", "femgpu_solve_multi", "femgpu_solve_multi_device", "femgpu_solve_batch",
-    "femgpu_save_hierarchy", "femgpu_load_hierarchy", "femgpu_test_copy_wait_limit",
+    "femgpu_save_hierarchy", "femgpu_load_hierarchy", "femgpu_test_copy_wait_limit", "femgpu_test_cluster_limit",
     "femgpu_read_tetgen", "femgpu_read_ply", "femgpu_read_mat_sparse", "femgpu_read_mat_array",
     "femgpu_write_mat_array", "femgpu_write_vtk",
 ]
@@ -117,6 +117,7 @@ def lib():
     L.femgpu_vcycle.argtypes = [_vp, _f64p, _f64p]
     L.femgpu_kernel_launches.argtypes = [_vp, _pi64]
     L.femgpu_test_copy_wait_limit.argtypes = [_vp, C.c_int]
+    L.femgpu_test_cluster_limit.argtypes = [_vp, C.c_int]
     L.femgpu_profile_kernel.argtypes = [_vp, C.c_int, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)]
     L.femgpu_read_tetgen.argtypes = [C.c_char_p, C.c_char_p, _pi64, _pi64, _vp, _vp, _vp]
     L.femgpu_read_ply.argtypes = [C.c_char_p, _pi64, _pi64, _vp, _vp]
@@ -305,6 +306,10 @@ class Solver:
     def test_copy_wait_limit(self, polls: int):
         """Failure-detection testing: polls of the smoother's copy wait (negative: default)."""
         _check(lib().femgpu_test_copy_wait_limit(self.h, int(polls)), self.h)
+
+    def test_cluster_limit(self, ctas: int):
+        """Testing: CTAs per cluster that the next setups may use (below 1: default)."""
+        _check(lib().femgpu_test_cluster_limit(self.h, int(ctas)), self.h)
 
     def profile_kernel(self, which: int, reps: int = 20):
         ms, nb = C.c_double(), C.c_double()
