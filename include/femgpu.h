@@ -70,7 +70,8 @@ typedef struct {
   int flexibleCG;           /* 0 = Fletcher-Reeves beta (reference), 1 = Polak-Ribiere (flexible) */
   void* stream;             /* cudaStream_t to run on; NULL = library-owned stream */
   void* mem_pool;           /* cudaMemPool_t for device buffers; NULL = a pool owned by the handle
-                               that keeps freed memory for reuse until femgpu_destroy */
+                               that keeps freed memory for reuse until femgpu_destroy.  A caller's
+                               pool gets freed buffers back at once, in the handle's stream order */
   int autotune;             /* 1 (default): at setup, time each level's result-neutral launch
                                choice (cross-partition lanes per row) once per device and level
                                shape and keep the fastest; the choices are cached for the

@@ -21,13 +21,15 @@ namespace {
 
 thread_local std::string g_last_global_error;
 
-// Routes the handle's allocations to its pool and cache for the duration of one call.
+// Routes the handle's allocations to its pool for the duration of one call, and to its cache
+// when the pool is its own: freed memory of a caller's pool goes back to it at once, where the
+// caller's other handles and the pool's owner can have it.
 struct PoolScope {
   cudaMemPool_t saved;
   BlockCache* saved_cache;
   explicit PoolScope(femgpu_handle h) : saved(g_alloc_pool), saved_cache(g_alloc_cache) {
     g_alloc_pool = h ? h->pool : nullptr;
-    g_alloc_cache = h ? &h->cache : nullptr;
+    g_alloc_cache = h && h->own_pool ? &h->cache : nullptr;
   }
   ~PoolScope() {
     g_alloc_pool = saved;

@@ -66,7 +66,8 @@ extern thread_local cudaMemPool_t g_alloc_pool;
 // 32 MB in all) for its next allocations on its stream: a setup makes about 100 short-lived
 // buffers per level, and each trip to the driver's pool costs the host 0.5-1 us, as much as
 // a launch.  Stream order makes the reuse safe (one stream, one thread at a time per handle).
-// Given back with the handle, and before an allocation is allowed to fail.
+// Given back with the handle, and before an allocation is allowed to fail.  Handles on a
+// caller's memory pool do without.
 struct BlockCache {
   static constexpr size_t kLargest = size_t(1) << 20, kMost = size_t(32) << 20;
   static constexpr int kClasses = 13;  // 256 B .. 1 MB
