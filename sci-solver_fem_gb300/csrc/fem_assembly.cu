@@ -286,6 +286,7 @@ __global__ void slot_map_kernel(const int32_t* __restrict__ rowptr, const int32_
     const int rb = rowptr[v], re = rowptr[v + 1];
     for (int q = vstart[v]; q < vstart[v + 1]; q++) {
       const int e = inc[q] / k;
+      int seen[3] = {-1, -1, -1};
       for (int b = 0; b < k; b++) {
         const int col = conn[(int64_t)e * k + b];
         const int s = lower_bound_i32(cols, rb, re, col);
@@ -294,8 +295,12 @@ __global__ void slot_map_kernel(const int32_t* __restrict__ rowptr, const int32_
           slot[(int64_t)q * k + b] = 0;
           continue;
         }
-        int turn = 0;
-        for (int o = 0; o < b; o++) turn += conn[(int64_t)e * k + o] == col;
+        int turn = 0;  // earlier vertices of the element that are the same
+#pragma unroll
+        for (int o = 0; o < 3; o++) {
+          turn += o < b && seen[o] == col;
+          if (o == b) seen[o] = col;
+        }
         if (turn) *repeats = 1;
         slot[(int64_t)q * k + b] = (uint8_t)((s - rb) | turn << kSlotTurn);
       }
