@@ -336,22 +336,24 @@ __device__ void sift_down(int32_t* a, int start, int end) {
   }
 }
 
-// Segments longer than a warp's capacity: block b looks at segments 1024 b .. 1024 b + 1023
-// (and so on over the grid), lists the long ones and sorts them one after the other, so the
-// host needs no look at the lengths.  Lists of that length are rare (a vertex in more than
-// 256 elements); without one the kernel reads the offsets and ends.
+// Segments longer than a warp's capacity: block b looks at segments b, b + grid, b + 2 grid, ...
+// (1024 at a time), lists the long ones and sorts them one after the other, so the host needs
+// no look at the lengths.  Lists of that length are rare (a vertex in more than 256 elements);
+// without one the kernel reads the offsets and ends (4 us for a million).  Neighbouring segments
+// go to different blocks, because vertices of many elements are often numbered together: 1000
+// vertices of 400 triangles each, set_mesh 33.6 -> 1.25 ms; 200 of 3000 triangles, 1577 -> 12 ms.
 __global__ void __launch_bounds__(1024) segsort_long_kernel(int32_t* vals, const int32_t* off, int nseg,
                                                             int32_t* ucount) {
   __shared__ int32_t s[kBlockCap];
   __shared__ int32_t list[1024];
   __shared__ int32_t cnt, nlist;
-  for (int64_t s0 = (int64_t)blockIdx.x * 1024; s0 < nseg; s0 += (int64_t)gridDim.x * 1024) {
-    const int mine = (int)s0 + (int)threadIdx.x;
+  for (int64_t s0 = blockIdx.x; s0 < nseg; s0 += (int64_t)gridDim.x * 1024) {
+    const int64_t mine = s0 + (int64_t)gridDim.x * threadIdx.x;
     const bool is_long = mine < nseg && off[mine + 1] - off[mine] > kWarpCap;
     if (!__syncthreads_or(is_long)) continue;
     if (threadIdx.x == 0) nlist = 0;
     __syncthreads();
-    if (is_long) list[atomicAdd(&nlist, 1)] = mine;
+    if (is_long) list[atomicAdd(&nlist, 1)] = (int)mine;
     __syncthreads();
     for (int k = 0; k < nlist; k++) {
       const int seg = list[k], b = off[seg], len = off[seg + 1] - b;
@@ -439,8 +441,7 @@ void iota_i32(int32_t* a, int64_t n, cudaStream_t s) {
 void segmented_sort_i32(int32_t* vals, const int32_t* off, int nseg, int32_t* ucount, cudaStream_t s) {
   if (nseg <= 0) return;
   FG_RUN(segsort_warp_kernel<<<grid_for(nseg, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, s>>>(vals, off, nseg, ucount));
-  const int64_t blocks = ((int64_t)nseg + 1023) / 1024;
-  FG_RUN(segsort_long_kernel<<<(int)(blocks < 152 * 4 ? blocks : 152 * 4), 1024, 0, s>>>(vals, off, nseg, ucount));
+  FG_RUN(segsort_long_kernel<<<nseg < 152 * 2 ? nseg : 152 * 2, 1024, 0, s>>>(vals, off, nseg, ucount));
 }
 
 }  // namespace femgpu
