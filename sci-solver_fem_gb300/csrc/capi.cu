@@ -379,6 +379,7 @@ femgpu_status femgpu_set_mesh(femgpu_handle h, int dim, int64_t nverts, const do
     FG_REQUIRE(nverts > 0 && nelems > 0 && xyz && conn, FEMGPU_ERR_INVALID, "empty mesh");
     FG_REQUIRE(nverts < INT32_MAX && nelems * (dim + 1) < INT32_MAX, FEMGPU_ERR_LIMIT, "mesh exceeds int32 indexing");
     invalidate_hierarchy(*h);
+    h->has_mesh = h->has_matrix = h->assembled_from_mesh = false;  // until the new mesh is complete
     cudaStream_t s = h->stream;
     Mesh& M = h->mesh;
     M.dim = dim;
@@ -395,9 +396,8 @@ femgpu_status femgpu_set_mesh(femgpu_handle h, int dim, int64_t nverts, const do
       M.labels.upload(labels, nelems);
     }
     build_mesh_pattern(*h);
-    h->has_mesh = true;
-    h->has_matrix = false;
     FG_CUDA(cudaStreamSynchronize(s));
+    h->has_mesh = true;
   });
 }
 
