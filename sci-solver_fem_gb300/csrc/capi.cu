@@ -461,8 +461,12 @@ femgpu_status femgpu_set_matrix_csr(femgpu_handle h, int64_t n, const int32_t* r
       }
     }
     invalidate_hierarchy(*h);
-    h->assembled_from_mesh = false;
+    h->assembled_from_mesh = h->has_matrix = false;
     cudaStream_t s = h->stream;
+    // a matrix of the mesh's size keeps the mesh's aggregation graph
+    const bool mesh_size = h->has_mesh && h->mesh.nv == n;
+    if (mesh_size && !h->mesh_graph) build_mesh_pattern(*h);
+    h->mesh_pattern = false;
     DCsr<double>& A = h->A;
     A.n = A.m = (int)n;
     A.nnz = nnz;
@@ -473,9 +477,12 @@ femgpu_status femgpu_set_matrix_csr(femgpu_handle h, int64_t n, const int32_t* r
     A.ci.upload(cols, nnz);
     A.v.alloc(nnz > 0 ? nnz : 1, s);
     A.v.upload(vals, nnz);
-    if (!(h->has_mesh && h->mesh.nv == n)) graph_from_matrix(*h);
-    h->has_matrix = true;
+    if (!mesh_size) {
+      h->mesh_graph = false;
+      graph_from_matrix(*h);
+    }
     FG_CUDA(cudaStreamSynchronize(s));
+    h->has_matrix = true;
   });
 }
 

@@ -209,6 +209,9 @@ struct Ctx {
   DBuf<int32_t> gxadj, gadj;     // level-0 aggregation graph
   int64_t graph_nnz = 0;
   bool has_matrix = false;
+  // A's pattern and the aggregation graph are the mesh's (femgpu_set_matrix_csr replaces the
+  // pattern, and the graph when its size is another)
+  bool mesh_pattern = false, mesh_graph = false;
 
   DBuf<uint32_t> mis_seeds;      // generator seeds of the randomized MIS for cfg.seed ...
   uint32_t mis_seeds_of = 0;     // ... made for this seed

@@ -589,6 +589,7 @@ void build_mesh_pattern(Ctx& c) {
   Mesh& M = c.mesh;
   const int nv = (int)M.nv, k = M.k;
   const int64_t nslots = M.ne * k;
+  c.mesh_pattern = c.mesh_graph = false;
   DBuf<int32_t> deg(nv + 1, s), bad(1, s);
   deg.zero();
   bad.zero();
@@ -640,6 +641,7 @@ void build_mesh_pattern(Ctx& c) {
   c.gadj.alloc(nnz - nv > 0 ? nnz - nv : 1, s);
   FG_LAUNCH(graph_from_pattern_kernel, grid_for(nv, 256), 256, 0, s, c.A.rp.p, c.A.ci.p, nv, c.gxadj.p, c.gadj.p);
   c.graph_nnz = nnz - nv;
+  c.mesh_pattern = c.mesh_graph = true;
 }
 
 void assemble_operator(Ctx& c, const double* coef_host, double lambda, bool coef_on_device) {
@@ -647,6 +649,10 @@ void assemble_operator(Ctx& c, const double* coef_host, double lambda, bool coef
   Mesh& M = c.mesh;
   const int64_t ne = M.ne;
   const int k = M.k;
+  if (!c.mesh_pattern) {  // a matrix was set since the mesh
+    c.has_matrix = false;
+    build_mesh_pattern(c);
+  }
   if (k == 4) {
     double t[10];
     tet_mass_table(t);

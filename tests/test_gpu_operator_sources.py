@@ -1,9 +1,13 @@
-"""One handle given meshes in turn: a mesh that is refused leaves no operator.  Needs a GB300."""
+"""One handle given meshes and matrices in turn: a mesh that is refused leaves no operator, an
+assembly after a matrix is the mesh's own, and a matrix of the mesh's size is aggregated on the
+mesh's graph whatever was set between.  Needs a GB300."""
 import numpy as np
 import pytest
 
 import femgpu
+import oracle as O
 from femgpu import meshes
+from test_gpu_long_rows import arrow
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +42,38 @@ def test_a_refused_mesh_leaves_no_operator(dim, vertex):
         # arguments that are refused before anything is replaced leave the operator
         assert status(s.set_mesh, xyz[:0], conn) == INVALID
         assert np.array_equal(s.matrix()[2], v)
+
+
+@pytest.mark.parametrize("other", ["same size", "smaller", "larger"])
+def test_assembly_after_a_matrix_is_the_mesh_operator(other):
+    xyz, conn = meshes.kuhn_cube(4)
+    n = xyz.shape[0]
+    rp, ci = O.build_pattern(n, conn)
+    v = O.assemble(xyz, conn, rp, ci, coef=None, lambda_mass=1.0)
+    with femgpu.Solver() as s:
+        s.set_mesh(xyz, conn)
+        m = {"same size": n, "smaller": n // 2, "larger": 3 * n}[other]
+        s.set_matrix_csr(*arrow(m))  # one row of m entries, past the row gather's 32
+        assert s.matrix()[0].shape[0] == m + 1
+        for _ in range(2):
+            s.assemble(None, 1.0)
+            grp, gci, gv = s.matrix()
+            assert np.array_equal(grp, rp) and np.array_equal(gci, ci) and np.array_equal(gv, v)
+
+
+def test_matrix_of_the_mesh_size_keeps_the_mesh_graph():
+    xyz, conn, kappa, f, mask = meshes.poisson3d_problem(9, sigma=1.0)
+    n = xyz.shape[0]
+    rp, ci = O.build_pattern(n, conn)
+    v = O.assemble(xyz, conn, rp, ci, coef=kappa, lambda_mass=1.0)
+    r = np.random.default_rng(0).standard_normal(n)
+    out = []
+    for between in (False, True):
+        with femgpu.Solver(solverType=1, seed=1) as s:
+            s.set_mesh(xyz, conn)
+            if between:
+                s.set_matrix_csr(*arrow(n // 3))
+            s.set_matrix_csr(rp, ci, v)
+            s.setup()
+            out.append((s.num_levels, s.level(0)["perm"], s.vcycle(r)))
+    assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
