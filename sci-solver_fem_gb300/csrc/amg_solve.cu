@@ -2417,7 +2417,8 @@ void autotune_level(Ctx& c, Level<T>& L) {
   const std::string key = device_tag(c.device) + "|lanes|" + std::to_string(sizeof(T)) + "_" + std::to_string(L.n) +
                           "_" + std::to_string(L.Aout.nnz);
   int best = 0;
-  if (!tune_lookup(key, &best)) {
+  // (a line of the file that is not a lane count is measured again)
+  if (!tune_lookup(key, &best) || best < 1 || best > 32 || (best & (best - 1))) {
     // inputs of the timed launches: finite values in the level's work vectors
     FG_CUDA(cudaMemsetAsync(L.x.p, 0, L.x.n * sizeof(T), s));
     FG_CUDA(cudaMemsetAsync(L.r.p, 0, L.r.n * sizeof(T), s));
