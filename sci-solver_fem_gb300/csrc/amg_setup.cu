@@ -1463,10 +1463,10 @@ __global__ void collect_big_rows_kernel(int n, const int32_t* items, int cap, in
 
 // Rows of more than thread_cap and at most kEscWarpCap items, one warp each.  A warp looks at
 // `look` rows' item counts at a time: 32 on large levels (one row at a time, 2.1 M rows with
-// none to sort took 0.4 ms per pass), few on small ones, whose rows need all the warps.  Items of a permuted row have distinct columns: up to
-// kRankCap of them are placed by counting the smaller ones (a broadcast read and a compare per
-// item and lane, no barriers) instead of a bitonic network: 80,338 rows of 100 items 406 ->
-// 191 us.
+// none to sort took 0.4 ms per pass), few on small ones, whose rows need all the warps.  Items
+// of a permuted row have distinct columns: up to kRankCap of them are placed by counting the
+// smaller ones (a broadcast read and a compare per item and lane, no barriers) instead of a
+// bitonic network: 80,338 rows of 100 items 406 -> 191 us.
 constexpr int kRankCap = 256;
 
 template <class T, int MODE, bool WRITE>
@@ -3569,7 +3569,8 @@ __global__ void sliced_values_kernel(int n, int nslices, const int32_t* __restri
 
 void amg_setup(Ctx& c) {
   cudaStream_t s = c.stream;
-  FG_REQUIRE(c.has_matrix, FEMGPU_ERR_NOT_READY, "no operator: call femgpu_set_mesh + femgpu_assemble or femgpu_set_matrix_csr");
+  FG_REQUIRE(c.has_matrix, FEMGPU_ERR_NOT_READY,
+             "no operator: call femgpu_set_mesh + femgpu_assemble or femgpu_set_matrix_csr");
   FG_REQUIRE(c.cfg.aggregatorType == 0, FEMGPU_ERR_INVALID, "only aggregatorType 0 (OldMIS) is implemented");
   cudaEvent_t e0, e1;
   FG_CUDA(cudaEventCreate(&e0));

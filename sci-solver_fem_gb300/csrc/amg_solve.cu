@@ -134,7 +134,8 @@ size_t slice_smem_bytes(int mcap, int scap, int ecap) {
 
 // Sum over slice row t's in-partition entries with S lanes per row: lane j adds
 // entries j, j+S, ... in order with fused multiply-adds (the reference adds them with
-// shared-memory atomics in any order), then an xor butterfly combines the lanes.  Every lane of the warp must call it (the butterfly shuffles the warp).
+// shared-memory atomics in any order), then an xor butterfly combines the lanes.  Every lane
+// of the warp must call it (the butterfly shuffles the warp).
 template <class T, bool STAGED, int S>
 __device__ __forceinline__ T slice_row_sum(const SliceSmem<T>& P, const T* x, int t, bool live, int j,
                                            const int32_t* __restrict__ ici, const T* __restrict__ iv, int es,
@@ -423,11 +424,11 @@ __device__ __forceinline__ void stage_group(unsigned char* sm, const RegSmemLayo
 // One buffer instead of two leaves FP64 (which an SM's 2 FP64 lanes bound: 80% of their rate
 // with one CTA, whose 13 busy warps of 16 load the 4 schedulers unevenly) room for a second
 // CTA per SM and FP32 more L1 for the gathers of b - A_out x: 708 FP64 groups pre 101.8 ->
-// 93.2, post 115.8 -> 104.7 us; 4991 FP32 groups pre 78.3 -> 77.6, post 120.3 -> 113.6 us.  Lane p of the warp that owns a 32-row
-// block smooths the block's row at sorted position p (rows by decreasing length), and
-// the entries are stored diagonal by diagonal, so the lanes read their k-th entries
-// from consecutive shared-memory words.  Each thread keeps its row's entries in
-// registers across the sweeps; x is double-buffered in shared memory, kXCopies copies
+// 93.2, post 115.8 -> 104.7 us; 4991 FP32 groups pre 78.3 -> 77.6, post 120.3 -> 113.6 us.
+// Lane p of the warp that owns a 32-row block smooths the block's row at sorted position p
+// (rows by decreasing length), and the entries are stored diagonal by diagonal, so the lanes
+// read their k-th entries from consecutive shared-memory words.  Each thread keeps its row's
+// entries in registers across the sweeps; x is double-buffered in shared memory, kXCopies copies
 // per buffer, every entry's column pointing into the copy that setup chose to spread the
 // warp's gathers over the banks (one barrier per sweep).  Row sums are the one-lane case
 // of the shared-memory smoother: fused multiply-adds in entry order.  A copy that does
@@ -465,8 +466,9 @@ __global__ void __launch_bounds__(512, 2) smooth_reg_kernel(
   const int t = threadIdx.x, lane = t & 31;
   // Group bounds travel across iterations, so no warp waits on a dependent global load
   // at a group's start: rows [rs, re) of this group and [rsn, ren) of the next one; sh_next
-  // (thread 0's, filled by asynchronous copies that it waits for one group later) holds the next
-  // group's entry range and cross-partition range for the staging it starts, sh_es is the entry offset where the staged group begins.
+  // (thread 0's, filled by asynchronous copies that it waits for one group later) holds the
+  // next group's entry range and cross-partition range for the staging it starts, sh_es is the
+  // entry offset where the staged group begins.
   __shared__ int sh_es, sh_next[4];
   const int g0 = blockIdx.x;
   int rs = 0, re = 0, rsn = 0, ren = 0;
@@ -872,8 +874,8 @@ __host__ __device__ inline RowSmemLayout row_smem_layout(int ecap) {
 template <class T, bool POST, int S>
 __global__ void __launch_bounds__(512) smooth_rows_kernel(
     const int32_t* __restrict__ grows, const int32_t* __restrict__ irp, const int32_t* __restrict__ qrp,
-    const uint16_t* __restrict__ rc, const T* __restrict__ rv, const uint8_t* __restrict__ rrow, const T* __restrict__ diag,
-    const T* __restrict__ dinv, const T* __restrict__ b, T w, int inner, const T* __restrict__ x_in,
+    const uint16_t* __restrict__ rc, const T* __restrict__ rv, const uint8_t* __restrict__ rrow,
+    const T* __restrict__ diag, const T* __restrict__ dinv, const T* __restrict__ b, T w, int inner, const T* __restrict__ x_in,
     T* __restrict__ x_out, T* __restrict__ r_out, int ecap, double* __restrict__ kerr, int wait_limit) {
   extern __shared__ __align__(128) unsigned char sm[];
   constexpr unsigned kAll = 0xffffffffu;
@@ -1228,9 +1230,9 @@ __global__ void residual_kernel(int n, const double* __restrict__ b, const doubl
 
 
 
-// The device-side PCG loop after an iteration: counts it and stops the loop on convergence (the host's test:
-// sqrt(r.r) / |b| <= tol), breakdown, a non-finite residual, a smoother copy that timed out,
-// or maxIters.
+// The device-side PCG loop after an iteration: counts it and stops the loop on convergence
+// (the host's test: sqrt(r.r) / |b| <= tol), breakdown, a non-finite residual, a smoother copy
+// that timed out, or maxIters.
 __device__ __forceinline__ void pcg_check(double* sc, cudaGraphConditionalHandle loop) {
   const double it = sc[S_IT] + 1.0;
   sc[S_IT] = it;
@@ -1542,8 +1544,8 @@ CregSmoothFn<T> pick_creg_kernel(bool post, int S, int K) {
 }
 
 template <class T>
-using RowSmoothFn = void (*)(const int32_t*, const int32_t*, const int32_t*, const uint16_t*, const T*, const uint8_t*, const T*,
-                             const T*, const T*, T, int, const T*, T*, T*, int, double*, int);
+using RowSmoothFn = void (*)(const int32_t*, const int32_t*, const int32_t*, const uint16_t*, const T*,
+                             const uint8_t*, const T*, const T*, const T*, T, int, const T*, T*, T*, int, double*, int);
 
 template <class T>
 RowSmoothFn<T> pick_row_kernel(bool post, int S) {
@@ -1569,7 +1571,8 @@ void launch_clustered(void (*k)(KArgs...), int grid, int block, size_t smem, int
   at[0].val.clusterDim.x = (unsigned)cluster;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
-  // both clustered smoothers call pdl_wait() before they touch memory other kernels write
+  // every clustered smoother (cluster, lane, split and row) calls pdl_wait() before it touches
+  // memory that other kernels write
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
@@ -1755,8 +1758,8 @@ void smooth_sweeps(Ctx& c, Level<T>& L, bool post, const T* b, const T* xin, T* 
     RowSmoothFn<T> k = pick_row_kernel<T>(post, L.smooth_lanes);
     ensure_smem(k, L.smooth_smem);
     launch_clustered(k, L.ngroups * L.rows_c, L.smooth_threads, L.smooth_smem, L.rows_c, s, (const int32_t*)L.grows.p,
-                     (const int32_t*)L.Ain.rp.p, (const int32_t*)L.qrp.p, (const uint16_t*)L.rc.p, (const T*)L.rv.p, (const uint8_t*)L.rrow.p,
-                     (const T*)L.diag.p, (const T*)L.dinv.p, b, w, inner, xin, xout, rout, L.rows_ecap,
+                     (const int32_t*)L.Ain.rp.p, (const int32_t*)L.qrp.p, (const uint16_t*)L.rc.p, (const T*)L.rv.p,
+                     (const uint8_t*)L.rrow.p, (const T*)L.diag.p, (const T*)L.dinv.p, b, w, inner, xin, xout, rout, L.rows_ecap,
                      c.red.p + 2 * kRedBlocks + S_KERR, c.copy_wait_limit);
     return;
   }

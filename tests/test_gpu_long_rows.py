@@ -17,8 +17,8 @@ def arrow(n):
     """A hub coupled to every other row."""
     i = np.arange(1, n)
     w = np.random.default_rng(n).uniform(0.5, 1.0, n - 1) / n
-    A = sp.coo_matrix((np.r_[np.linspace(2.0, 4.0, n), -w, -w], (np.r_[np.arange(n), 0 * i, i], np.r_[np.arange(n), i, 0 * i])),
-                      shape=(n, n)).tocsr()
+    rows, cols = np.r_[np.arange(n), 0 * i, i], np.r_[np.arange(n), i, 0 * i]
+    A = sp.coo_matrix((np.r_[np.linspace(2.0, 4.0, n), -w, -w], (rows, cols)), shape=(n, n)).tocsr()
     A.sort_indices()
     return A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
 
