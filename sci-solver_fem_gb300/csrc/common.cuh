@@ -15,6 +15,7 @@
 
 #include <atomic>
 #include <cstdio>
+#include <new>
 #include <stdexcept>
 #include <string>
 #include <utility>
@@ -87,13 +88,16 @@ struct BlockCache {
     bytes -= class_bytes(c);
     return p;
   }
-  void give(void* p, int c) {
-    if (bytes + class_bytes(c) > kMost) {
-      cudaFreeAsync(p, stream);
-      return;
+  void give(void* p, int c) noexcept {  // called by destructors
+    if (bytes + class_bytes(c) <= kMost) {
+      try {
+        kept[c].push_back(p);
+        bytes += class_bytes(c);
+        return;
+      } catch (const std::bad_alloc&) {  // no host memory to note it: back to the pool
+      }
     }
-    kept[c].push_back(p);
-    bytes += class_bytes(c);
+    cudaFreeAsync(p, stream);
   }
   void release() {
     for (auto& k : kept) {
